@@ -451,6 +451,7 @@ template <class Epi>
 void base_shape(UmmaParams<Epi>& P, int npc, int M, int N, int K, int batch, int bn, int* err) {
   P.s.npa = P.s.npb = npc;
   P.s.npairs = pairs_for(npc, P.s.pa, P.s.pb);
+  P.s.std_npc = npc;  // every caller below accumulates in two groups
   P.s.M = M;
   P.s.N = N;
   P.s.K = K;

@@ -55,9 +55,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // Bounded wait: ~1e8 polls (each try_wait already suspends for a while).
 constexpr uint32_t kMaxPolls = 1u << 27;
 
+// The first poll stands apart from the loop: a wait on a barrier that is
+// already complete then costs 41 cycles instead of 264 (one thread, per K block
+// of the GEMMs' issue loop).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
                                           uint32_t max_polls = kMaxPolls) {
-  for (uint32_t i = 0; i < max_polls; ++i)
+  if (mbar_try_wait(bar, parity)) return true;
+#pragma unroll 1
+  for (uint32_t i = 1; i < max_polls; ++i)
     if (mbar_try_wait(bar, parity)) return true;
   return false;
 }
@@ -65,6 +70,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
 // as mbar_wait, but also gives up once *abort becomes non-zero
 __device__ __forceinline__ bool mbar_wait_abortable(uint64_t* bar, uint32_t parity,
                                                     volatile int* abort) {
+  if (mbar_try_wait(bar, parity)) return true;
+#pragma unroll 1
   for (uint32_t i = 0; i < kMaxPolls; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((i & 1023) == 1023 && *abort) return false;
@@ -228,6 +235,21 @@ __device__ __forceinline__ void umma_bf16(uint32_t dtmem, uint64_t adesc, uint64
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(dtmem),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// The low words of two such descriptors (the high word is the same for every
+// K-major SW128 operand): 32-bit address arithmetic per MMA, which issues one
+// MMA every ~50 cycles where 64-bit descriptors built from operand pointers
+// took 66-80.
+__device__ __forceinline__ uint32_t smem_desc_lo(uint32_t saddr) { return (saddr >> 4) | (1u << 16); }
+__device__ __forceinline__ void umma_bf16_lo(uint32_t dtmem, uint32_t alo, uint32_t blo,
+                                             uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n .reg .b64 da, db;\n setp.ne.b32 p, %4, 0;\n"
+      " mov.b64 da, {%1, %5};\n mov.b64 db, {%2, %5};\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n}" ::"r"(dtmem),
+      "r"(alo), "r"(blo), "r"(idesc), "r"(accumulate), "r"(0x40004040u)
       : "memory");
 }
 

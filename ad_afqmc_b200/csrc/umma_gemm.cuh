@@ -38,6 +38,7 @@ struct UmmaShape {
   int npa, npb;      // pieces of A and B
   int npairs;
   int pa[6], pb[6];
+  int std_npc;       // 2, 3: the pair list of two- or three-piece operands in two groups; 0: any other
   int ngroups;       // 1, or 2: pair 0 (the hi x hi product) accumulates apart from the rest
   int kc;            // K blocks per accumulator chunk (0: the whole K of a tile in one chunk)
   int epi_bytes;     // epilogue scratch per epilogue warpgroup (bytes, multiple of 256)
@@ -147,6 +148,39 @@ struct UmmaMany {
     return G.entries[lo];
   }
 };
+
+// The products of one K block of two- or three-piece operands, in the order of
+// the pair list: (0,0) into accumulator group 0; (0,1), (1,0) and, with three
+// pieces, (0,2), (1,1), (2,0) into group 1, BN columns further on.  NKS: 16-wide
+// K steps of the block that hold data (the zero-filled tail of a row adds
+// nothing and is not issued).  Written out, as one thread issues it all: a loop
+// over the pair list in the parameter block took 150-200 cycles per MMA, this
+// takes 50, and the tensor core 52 (N = 80) to 64 (N = 128), when it reads
+// 128 x 16 and N x 16 operands from shared memory at 128 bytes per cycle.
+template <int BN, int NPC, int NKS>
+__device__ __forceinline__ void issue_block(uint32_t dt, uint32_t alo, uint32_t blo, uint32_t as,
+                                            uint32_t bs, uint32_t acc) {
+  constexpr uint32_t idesc = instr_desc(kUBM, BN, 1);
+  constexpr int NP = NPC == 2 ? 3 : 6;
+  constexpr int pa[6] = {0, 0, 1, 0, 1, 2}, pb[6] = {0, 1, 0, 2, 1, 0};
+#pragma unroll
+  for (int p = 0; p < NP; ++p)
+#pragma unroll
+    for (int ks = 0; ks < NKS; ++ks)
+      umma_bf16_lo(dt + (p ? BN : 0), alo + pa[p] * as + 2 * ks, blo + pb[p] * bs + 2 * ks, idesc,
+                   ks != 0 || p > 1 ? 1u : acc);
+}
+
+// sa, sb: shared-memory addresses of piece 0; a_bytes, b_bytes: distance of the pieces
+template <int BN, int NPC>
+__device__ __forceinline__ void issue_pairs(uint32_t dt, uint32_t sa, uint32_t sb, uint32_t a_bytes,
+                                            uint32_t b_bytes, int nks, bool acc) {
+  const uint32_t alo = smem_desc_lo(sa), blo = smem_desc_lo(sb), as = a_bytes >> 4, bs = b_bytes >> 4;
+  if (nks == 4) issue_block<BN, NPC, 4>(dt, alo, blo, as, bs, acc);
+  else if (nks == 3) issue_block<BN, NPC, 3>(dt, alo, blo, as, bs, acc);
+  else if (nks == 2) issue_block<BN, NPC, 2>(dt, alo, blo, as, bs, acc);
+  else issue_block<BN, NPC, 1>(dt, alo, blo, as, bs, acc);
+}
 
 template <int BN, class Epi, int EG, class Src>
 __device__ __forceinline__ void umma_body(const Src& src) {
@@ -260,6 +294,7 @@ __device__ __forceinline__ void umma_body(const Src& src) {
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc = instr_desc(kUBM, BN, 1);
+      const uint32_t smem_base = su32(smem);
       int stage = 0;
       uint32_t phase = 0;
       int it = 0, t = 0;
@@ -272,6 +307,8 @@ __device__ __forceinline__ void umma_body(const Src& src) {
         const int KB = tl.KB;
         if (KB == 0) continue;  // (debug builds: a tile skipped by every role)
         const int kc = S.kc > 0 ? S.kc : KB;
+        const int klen = min(S.kchunk, S.K - tl.k0);
+        const int tail = (klen - (KB - 1) * kUBK + 15) >> 4;  // 16-wide K steps of the last block
         bool ok = true;
         for (int c0 = 0; c0 < KB && ok; c0 += kc, ++it) {
           const int buf = EG > 1 ? (t % EG) : (it & 1);
@@ -283,18 +320,24 @@ __device__ __forceinline__ void umma_body(const Src& src) {
           for (int kb = c0; kb < c1; ++kb) {
             if (!mbar_wait(&full[stage], phase)) { fail(S.err); ok = false; break; }
             tc_fence_after();
-            const uint8_t* sa = smem + stage * stage_bytes;
-            const uint8_t* sb = sa + npa * a_bytes;
-            for (int p = 0; p < S.npairs; ++p) {
-              const uint64_t ad = smem_desc_sw128(sa + S.pa[p] * a_bytes);
-              const uint64_t bd = smem_desc_sw128(sb + S.pb[p] * b_bytes);
-              // group 0: pair 0 alone; group 1 (if any): the remaining pairs
-              const int grp = (ngrp == 2 && p > 0) ? 1 : 0;
-              const int first = (p == 0) || (ngrp == 2 && p == 1);
-#pragma unroll
-              for (int ks = 0; ks < kUBK / 16; ++ks)
-                umma_bf16(dt + grp * BN, ad + 2 * ks, bd + 2 * ks, idesc,
-                          (kb - c0) != 0 || ks != 0 || !first);
+            const uint32_t sa = smem_base + stage * stage_bytes;
+            const uint32_t sb = sa + npa * a_bytes;
+            const int nks = kb + 1 < KB ? 4 : tail;
+            if (S.std_npc == 2) {
+              issue_pairs<BN, 2>(dt, sa, sb, a_bytes, b_bytes, nks, kb != c0);
+            } else if (S.std_npc == 3) {
+              issue_pairs<BN, 3>(dt, sa, sb, a_bytes, b_bytes, nks, kb != c0);
+            } else {
+              for (int p = 0; p < S.npairs; ++p) {
+                const uint32_t alo = smem_desc_lo(sa + S.pa[p] * a_bytes);
+                const uint32_t blo = smem_desc_lo(sb + S.pb[p] * b_bytes);
+                // group 0: pair 0 alone; group 1 (if any): the remaining pairs
+                const int grp = (ngrp == 2 && p > 0) ? 1 : 0;
+                const int first = (p == 0) || (ngrp == 2 && p == 1);
+                for (int ks = 0; ks < nks; ++ks)
+                  umma_bf16_lo(dt + grp * BN, alo + 2 * ks, blo + 2 * ks, idesc,
+                               kb != c0 || ks != 0 || !first);
+              }
             }
             umma_commit(&empty[stage]);
             if (++stage == ST) { stage = 0; phase ^= 1; }
