@@ -67,16 +67,32 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   return false;
 }
 
-// as mbar_wait, but also gives up once *abort becomes non-zero
-__device__ __forceinline__ bool mbar_wait_abortable(uint64_t* bar, uint32_t parity,
-                                                    volatile int* abort) {
-  if (mbar_try_wait(bar, parity)) return true;
-#pragma unroll 1
+// The waits of the GEMM kernels.  A wait that runs out sets the error flag and
+// the CTA's abort word and returns like any other; from then on every wait of
+// the CTA that is not complete at once returns too, so all roles run on to
+// their end (over data that nobody uses) and meet at the same barriers.  The
+// caller's control flow therefore does not depend on the outcome: it stays
+// uniform over the warp, and the operands of tcgen05.mma and of the TMA loads
+// stay in uniform registers.  With waits that returned a status and a single
+// branching thread, an MMA took 100-150 cycles to issue.
+static __device__ __noinline__ void mbar_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort, int* err) {
   for (uint32_t i = 0; i < kMaxPolls; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 1023) == 1023 && *abort) return false;
+    if ((i & 1023) == 0 && *abort) return;
+    if (mbar_try_wait(bar, parity)) return;
   }
-  return false;
+  atomicExch(err, 1);
+  *abort = 1;
+}
+__device__ __forceinline__ void mbar_wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort,
+                                                   int* err) {
+  if (!mbar_try_wait(bar, parity)) mbar_wait_slow(bar, parity, abort, err);
+}
+
+// true in one lane of the (converged) warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred P;\n elect.sync _|P, 0xffffffff;\n selp.u32 %0, 1, 0, P;\n}" : "=r"(p));
+  return p != 0;
 }
 
 // ---------------------------------------------------------------------------

@@ -16,7 +16,7 @@
 //               rotate over the groups, tile t in accumulator t % EG for all its
 //               K chunks, so a long epilogue of one tile runs while the other
 //               groups drain and process the next tiles
-// All waits are bounded; on timeout the CTA records an error and unwinds.
+// All waits are bounded; on timeout the CTA records an error and runs to its end.
 #pragma once
 
 #include "common.cuh"
@@ -229,10 +229,6 @@ __device__ __forceinline__ void umma_body(const Src& src) {
   const uint32_t tbase = *tmem_slot;
 
   const int tiles = src.tiles();
-  auto fail = [&](int* err) {
-    atomicExch(err, 1);
-    *abort_s = 1;
-  };
   // (global iteration) -> entry, tile of the entry, and its coordinates
   struct TileAt {
     int z, mti, nti, b, k0, KB;
@@ -260,69 +256,69 @@ __device__ __forceinline__ void umma_body(const Src& src) {
     return t;
   };
 
+  // The producer and MMA warps run their loops whole, one elected lane issues:
+  // see mbar_wait_or_abort.
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int it_ = blockIdx.x; it_ < tiles && !*abort_s; it_ += gridDim.x) {
-        int local;
-        const UmmaParams<Epi>& P = src.entry(it_, local);
-        const UmmaShape& S = P.s;
-        const TileAt t = locate(S, local);
-        bool ok = true;
-        for (int kb = 0; kb < t.KB; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1)) { fail(S.err); ok = false; break; }
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int it_ = blockIdx.x; it_ < tiles; it_ += gridDim.x) {
+      int local;
+      const UmmaParams<Epi>& P = src.entry(it_, local);
+      const UmmaShape& S = P.s;
+      const TileAt t = locate(S, local);
+      const int arow = t.mti * S.a_step, abat = S.a_batched ? t.b : 0, brow = t.nti * S.b_step;
+      for (int kb = 0; kb < t.KB; ++kb) {
+        mbar_wait_or_abort(&empty[stage], phase ^ 1, abort_s, S.err);
+        if (elect_one()) {
           mbar_arrive_expect_tx(&full[stage], stage_bytes);
           uint8_t* sa = smem + stage * stage_bytes;
           uint8_t* sb = sa + npa * a_bytes;
+          const int k = t.k0 + kb * kUBK;
           for (int i = 0; i < npa; ++i)
-            tma_load_3d(sa + i * a_bytes, &P.ta[i], &full[stage], t.k0 + kb * kUBK,
-                        t.mti * S.a_step, S.a_batched ? t.b : 0);
+            tma_load_3d(sa + i * a_bytes, &P.ta[i], &full[stage], k, arow, abat);
           for (int j = 0; j < npb; ++j)
-            tma_load_3d(sb + j * b_bytes, &P.tb[j], &full[stage], t.k0 + kb * kUBK,
-                        t.nti * S.b_step, t.b);
-          if (++stage == ST) { stage = 0; phase ^= 1; }
+            tma_load_3d(sb + j * b_bytes, &P.tb[j], &full[stage], k, brow, t.b);
         }
-        if (!ok) break;
-      }
-      // drain: wait (bounded) until the MMA side released every stage we filled
-      for (int s = 0; s < ST; ++s) {
-        if (!mbar_wait(&empty[stage], phase ^ 1)) { fail(P0.s.err); break; }
+        __syncwarp();
         if (++stage == ST) { stage = 0; phase ^= 1; }
       }
     }
+    // drain: wait (bounded) until the MMA side released every stage we filled
+    for (int s = 0; s < ST; ++s) {
+      mbar_wait_or_abort(&empty[stage], phase ^ 1, abort_s, P0.s.err);
+      if (++stage == ST) { stage = 0; phase ^= 1; }
+    }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = instr_desc(kUBM, BN, 1);
-      const uint32_t smem_base = su32(smem);
-      int stage = 0;
-      uint32_t phase = 0;
-      int it = 0, t = 0;
-      uint32_t uses[NBUF] = {};  // EG > 1: chunks accumulated so far in each buffer
-      for (int it_ = blockIdx.x; it_ < tiles && !*abort_s; it_ += gridDim.x, ++t) {
-        int local;
-        const UmmaParams<Epi>& P = src.entry(it_, local);
-        const UmmaShape& S = P.s;
-        const TileAt tl = locate(S, local);
-        const int KB = tl.KB;
-        if (KB == 0) continue;  // (debug builds: a tile skipped by every role)
-        const int kc = S.kc > 0 ? S.kc : KB;
-        const int klen = min(S.kchunk, S.K - tl.k0);
-        const int tail = (klen - (KB - 1) * kUBK + 15) >> 4;  // 16-wide K steps of the last block
-        bool ok = true;
-        for (int c0 = 0; c0 < KB && ok; c0 += kc, ++it) {
-          const int buf = EG > 1 ? (t % EG) : (it & 1);
-          const uint32_t use = EG > 1 ? uses[buf]++ : (uint32_t)(it >> 1);
-          if (!mbar_wait(&acce[buf], (use & 1) ^ 1)) { fail(S.err); ok = false; break; }
+    constexpr uint32_t idesc = instr_desc(kUBM, BN, 1);
+    const uint32_t smem_base = su32(smem);
+    int stage = 0;
+    uint32_t phase = 0;
+    int it = 0, t = 0;
+    uint32_t uses[NBUF] = {};  // EG > 1: chunks accumulated so far in each buffer
+    for (int it_ = blockIdx.x; it_ < tiles; it_ += gridDim.x, ++t) {
+      int local;
+      const UmmaParams<Epi>& P = src.entry(it_, local);
+      const UmmaShape& S = P.s;
+      const TileAt tl = locate(S, local);
+      const int KB = tl.KB;
+      if (KB == 0) continue;  // (debug builds: a tile skipped by every role)
+      const int kc = S.kc > 0 ? S.kc : KB;
+      const int klen = min(S.kchunk, S.K - tl.k0);
+      const int tail = (klen - (KB - 1) * kUBK + 15) >> 4;  // 16-wide K steps of the last block
+      for (int c0 = 0; c0 < KB; c0 += kc, ++it) {
+        const int buf = EG > 1 ? (t % EG) : (it & 1);
+        const uint32_t use = EG > 1 ? uses[buf]++ : (uint32_t)(it >> 1);
+        mbar_wait_or_abort(&acce[buf], (use & 1) ^ 1, abort_s, S.err);
+        tc_fence_after();
+        const uint32_t dt = tbase + buf * acc_stride;
+        const int c1 = min(KB, c0 + kc);
+        for (int kb = c0; kb < c1; ++kb) {
+          mbar_wait_or_abort(&full[stage], phase, abort_s, S.err);
           tc_fence_after();
-          const uint32_t dt = tbase + buf * acc_stride;
-          const int c1 = min(KB, c0 + kc);
-          for (int kb = c0; kb < c1; ++kb) {
-            if (!mbar_wait(&full[stage], phase)) { fail(S.err); ok = false; break; }
-            tc_fence_after();
-            const uint32_t sa = smem_base + stage * stage_bytes;
-            const uint32_t sb = sa + npa * a_bytes;
-            const int nks = kb + 1 < KB ? 4 : tail;
+          const uint32_t sa = smem_base + stage * stage_bytes;
+          const uint32_t sb = sa + npa * a_bytes;
+          const int nks = kb + 1 < KB ? 4 : tail;
+          if (elect_one()) {
             if (S.std_npc == 2) {
               issue_pairs<BN, 2>(dt, sa, sb, a_bytes, b_bytes, nks, kb != c0);
             } else if (S.std_npc == 3) {
@@ -340,12 +336,12 @@ __device__ __forceinline__ void umma_body(const Src& src) {
               }
             }
             umma_commit(&empty[stage]);
-            if (++stage == ST) { stage = 0; phase ^= 1; }
           }
-          if (!ok) break;
-          umma_commit(&accf[buf]);
+          __syncwarp();
+          if (++stage == ST) { stage = 0; phase ^= 1; }
         }
-        if (!ok) break;
+        if (elect_one()) umma_commit(&accf[buf]);
+        __syncwarp();
       }
     }
   } else {
@@ -356,8 +352,7 @@ __device__ __forceinline__ void umma_body(const Src& src) {
     float* srow = reinterpret_cast<float*>(escr) + row * (BN + 1);
     int it = 0, t = 0;
     uint32_t uses = 0;  // EG = 2: chunks drained from this group's buffer so far
-    bool ok = true;
-    for (int it_ = blockIdx.x; it_ < tiles && ok; it_ += gridDim.x, ++t) {
+    for (int it_ = blockIdx.x; it_ < tiles; it_ += gridDim.x, ++t) {
       if (EG > 1 && (t % EG) != eg) continue;
       int local;
       const UmmaParams<Epi>& P = src.entry(it_, local);
@@ -370,7 +365,7 @@ __device__ __forceinline__ void umma_body(const Src& src) {
       for (int ch = 0; ch < nch; ++ch, ++it) {
         const int buf = EG > 1 ? eg : (it & 1);
         const uint32_t use = EG > 1 ? uses++ : (uint32_t)(it >> 1);
-        if (!mbar_wait_abortable(&accf[buf], use & 1, abort_s)) { fail(S.err); ok = false; break; }
+        mbar_wait_or_abort(&accf[buf], use & 1, abort_s, S.err);
         tc_fence_after();
         const uint32_t taddr = tbase + ((uint32_t)(sub * 32) << 16) + buf * acc_stride;
         if (nch == 1) {
