@@ -25,6 +25,7 @@
 
 #include "afqmc_b200.h"
 #include "common.cuh"
+#include "exch_umma.cuh"
 #include "ops.h"
 #include "profile.cuh"
 #include "umma_gemm.cuh"
@@ -37,8 +38,6 @@ int make_tmap_bf16(CUtensorMap* map, const void* base, long long K, long long ro
 int sm_count();
 
 namespace {
-
-__device__ __forceinline__ void named_sync_epi() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 inline int pairs_for(int npc, int* pa, int* pb) {
   if (npc == 2) {
@@ -285,149 +284,6 @@ struct PropEpiU {
   }
 };
 
-struct ExchEpiU {
-  int G, no, W, gpt, wpt;
-  double* cout;    // (W, G) complex
-  double* excout;  // (mt, W) complex
-  // Per walker of the tile: stage f (gcount*No rows x 2No floats) in shared
-  // memory as (re, im) pairs, row stride exch_fs2(No) pairs (odd: 64-bit
-  // accesses by consecutive rows or consecutive pairs are bank-conflict free).
-  // Row (g, i) forms sum_j f[i][j] f[j][i] in four FP32 chains combined in
-  // FP64; the rows of one Cholesky vector are summed by a segmented shuffle
-  // reduction inside each warp plus at most three cross-warp partials, then
-  // the Cholesky vectors of the tile by a shuffle reduction in the first
-  // warp.  Every sum has a fixed order, so results are reproducible.
-  template <int BN>
-  __device__ void tile(int, int mti, int nti, int row, const AccSrc& src, const UmmaShape& s,
-                       uint8_t* smem) const {
-    const int nc = 2 * no, fs2 = exch_fs2(no);
-    float2* Fs = reinterpret_cast<float2*>(smem);
-    double4* pr = reinterpret_cast<double4*>(smem + exch_fs_bytes(no));
-    double2* ge = reinterpret_cast<double2*>(pr + 128);
-    const int g0 = mti * gpt, w0 = nti * wpt;
-    const int gcount = min(gpt, G - g0), wcount = min(wpt, W - w0);
-    const bool valid = row < gcount * no;
-    const int gl = row / no, i = row - (row / no) * no;
-    const int lane = row & 31;
-    const int seg = valid ? gl : -1;
-    for (int wl = 0; wl < wcount; ++wl) {
-      const int cb = wl * nc;  // even; chunk starts are multiples of 16, so pairs stay aligned
-      const int c_lo = cb & ~15, c_hi = (cb + nc + 15) & ~15;
-      for (int c = c_lo; c < c_hi; c += 16) {
-        float v[16];
-        src.load16(c, v);
-#pragma unroll
-        for (int k = 0; k < 16; k += 2) {
-          const int col = c + k - cb;
-          if (col >= 0 && col < nc) Fs[row * fs2 + (col >> 1)] = make_float2(v[k], v[k + 1]);
-        }
-      }
-      named_sync_epi();
-      double4 q = make_double4(0.0, 0.0, 0.0, 0.0);
-      if (valid) {
-        const float2* fr = Fs + row * fs2;
-        const float2* fc = Fs + (gl * no) * fs2 + i;
-        float ar[4] = {0.f, 0.f, 0.f, 0.f}, ai[4] = {0.f, 0.f, 0.f, 0.f};
-        int j = 0;
-        for (; j + 4 <= no; j += 4) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const float2 a = fr[j + u];
-            const float2 b = fc[(j + u) * fs2];
-            ar[u] = fmaf(a.x, b.x, fmaf(-a.y, b.y, ar[u]));
-            ai[u] = fmaf(a.x, b.y, fmaf(a.y, b.x, ai[u]));
-          }
-        }
-        for (; j < no; ++j) {
-          const float2 a = fr[j];
-          const float2 b = fc[j * fs2];
-          ar[0] = fmaf(a.x, b.x, fmaf(-a.y, b.y, ar[0]));
-          ai[0] = fmaf(a.x, b.y, fmaf(a.y, b.x, ai[0]));
-        }
-        const float2 d = fr[i];
-        q = make_double4(((double)ar[0] + (double)ar[1]) + ((double)ar[2] + (double)ar[3]),
-                         ((double)ai[0] + (double)ai[1]) + ((double)ai[2] + (double)ai[3]),
-                         (double)d.x, (double)d.y);
-      }
-      // suffix sums inside each run of equal `seg` within the warp
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const double tx = __shfl_down_sync(0xffffffffu, q.x, off);
-        const double ty = __shfl_down_sync(0xffffffffu, q.y, off);
-        const double tz = __shfl_down_sync(0xffffffffu, q.z, off);
-        const double tw = __shfl_down_sync(0xffffffffu, q.w, off);
-        const int st = __shfl_down_sync(0xffffffffu, seg, off);
-        if (lane + off < 32 && st == seg) {
-          q.x += tx;
-          q.y += ty;
-          q.z += tz;
-          q.w += tw;
-        }
-      }
-      const int sp = __shfl_up_sync(0xffffffffu, seg, 1);
-      if (valid && (lane == 0 || sp != seg)) pr[row] = q;  // run heads
-      named_sync_epi();
-      if (gcount <= 32) {
-        if (row < 32) {
-          double sr = 0.0, si = 0.0;
-          if (row < gcount) {
-            const int h = row * no;
-            double4 a = pr[h];
-            for (int r = (h / 32 + 1) * 32; r < h + no; r += 32) {
-              const double4 b = pr[r];
-              a.x += b.x;
-              a.y += b.y;
-              a.z += b.z;
-              a.w += b.w;
-            }
-            const long long co = 2 * ((long long)(w0 + wl) * G + g0 + row);
-            cout[co] = a.z;
-            cout[co + 1] = a.w;
-            sr = a.x;
-            si = a.y;
-          }
-#pragma unroll
-          for (int off = 16; off > 0; off >>= 1) {
-            sr += __shfl_down_sync(0xffffffffu, sr, off);
-            si += __shfl_down_sync(0xffffffffu, si, off);
-          }
-          if (row == 0) {
-            excout[2 * ((long long)mti * W + w0 + wl)] = sr;
-            excout[2 * ((long long)mti * W + w0 + wl) + 1] = si;
-          }
-        }
-      } else {  // more than 32 Cholesky vectors per tile (No < 4)
-        if (row < gcount) {
-          const int h = row * no;
-          double4 a = pr[h];
-          for (int r = (h / 32 + 1) * 32; r < h + no; r += 32) {
-            const double4 b = pr[r];
-            a.x += b.x;
-            a.y += b.y;
-            a.z += b.z;
-            a.w += b.w;
-          }
-          const long long co = 2 * ((long long)(w0 + wl) * G + g0 + row);
-          cout[co] = a.z;
-          cout[co + 1] = a.w;
-          ge[row] = make_double2(a.x, a.y);
-        }
-        named_sync_epi();
-        if (row == 0) {
-          double sx = 0, sy = 0;
-          for (int g = 0; g < gcount; ++g) {
-            sx += ge[g].x;
-            sy += ge[g].y;
-          }
-          excout[2 * ((long long)mti * W + w0 + wl)] = sx;
-          excout[2 * ((long long)mti * W + w0 + wl) + 1] = sy;
-        }
-      }
-    }
-  }
-  static size_t smem_extra(int no) { return exch_epi_extra(no); }
-};
-
 // ---------------------------------------------------------------------------
 // host helpers
 // ---------------------------------------------------------------------------
@@ -565,33 +421,66 @@ int prop_launch(const Layout& L, const double* prep, double* work, int s, int nc
   return run<BN, 1>(P, ex, st, K_PROP, L.tune);
 }
 
+template <class Kernel>
+int exch_run(Kernel kernel, int threads, const ExchParams& P, size_t smem, int ctas, cudaStream_t st) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return AFQ_ERR_CUDA;
+  const long long tiles = (long long)P.mt * P.nt;
+  ProfScope ps(K_EXCH, st);
+  kernel<<<(int)(tiles < ctas ? tiles : ctas), threads, smem, st>>>(P);
+  return cudaGetLastError() == cudaSuccess ? AFQ_OK : AFQ_ERR_CUDA;
+}
+
 template <int BN>
 int exch_launch(const Layout& L, const double* prep, double* work, int s, cudaStream_t st) {
   const UExchTile& X = L.uex[s];
   const int no = L.no[s];
-  UmmaParams<ExchEpiU> P{};
+  ExchParams P{};
   bf16* a[3];
   bf16* b[3];
   piece_ptrs(const_cast<double*>(prep), L.q_rc[s], L.q_rc_ps[s], L.npc, a);
   piece_ptrs(work, L.v_gt[s], L.v_gt_ps[s], L.npc, b);
   const long long arows = (long long)L.G * no, brows = (long long)L.W * 2 * no;
-  int rc = setup_maps(P, a, L.npc, L.N, arows, 1, L.Nb, arows * L.Nb, b, L.npc, L.N, brows, 1,
-                      L.Nb, brows * L.Nb, BN);
-  if (rc != AFQ_OK) return rc;
-  base_shape(P, L.npc, (int)arows, (int)brows, L.N, 1, BN, err_flag(L, work));
-  P.s.ngroups = 2;  // hi x hi products apart from the cross terms: shorter rounding chains
-  P.s.a_step = X.gpt * no;
-  P.s.b_step = X.wpt * 2 * no;
-  P.s.mt = X.mt;
-  P.s.nt = (L.W + X.wpt - 1) / X.wpt;
-  P.epi.G = L.G;
-  P.epi.no = no;
-  P.epi.W = L.W;
-  P.epi.gpt = X.gpt;
-  P.epi.wpt = X.wpt;
-  P.epi.cout = work + L.w_c[s];
-  P.epi.excout = work + L.w_exc[s];
-  return run<BN>(P, ExchEpiU::smem_extra(no), st, K_EXCH, L.tune);
+  P.arows = (X.gpt * no + 7) & ~7;
+  P.brows = (X.wpt * 2 * no + 7) & ~7;
+  for (int i = 0; i < L.npc; ++i) {
+    int rc = make_tmap_bf16(&P.ta[i], a[i], L.N, arows, 1, L.Nb, arows * L.Nb, P.arows);
+    if (rc != AFQ_OK) return rc;
+    rc = make_tmap_bf16(&P.tb[i], b[i], L.N, brows, 1, L.Nb, brows * L.Nb, P.brows);
+    if (rc != AFQ_OK) return rc;
+  }
+  P.npc = L.npc;
+  P.G = L.G;
+  P.no = no;
+  P.W = L.W;
+  P.K = L.N;
+  P.gpt = X.gpt;
+  P.wpt = X.wpt;
+  P.mt = X.mt;
+  P.nt = (L.W + X.wpt - 1) / X.wpt;
+  if ((long long)P.mt * P.nt >= (1LL << 31) - 65536) return AFQ_ERR_SHAPE;
+  // walkers per pass over the row tiles: their operand pieces take at most
+  // 32 MB, a quarter of the L2, next to the row operand that streams through
+  const long long wbytes = (long long)X.wpt * 2 * no * L.Nb * 2 * L.npc;
+  const long long ncw = (32LL << 20) / wbytes;
+  P.ncw = ncw < 1 ? 1 : (ncw > P.nt ? P.nt : (int)ncw);
+  const ExchPlan plan = exch_plan(L.npc, no, L.N, X, P.arows, P.brows, L.tune.max_stages);
+  if (plan.stages < 2) return AFQ_ERR_SHAPE;
+  P.stages = plan.stages;
+  P.gsub = plan.gsub;
+  P.lot = plan.lot;
+  for (int i = 0; i < 2; ++i) P.a[i] = a[i];
+  P.lda = L.Nb;
+  P.cout = reinterpret_cast<float4*>(work + L.w_c[s]);
+  P.excout = reinterpret_cast<float4*>(work + L.w_exc[s]);
+  P.err = err_flag(L, work);
+  int ctas = sm_count();
+  if (L.tune.grid_cap > 0 && L.tune.grid_cap < ctas) ctas = L.tune.grid_cap;
+  if (plan.ts)
+    return plan.nbuf == 2 ? exch_run(umma_exch_ts_kernel<BN, (BN <= 96 ? 2 : 1)>, kExchThreads, P, plan.smem, ctas, st)
+                          : exch_run(umma_exch_ts_kernel<BN, 1>, kExchThreads, P, plan.smem, ctas, st);
+  return L.npc == 2 ? exch_run(umma_exch_kernel<BN, 2>, kExchThreads, P, plan.smem, ctas, st)
+                    : exch_run(umma_exch_kernel<BN, 3>, kExchThreads, P, plan.smem, ctas, st);
 }
 
 }  // namespace
