@@ -83,9 +83,12 @@ static __device__ __noinline__ void mbar_wait_slow(uint64_t* bar, uint32_t parit
   atomicExch(err, 1);
   *abort = 1;
 }
+// Called by whole warps: the lanes meet again before the .aligned instructions
+// that follow (a lane may see the barrier complete while its neighbour polls on).
 __device__ __forceinline__ void mbar_wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort,
                                                    int* err) {
   if (!mbar_try_wait(bar, parity)) mbar_wait_slow(bar, parity, abort, err);
+  __syncwarp();
 }
 
 // true in one lane of the (converged) warp
