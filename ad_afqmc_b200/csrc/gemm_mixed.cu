@@ -106,6 +106,22 @@ int make_tmap_bf16(CUtensorMap* map, const void* base, long long K, long long ro
   return r == CUDA_SUCCESS ? AFQ_OK : AFQ_ERR_ARG;
 }
 
+// declared in f64_tma.cuh
+int make_tmap_f64(CUtensorMap* map, const void* base, long long x, long long y, long long z,
+                  long long ystride, long long zstride, int bx, int by) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return AFQ_ERR_CUDA;
+  if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0 || (ystride & 1) || (zstride & 1)) return AFQ_ERR_ALIGN;
+  cuuint64_t dims[3] = {(cuuint64_t)x, (cuuint64_t)y, (cuuint64_t)z};
+  cuuint64_t strides[2] = {(cuuint64_t)ystride * 8, (cuuint64_t)zstride * 8};
+  cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, bx == 16 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? AFQ_OK : AFQ_ERR_ARG;
+}
+
 cudaError_t launch_split(const double* x, long long n, int np, void* o0, void* o1, void* o2,
                          cudaStream_t st) {
   long long blocks = (n + 255) / 256;

@@ -11,50 +11,38 @@
 //               fused: f lives only in registers/shared memory
 //               (wavefunctions.py:1128-1174, 1331-1363)
 #include "common.cuh"
-#include "gemm_f64.cuh"
+#include "f64_tma.cuh"
 #include "ops.h"
 #include "profile.cuh"
 
 namespace afq {
 
+int sm_count();
+
 namespace {
 
-constexpr int kUnseg = 1 << 30;
-
-using CfgBig = F64Cfg<4, 8, 4, 2>;   // 128 x 128, 8 warps
-using CfgP32 = F64Cfg<2, 2, 2, 2>;   // 32 x 32,  4 warps
-using CfgP80 = F64Cfg<5, 5, 1, 2>;   // 40 x 80,  2 warps
-using CfgP120 = F64Cfg<5, 5, 1, 3>;  // 40 x 120, 3 warps
-using CfgX80 = F64Cfg<5, 5, 3, 2>;   // 120 x 80,  6 warps (exchange)
-using CfgX120 = F64Cfg<5, 5, 3, 3>;  // 120 x 120, 9 warps (exchange)
-using CfgX160 = F64Cfg<4, 5, 4, 4>;  // 128 x 160, 16 warps (exchange, No > 60)
-
-template <class Cfg>
-cudaError_t set_smem(const void* fn, size_t bytes) {
-  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
+constexpr int kPlain = 1 << 20;  // column groups of a plain (not per-walker) operand
 
 // ---------------------------------------------------------------------------
 // force bias: C[z] (2W x G) = Gpl (2W x Kfb) * RCcat^T, K split over z
 // ---------------------------------------------------------------------------
-template <class Cfg>
-__global__ void __launch_bounds__(Cfg::NT) fb_gemm_kernel(F64Operand A, F64Operand B, int M,
-                                                          int N, int K, int kchunk, double* C,
-                                                          long long ldc, long long zstride) {
-  extern __shared__ double smem[];
-  const int m0 = blockIdx.x * Cfg::BM, n0 = blockIdx.y * Cfg::BN, z = blockIdx.z;
-  const int kb = z * kchunk, ke = min(K, kb + kchunk);
-  double acc[Cfg::FM][Cfg::FN][2];
-  f64_zero<Cfg>(acc);
-  f64_mainloop<Cfg, B_NMAJOR>(acc, A, B, M, N, kb, ke, m0, n0, 0, false, smem);
-  double* Cz = C + (long long)z * zstride;
-  f64_foreach<Cfg>(acc, m0, n0, [&](int m, int n, double v0, double v1) {
-    if (m < M) {
-      if (n < N) Cz[(long long)m * ldc + n] = v0;
-      if (n + 1 < N) Cz[(long long)m * ldc + n + 1] = v1;
-    }
-  });
-}
+struct FbEpi {
+  double* C;
+  long long ldc, zstride;
+  int M, N;
+  template <class T>
+  __device__ void tile(const F64At& at, double (&acc)[T::FM][T::NG][2][2], int wm, int wn, int g, int t4,
+                       uint8_t*) const {
+    double* const Cz = C + at.z * zstride;
+    f64_each<T>(acc, wm, wn, g, t4, [&](int r, int c, double v0, double v1, double v2, double v3) {
+      const int m = at.mti * T::BM + r, n = at.nti * T::BN + c;
+      if (m >= M) return;
+      double* p = Cz + m * ldc + n;  // ldc even, n even: pairs are aligned, the pad column is never read
+      if (n < N) *reinterpret_cast<double2*>(p) = make_double2(v0, v1);
+      if (n + 8 < N) *reinterpret_cast<double2*>(p + 8) = make_double2(v2, v3);
+    });
+  }
+};
 
 // ---------------------------------------------------------------------------
 // field preparation (one CTA per walker)
@@ -149,144 +137,160 @@ __global__ void __launch_bounds__(256) prep_kernel_grouped(const PrepArgs* A, Bl
 // ---------------------------------------------------------------------------
 // VHS: C (2W x N*N) = Xt (2W x G) * chol (G x N*N), scattered to (W, N, 2Npad)
 // ---------------------------------------------------------------------------
-template <class Cfg>
-__global__ void __launch_bounds__(Cfg::NT) vhs_gemm_kernel(F64Operand A, F64Operand B, int M,
-                                                           int NN, int K, int N, long long Npad,
-                                                           double* vhs) {
-  extern __shared__ double smem[];
-  const int m0 = blockIdx.x * Cfg::BM, n0 = blockIdx.y * Cfg::BN;
-  double acc[Cfg::FM][Cfg::FN][2];
-  f64_zero<Cfg>(acc);
-  f64_mainloop<Cfg, B_KMAJOR>(acc, A, B, M, NN, 0, K, m0, n0, 0, false, smem);
-  const long long ld = 2 * Npad;
-  f64_foreach<Cfg>(acc, m0, n0, [&](int m, int n, double v0, double v1) {
-    if (m >= M) return;
-    const int w = m >> 1, c = m & 1;
-    double* base = vhs + (long long)w * N * ld + c * Npad;
-    if (n < NN) {
-      const int p = n / N, r = n - p * N;
-      base[(long long)p * ld + r] = v0;
-    }
-    if (n + 1 < NN) {
-      const int p = (n + 1) / N, r = (n + 1) - p * N;
-      base[(long long)p * ld + r] = v1;
-    }
-  });
-}
-
-// ---------------------------------------------------------------------------
-// batched per-walker GEMM for the one-body half-steps and the Taylor chain
-//   mode 0: out = A*B
-//   mode 1: t = s*(A*B); out = t; acc = yin + t
-//   mode 2: t = s*(A*B); out = t; acc += t
-//   mode 3: t = s*(A*B);           acc += t
-// nseg == 2 adds A2 * rot(B) (imaginary part of a complex A).
-// ---------------------------------------------------------------------------
-struct PropEpi {
-  int mode;
-  double scale;
-  double* out;
-  const double* yin;
-  double* acc;
-  long long ld, bstride;
+struct VhsEpi {
+  double* vhs;
+  int M, NN, N;
+  long long Npad;
+  template <class T>
+  __device__ void tile(const F64At& at, double (&acc)[T::FM][T::NG][2][2], int wm, int wn, int g, int t4,
+                       uint8_t*) const {
+    const long long ld = 2 * Npad;
+    const int n_ = N;
+    f64_each<T>(acc, wm, wn, g, t4, [&](int row, int c, double v0, double v1, double v2, double v3) {
+      const int m = at.mti * T::BM + row, n = at.nti * T::BN + c;
+      if (m >= M || n >= NN) return;
+      double* base = vhs + (long long)(m >> 1) * n_ * ld + (m & 1) * Npad;
+      int p = n / n_, r = n - p * n_;
+      const double v[4] = {v0, v1, v2, v3};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (n + q < NN) base[(long long)p * ld + r] = v[q];
+        if (++r == n_) { r = 0; ++p; }
+      }
+    });
+  }
 };
 
-template <class Cfg>
-__global__ void __launch_bounds__(Cfg::NT) prop_gemm_kernel(F64Operand A1, F64Operand A2,
-                                                            F64Operand B, int M, int N, int K,
-                                                            int nseg, PropEpi e) {
-  extern __shared__ double smem[];
-  const int m0 = blockIdx.x * Cfg::BM, n0 = blockIdx.y * Cfg::BN, b = blockIdx.z;
-  double acc[Cfg::FM][Cfg::FN][2];
-  f64_zero<Cfg>(acc);
-  f64_mainloop<Cfg, B_KMAJOR>(acc, A1, B, M, N, 0, K, m0, n0, b, false, smem);
-  if (nseg == 2) f64_mainloop<Cfg, B_KMAJOR>(acc, A2, B, M, N, 0, K, m0, n0, b, true, smem);
-  const long long boff = (long long)b * e.bstride;
-  f64_foreach<Cfg>(acc, m0, n0, [&](int m, int n, double v0, double v1) {
-    if (m >= M) return;
-    const long long o = boff + (long long)m * e.ld + n;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      if (n + q >= N) break;
-      const double v = q ? v1 : v0;
-      if (e.mode == 0) {
-        e.out[o + q] = v;
-      } else {
-        const double tv = v * e.scale;
-        if (e.mode != 3) e.out[o + q] = tv;
-        if (e.mode == 1)
-          e.acc[o + q] = e.yin[o + q] + tv;
-        else
-          e.acc[o + q] += tv;
+// ---------------------------------------------------------------------------
+// batched per-walker products of the one-body half-steps and the Taylor series
+// (Horner: z_{n-1} = y + VHS z_n / n):  out = (yin) + scale * A B
+// ---------------------------------------------------------------------------
+struct PropEpi {
+  double* out;
+  const double* yin;  // nullptr: none
+  double scale;
+  int M, nc;
+  template <class T>
+  __device__ void tile(const F64At& at, double (&acc)[T::FM][T::NG][2][2], int wm, int wn, int g, int t4,
+                       uint8_t*) const {
+    const long long boff = (long long)at.z * M * nc;
+    const double s = scale;
+    const double* const y = yin ? yin + boff : nullptr;
+    double* const o = out + boff;
+    const int M_ = M, n_ = nc;
+    f64_each<T>(acc, wm, wn, g, t4, [&](int row, int c, double v0, double v1, double v2, double v3) {
+      const int m = at.mti * T::BM + row, n = at.nti * T::BN + c;
+      if (m >= M_ || n >= n_) return;
+      const long long e = (long long)m * n_ + n;
+      double2 u = make_double2(s * v0, s * v1), w = make_double2(s * v2, s * v3);
+      const bool two = n + 2 < n_;  // nc is even
+      if (y) {
+        const double2 y0 = *reinterpret_cast<const double2*>(y + e);
+        u = make_double2(y0.x + u.x, y0.y + u.y);
+        if (two) {
+          const double2 y1 = *reinterpret_cast<const double2*>(y + e + 2);
+          w = make_double2(y1.x + w.x, y1.y + w.y);
+        }
       }
-    }
+      *reinterpret_cast<double2*>(o + e) = u;
+      if (two) *reinterpret_cast<double2*>(o + e + 2) = w;
+    });
+  }
+};
+
+template <class T>
+__device__ __forceinline__ void f64_consumer_sync() {
+  asm volatile("bar.sync 1, %0;" ::"n"(32 * T::CW) : "memory");
+}
+
+// The tile of f in shared memory: rows (Cholesky vector, i), a walker's columns
+// at a stride of 16 gpw doubles; row stride BN + 2 doubles, so that 16-byte loads
+// down a column (4 banks apart) and along a row are conflict-free.
+template <class T>
+__device__ __forceinline__ double* exch_stage(double (&acc)[T::FM][T::NG][2][2], int wm, int wn, int g, int t4,
+                                              uint8_t* smem) {
+  constexpr int CS = T::BN + 2;
+  double* Ct = reinterpret_cast<double*>(smem);
+  f64_each<T>(acc, wm, wn, g, t4, [&](int row, int c, double v0, double v1, double v2, double v3) {
+    double2* p = reinterpret_cast<double2*>(Ct + row * CS + c);
+    p[0] = make_double2(v0, v1);
+    p[1] = make_double2(v2, v3);
   });
+  f64_consumer_sync<T>();
+  return Ct;
+}
+template <class T>
+inline size_t exch_stage_bytes(int extra) {
+  return size_t(T::BM) * (T::BN + 2) * 8 + size_t(extra) * 8;
 }
 
 // ---------------------------------------------------------------------------
-// fused exchange: tile = gpt Cholesky vectors x wpt walkers
+// fused exchange: tile = gpt Cholesky vectors x wpt walkers.  Per block (g, w):
+// tr f and sum_ij f_ij f_ji = sum_i f_ii^2 + 2 sum_{i<j} f_ij f_ji, rows dealt to
+// the warps of the block.
 // ---------------------------------------------------------------------------
-template <class Cfg>
-__global__ void __launch_bounds__(Cfg::NT) exch_kernel(F64Operand A, F64Operand B, int G, int no,
-                                                       int N, int W, int gpt, int wpt,
-                                                       double* cout, double* excout) {
-  extern __shared__ double smem[];
-  const int mt = blockIdx.x, nt = blockIdx.y;
-  const int g0 = mt * gpt, w0 = nt * wpt;
-  const int gcount = min(gpt, G - g0), wcount = min(wpt, W - w0);
-  const int m0 = g0 * no, n0 = w0 * 2 * no;
-  const int M_lim = (g0 + gcount) * no, N_lim = (w0 + wcount) * 2 * no;
-  double acc[Cfg::FM][Cfg::FN][2];
-  f64_zero<Cfg>(acc);
-  f64_mainloop<Cfg, B_KMAJOR>(acc, A, B, M_lim, N_lim, 0, N, m0, n0, 0, false, smem);
-
-  constexpr int CS = Cfg::BN + 2;  // staged tile row stride (doubles)
-  double* Ct = smem;
-  double2* blk = reinterpret_cast<double2*>(smem + Cfg::BM * CS);
-  f64_foreach<Cfg>(acc, 0, 0, [&](int m, int n, double v0, double v1) {
-    *reinterpret_cast<double2*>(Ct + m * CS + n) = make_double2(v0, v1);
-  });
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = Cfg::NT / 32;
-  const int nblk = gcount * wcount;
-  for (int bi = warp; bi < nblk; bi += nwarps) {
-    const int gl = bi % gcount, wl = bi / gcount;
-    const double* F = Ct + gl * no * CS + wl * 2 * no;
-    double er = 0, ei = 0, cr = 0, ci = 0;
-    for (int e = lane; e < no * no; e += 32) {
-      const int i = e / no, j = e - (e / no) * no;
-      const double2 fij = *reinterpret_cast<const double2*>(F + i * CS + 2 * j);
-      const double2 fji = *reinterpret_cast<const double2*>(F + j * CS + 2 * i);
-      er += fij.x * fji.x - fij.y * fji.y;
-      ei += fij.x * fji.y + fij.y * fji.x;
-      if (i == j) {
-        cr += fij.x;
-        ci += fij.y;
+struct ExchEpi {
+  int G, no, W, gpt, wpt, gpw;
+  double* cout;
+  double* excout;
+  template <class T>
+  __device__ void tile(const F64At& at, double (&acc)[T::FM][T::NG][2][2], int wm, int wn, int g, int t4,
+                       uint8_t* smem) const {
+    constexpr int CS = T::BN + 2, CW = T::CW;
+    const double* Ct = exch_stage<T>(acc, wm, wn, g, t4, smem);
+    double4* blk = reinterpret_cast<double4*>(smem + size_t(T::BM) * CS * 8);  // [CW or more][block]
+    const int g0 = at.mti * gpt, w0 = at.nti * wpt;
+    const int gcount = min(gpt, G - g0), wcount = min(wpt, W - w0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nblk = gcount * wcount, parts = max(1, CW / nblk);
+    for (int e = warp; e < nblk * parts; e += CW) {
+      const int b = e / parts, part = e - b * parts;
+      const int gl = b % gcount, wl = b / gcount;
+      const double* F = Ct + gl * no * CS + wl * 16 * gpw;
+      double er = 0, ei = 0, dr = 0, di = 0, cr = 0, ci = 0;
+      for (int i = part; i < no; i += parts)
+        for (int j = i + lane; j < no; j += 32) {
+          const double2 fij = *reinterpret_cast<const double2*>(F + i * CS + 2 * j);
+          const double2 fji = *reinterpret_cast<const double2*>(F + j * CS + 2 * i);
+          if (j == i) {
+            dr += fij.x * fij.x - fij.y * fij.y;
+            di += 2.0 * fij.x * fij.y;
+            cr += fij.x;
+            ci += fij.y;
+          } else {
+            er += fij.x * fji.x - fij.y * fji.y;
+            ei += fij.x * fji.y + fij.y * fji.x;
+          }
+        }
+      er = warp_sum(dr + 2.0 * er);
+      ei = warp_sum(di + 2.0 * ei);
+      cr = warp_sum(cr);
+      ci = warp_sum(ci);
+      if (lane == 0) blk[e] = make_double4(er, ei, cr, ci);
+    }
+    f64_consumer_sync<T>();
+    for (int b = threadIdx.x; b < nblk; b += 32 * CW) {
+      double4 s = blk[b * parts];
+      for (int q = 1; q < parts; ++q) {
+        const double4 u = blk[b * parts + q];
+        s.x += u.x; s.y += u.y; s.z += u.z; s.w += u.w;
       }
+      const long long co = 2 * ((long long)(w0 + b / gcount) * G + g0 + b % gcount);
+      cout[co] = s.z;
+      cout[co + 1] = s.w;
     }
-    er = warp_sum(er);
-    ei = warp_sum(ei);
-    cr = warp_sum(cr);
-    ci = warp_sum(ci);
-    if (lane == 0) {
-      const long long co = 2 * ((long long)(w0 + wl) * G + g0 + gl);
-      cout[co] = cr;
-      cout[co + 1] = ci;
-      blk[gl * wpt + wl] = make_double2(er, ei);
+    for (int wl = threadIdx.x; wl < wcount; wl += 32 * CW) {
+      double sx = 0, sy = 0;
+      for (int e = wl * gcount * parts; e < (wl + 1) * gcount * parts; ++e) {
+        sx += blk[e].x;
+        sy += blk[e].y;
+      }
+      excout[2 * ((long long)at.mti * W + w0 + wl)] = sx;
+      excout[2 * ((long long)at.mti * W + w0 + wl) + 1] = sy;
     }
+    f64_consumer_sync<T>();
   }
-  __syncthreads();
-  for (int wl = threadIdx.x; wl < wcount; wl += Cfg::NT) {
-    double sx = 0, sy = 0;
-    for (int gl = 0; gl < gcount; ++gl) {
-      const double2 v = blk[gl * wpt + wl];
-      sx += v.x;
-      sy += v.y;
-    }
-    excout[2 * ((long long)mt * W + w0 + wl)] = sx;
-    excout[2 * ((long long)mt * W + w0 + wl) + 1] = sy;
-  }
-}
+};
 
 // ---------------------------------------------------------------------------
 // LNO orbital energy (rhf_lno._calc_orbenergy, wavefunctions.py:6904-6923):
@@ -298,76 +302,71 @@ __global__ void __launch_bounds__(Cfg::NT) exch_kernel(F64Operand A, F64Operand 
 // ---------------------------------------------------------------------------
 constexpr int kMaxLo = 8;
 
-template <class Cfg>
-__global__ void __launch_bounds__(Cfg::NT) orb_kernel(F64Operand A, F64Operand B, int G, int no,
-                                                      int N, int W, int gpt, int wpt,
-                                                      const double* prj, int nlo, double* orbout) {
-  extern __shared__ double smem[];
-  const int mt = blockIdx.x, nt = blockIdx.y;
-  const int g0 = mt * gpt, w0 = nt * wpt;
-  const int gcount = min(gpt, G - g0), wcount = min(wpt, W - w0);
-  const int m0 = g0 * no, n0 = w0 * 2 * no;
-  const int M_lim = (g0 + gcount) * no, N_lim = (w0 + wcount) * 2 * no;
-  double acc[Cfg::FM][Cfg::FN][2];
-  f64_zero<Cfg>(acc);
-  f64_mainloop<Cfg, B_KMAJOR>(acc, A, B, M_lim, N_lim, 0, N, m0, n0, 0, false, smem);
-
-  constexpr int CS = Cfg::BN + 2;
-  double* Ct = smem;
-  double* P = smem + Cfg::BM * CS;  // nlo x no projector rows
-  double2* blk = reinterpret_cast<double2*>(P + kMaxLo * 64);
-  f64_foreach<Cfg>(acc, 0, 0, [&](int m, int n, double v0, double v1) {
-    *reinterpret_cast<double2*>(Ct + m * CS + n) = make_double2(v0, v1);
-  });
-  for (int e = threadIdx.x; e < nlo * no; e += Cfg::NT) P[e] = prj[e];
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = Cfg::NT / 32;
-  const int nblk = gcount * wcount;
-  for (int bi = warp; bi < nblk; bi += nwarps) {
-    const int gl = bi % gcount, wl = bi / gcount;
-    const double* F = Ct + gl * no * CS + wl * 2 * no;
-    double cr = 0, ci = 0, ar = 0, ai = 0, br = 0, bi_ = 0;
-    for (int k = lane; k < no; k += 32) {
-      cr += F[k * CS + 2 * k];
-      ci += F[k * CS + 2 * k + 1];
-    }
-    for (int r = 0; r < nlo; ++r) {
-      const double* p = P + r * no;
+struct OrbEpi {
+  int G, no, W, gpt, wpt, gpw, nlo;
+  const double* prj;
+  double* orbout;
+  template <class T>
+  __device__ void tile(const F64At& at, double (&acc)[T::FM][T::NG][2][2], int wm, int wn, int g, int t4,
+                       uint8_t* smem) const {
+    constexpr int CS = T::BN + 2, CW = T::CW;
+    double* P = reinterpret_cast<double*>(smem) + T::BM * CS;  // nlo x no projector rows
+    double2* blk = reinterpret_cast<double2*>(P + kMaxLo * 64);
+    for (int e = threadIdx.x; e < nlo * no; e += 32 * CW) P[e] = prj[e];
+    const double* Ct = exch_stage<T>(acc, wm, wn, g, t4, smem);
+    const int g0 = at.mti * gpt, w0 = at.nti * wpt;
+    const int gcount = min(gpt, G - g0), wcount = min(wpt, W - w0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nblk = gcount * wcount;
+    for (int bi = warp; bi < nblk; bi += CW) {
+      const int gl = bi % gcount, wl = bi / gcount;
+      const double* F = Ct + gl * no * CS + wl * 16 * gpw;
+      double cr = 0, ci = 0, ar = 0, ai = 0, br = 0, bi_ = 0;
       for (int k = lane; k < no; k += 32) {
-        double ur = 0, ui = 0, vr = 0, vi = 0;  // u = (p f)[k], v = (f p^T)[k]
-        for (int x = 0; x < no; ++x) {
-          ur = fma(p[x], F[x * CS + 2 * k], ur);
-          ui = fma(p[x], F[x * CS + 2 * k + 1], ui);
-          vr = fma(F[k * CS + 2 * x], p[x], vr);
-          vi = fma(F[k * CS + 2 * x + 1], p[x], vi);
-        }
-        ar = fma(ur, p[k], ar);
-        ai = fma(ui, p[k], ai);
-        br += ur * vr - ui * vi;
-        bi_ += ur * vi + ui * vr;
+        cr += F[k * CS + 2 * k];
+        ci += F[k * CS + 2 * k + 1];
       }
+      for (int r = 0; r < nlo; ++r) {
+        const double* p = P + r * no;
+        for (int k = lane; k < no; k += 32) {
+          double ur = 0, ui = 0, vr = 0, vi = 0;  // u = (p f)[k], v = (f p^T)[k]
+          for (int x = 0; x < no; ++x) {
+            const double2 fu = *reinterpret_cast<const double2*>(F + x * CS + 2 * k);
+            const double2 fv = *reinterpret_cast<const double2*>(F + k * CS + 2 * x);
+            ur = fma(p[x], fu.x, ur);
+            ui = fma(p[x], fu.y, ui);
+            vr = fma(fv.x, p[x], vr);
+            vi = fma(fv.y, p[x], vi);
+          }
+          ar = fma(ur, p[k], ar);
+          ai = fma(ui, p[k], ai);
+          br += ur * vr - ui * vi;
+          bi_ += ur * vi + ui * vr;
+        }
+      }
+      cr = warp_sum(cr);
+      ci = warp_sum(ci);
+      ar = warp_sum(ar);
+      ai = warp_sum(ai);
+      br = warp_sum(br);
+      bi_ = warp_sum(bi_);
+      if (lane == 0)  // 2 c s1 - s2
+        blk[gl * wpt + wl] = make_double2(2.0 * (cr * ar - ci * ai) - br, 2.0 * (cr * ai + ci * ar) - bi_);
     }
-    cr = warp_sum(cr);
-    ci = warp_sum(ci);
-    ar = warp_sum(ar);
-    ai = warp_sum(ai);
-    br = warp_sum(br);
-    bi_ = warp_sum(bi_);
-    if (lane == 0)  // 2 c s1 - s2
-      blk[gl * wpt + wl] = make_double2(2.0 * (cr * ar - ci * ai) - br, 2.0 * (cr * ai + ci * ar) - bi_);
-  }
-  __syncthreads();
-  for (int wl = threadIdx.x; wl < wcount; wl += Cfg::NT) {
-    double sx = 0, sy = 0;
-    for (int gl = 0; gl < gcount; ++gl) {
-      const double2 v = blk[gl * wpt + wl];
-      sx += v.x;
-      sy += v.y;
+    f64_consumer_sync<T>();
+    for (int wl = threadIdx.x; wl < wcount; wl += 32 * CW) {
+      double sx = 0, sy = 0;
+      for (int gl = 0; gl < gcount; ++gl) {
+        const double2 v = blk[gl * wpt + wl];
+        sx += v.x;
+        sy += v.y;
+      }
+      orbout[2 * ((long long)at.mti * W + w0 + wl)] = sx;
+      orbout[2 * ((long long)at.mti * W + w0 + wl) + 1] = sy;
     }
-    orbout[2 * ((long long)mt * W + w0 + wl)] = sx;
-    orbout[2 * ((long long)mt * W + w0 + wl) + 1] = sy;
+    f64_consumer_sync<T>();
   }
-}
+};
 
 // Theta (W, N, No) complex: rows p < No set to zero (the occupied block)
 __global__ void theta_zero_occ_kernel(double2* theta, int W, int N, int no) {
@@ -455,42 +454,179 @@ __global__ void energy_combine_kernel(int W, int G, int ns, int restricted, cons
   }
 }
 
-template <class Cfg>
-cudaError_t run_prop(const F64Operand& A1, const F64Operand& A2, const F64Operand& B, int M,
-                     int N, int K, int nseg, int batch, const PropEpi& e, cudaStream_t st) {
-  cudaError_t err = set_smem<Cfg>((const void*)prop_gemm_kernel<Cfg>, Cfg::SMEM);
-  if (err != cudaSuccess) return err;
-  dim3 grid((M + Cfg::BM - 1) / Cfg::BM, (N + Cfg::BN - 1) / Cfg::BN, batch);
-  ProfScope ps(K_PROP, st);
-  prop_gemm_kernel<Cfg><<<grid, Cfg::NT, Cfg::SMEM, st>>>(A1, A2, B, M, N, K, nseg, e);
-  return cudaGetLastError();
+// Tile of the two plain contractions (force bias, VHS): from 128 x 128 (8 warps,
+// 32 x 64 each) down to 32 x 32, whichever gives the shortest sum of waves; a tile
+// costs its MMAs per warp (FM NG) and about 1.5 for its loads and stores.  A
+// wave of big tiles that leaves SMs idle loses to more waves of smaller ones
+// (N = 95, G = 471, 161 walkers, force bias: 64 x 64 tiles).
+template <int BMODE, class F>
+cudaError_t with_gemm_tile(long long M, long long N, int nz, F&& f) {
+  const int fm[5] = {4, 2, 2, 1, 1}, ng[5] = {4, 4, 2, 2, 1}, sms = sm_count();
+  int best = 0;
+  double cost = 1e300;
+  for (int i = 0; i < 5; ++i) {
+    const long long tiles = ((M + 32 * fm[i] - 1) / (32 * fm[i])) * ((N + 32 * ng[i] - 1) / (32 * ng[i])) * nz;
+    const double c = double((tiles + sms - 1) / sms) * (fm[i] * ng[i] + 1.5);
+    if (c < cost - 1e-9) { cost = c; best = i; }
+  }
+  switch (best) {
+    case 0: return f(F64Tile<4, 2, 4, F64_REAL, BMODE>());
+    case 1: return f(F64Tile<2, 2, 4, F64_REAL, BMODE>());
+    case 2: return f(F64Tile<2, 2, 2, F64_REAL, BMODE>());
+    case 3: return f(F64Tile<1, 2, 2, F64_REAL, BMODE>());
+    default: return f(F64Tile<1, 2, 1, F64_REAL, BMODE>());
+  }
 }
 
-cudaError_t prop_gemm(const F64Operand& A1, const F64Operand& A2, const F64Operand& B, int M,
-                      int N, int K, int nseg, int batch, const PropEpi& e, cudaStream_t st) {
-  if (N <= 32) return run_prop<CfgP32>(A1, A2, B, M, N, K, nseg, batch, e, st);
-  if (N <= 80) return run_prop<CfgP80>(A1, A2, B, M, N, K, nseg, batch, e, st);
-  return run_prop<CfgP120>(A1, A2, B, M, N, K, nseg, batch, e, st);
+int* f64_err(const Layout& L, double* work) { return reinterpret_cast<int*>(work + L.w_misc); }
+
+// CTAs for a persistent launch of a kernel of `threads` threads and tiles of
+// shared memory `smem`: small tiles share an SM
+int f64_ctas(int threads, size_t smem) {
+  int per = (int)(kF64SmemBudget / (smem ? smem : 1));
+  const int byt = 1024 / threads;
+  if (per > byt) per = byt;
+  return sm_count() * (per < 1 ? 1 : (per > 3 ? 3 : per));
+}
+
+struct PropCall {
+  const double *a1, *a2;  // A (second: imaginary part), row stride lda, batch stride abs (0: shared)
+  long long lda, abs;
+  const double* b;        // (W, N, nc)
+  double* out;
+  const double* yin;
+  double scale;
+};
+
+template <int FM, int WN, int KIND>
+cudaError_t prop_run(const Layout& L, double* work, int nc, const PropCall& c, cudaStream_t st) {
+  using T = F64Tile<FM, WN, 1, KIND, F64_B_N>;
+  F64Params<PropEpi> P{};
+  const int N = L.N, W = L.W;
+  const int nb = c.abs ? W : 1;
+  if (make_tmap_f64(&P.ta, c.a1, N, N, nb, c.lda, c.abs ? c.abs : c.lda * N, 8, T::BM) != AFQ_OK ||
+      (KIND == F64_COMPLEX && make_tmap_f64(&P.ta2, c.a2, N, N, nb, c.lda, c.abs, 8, T::BM) != AFQ_OK) ||
+      make_tmap_f64(&P.tb, c.b, nc, N, W, nc, (long long)N * nc, 16, 16) != AFQ_OK)
+    return cudaErrorInvalidValue;
+  P.s.K = N;
+  P.s.mt = (N + T::BM - 1) / T::BM;
+  P.s.nt = (nc + T::BN - 1) / T::BN;
+  P.s.nz = W;
+  P.s.arow_step = T::BM;
+  P.s.a_batched = c.abs != 0;
+  P.s.gpw = kPlain;
+  P.s.err = f64_err(L, work);
+  P.epi = PropEpi{c.out, c.yin, c.scale, N, nc};
+  const size_t smem = 1024 + f64_stages<T>(0) * size_t(T::STAGE) + 256;
+  ProfScope ps(K_PROP, st);
+  return f64_launch<T>(P, f64_ctas(T::NT, smem), st);
+}
+
+// Tile of the per-walker products: 32 FM rows by 16 WN columns.  Every scheduler
+// runs WN of the 4 WN consumer warps, 2 FM MMAs per K step each, so a tile costs
+// FM WN and the launch ceil(tiles / SMs) of them; the choice with the least padding
+// and the fullest last wave (N = 200, No = 40, 512 walkers: 7 x 5, 4 waves).
+template <int KIND>
+cudaError_t prop_gemm(const Layout& L, double* work, int nc, const PropCall& c, cudaStream_t st) {
+  const int fms[6] = {1, 2, 3, 4, 5, 7};
+  const int groups = (nc + 15) / 16, sms = sm_count();
+  double best = 1e300;
+  int bf = 1, bw = 1;
+  for (int fm : fms)
+    for (int wn = 1; wn <= 5; ++wn) {
+      const long long tiles = (long long)((L.N + 32 * fm - 1) / (32 * fm)) * ((groups + wn - 1) / wn) * L.W;
+      const double cost = double((tiles + sms - 1) / sms) * (fm * wn + 1.0) * (wn == 1 ? 1.3 : 1.0);
+      if (cost < best - 1e-9) { best = cost; bf = fm; bw = wn; }
+    }
+#define AFQ_PROP_WN(FM)                                              \
+  switch (bw) {                                                      \
+    case 1: return prop_run<FM, 1, KIND>(L, work, nc, c, st);        \
+    case 2: return prop_run<FM, 2, KIND>(L, work, nc, c, st);        \
+    case 3: return prop_run<FM, 3, KIND>(L, work, nc, c, st);        \
+    case 4: return prop_run<FM, 4, KIND>(L, work, nc, c, st);        \
+    default: return prop_run<FM, 5, KIND>(L, work, nc, c, st);       \
+  }
+  switch (bf) {
+    case 1: AFQ_PROP_WN(1)
+    case 2: AFQ_PROP_WN(2)
+    case 3: AFQ_PROP_WN(3)
+    case 4: AFQ_PROP_WN(4)
+    case 5: AFQ_PROP_WN(5)
+    default: AFQ_PROP_WN(7)
+  }
+#undef AFQ_PROP_WN
+}
+
+// Exchange and orbital-energy tiles: 128 rows (the layout's gpt Cholesky vectors), wpt
+// walkers of gpw column groups; calls f with the tile type.
+template <class F>
+cudaError_t with_exch_tile(int no, int& wpt, int& gpw, F&& f) {
+  gpw = (2 * no + 15) / 16;
+  wpt = gpw == 1 ? 4 : (gpw <= 3 ? 2 : 1);
+  switch (gpw) {
+    case 1:
+    case 2:
+    case 4: return f(F64Tile<4, 4, 1, F64_REAL, F64_B_N>());
+    case 3:
+    case 6: return f(F64Tile<4, 3, 2, F64_REAL, F64_B_N>());
+    case 5: return f(F64Tile<4, 5, 1, F64_REAL, F64_B_N>());
+    default: return f(F64Tile<4, 4, 2, F64_REAL, F64_B_N>());  // 7, 8
+  }
+}
+
+template <class T, class Epi>
+cudaError_t exch_run(const Layout& L, const double* prep, double* work, int s, F64Params<Epi>& P, int wpt,
+                     int gpw, int extra, cudaStream_t st) {
+  const int no = L.no[s], gpt = L.ex[s].bm / no;
+  if (make_tmap_f64(&P.ta, prep + L.p_rc[s], L.N, (long long)L.G * no, 1, L.Npad, L.Npad * L.G * no, 8, T::BM) !=
+          AFQ_OK ||
+      make_tmap_f64(&P.tb, work + L.w_theta[s], 2 * no, L.N, L.W, 2 * no, (long long)L.N * 2 * no, 16, 16) !=
+          AFQ_OK)
+    return cudaErrorInvalidValue;
+  P.s.K = L.N;
+  P.s.mt = (L.G + gpt - 1) / gpt;
+  P.s.nt = (L.W + wpt - 1) / wpt;
+  P.s.nz = 1;
+  P.s.arow_step = gpt * no;
+  P.s.gpw = gpw;
+  P.s.wpt = wpt;
+  P.s.err = f64_err(L, work);
+  P.s.epi_bytes = (int)exch_stage_bytes<T>(extra);
+  ProfScope ps(K_EXCH, st);
+  return f64_launch<T>(P, sm_count(), st);
 }
 
 }  // namespace
 
 cudaError_t launch_fb_gemm(const Layout& L, const double* prep, double* work, cudaStream_t st) {
-  using Cfg = CfgBig;
   const int M = 2 * L.W, N = L.G;
   const long long K = L.Kfb_used;
-  F64Operand A{work + L.w_gpl, L.Kfb, 0, 0, kUnseg};
-  F64Operand B{prep + L.p_rccat, L.Kfb, 0, 0, kUnseg};
   int kchunk = (int)((K + L.splitk - 1) / L.splitk);
-  kchunk = (kchunk + Cfg::BK - 1) / Cfg::BK * Cfg::BK;
-  cudaError_t err = set_smem<Cfg>((const void*)fb_gemm_kernel<Cfg>, Cfg::SMEM);
-  if (err != cudaSuccess) return err;
-  dim3 grid((M + Cfg::BM - 1) / Cfg::BM, (N + Cfg::BN - 1) / Cfg::BN, L.splitk);
-  ProfScope ps(K_FB, st);
-  fb_gemm_kernel<Cfg><<<grid, Cfg::NT, Cfg::SMEM, st>>>(A, B, M, N, (int)K, kchunk,
-                                                        work + L.w_fbpart, L.Gpad,
-                                                        2LL * L.W * L.Gpad);
-  return cudaGetLastError();
+  kchunk = (kchunk + 15) / 16 * 16;
+  const int ks = (int)((K + kchunk - 1) / kchunk);
+  double* part = work + L.w_fbpart;
+  const long long zs = 2LL * L.W * L.Gpad;
+  for (int z = ks; z < L.splitk; ++z) {  // splits without work: their partial sums are zero
+    cudaError_t e = cudaMemsetAsync(part + z * zs, 0, zs * sizeof(double), st);
+    if (e != cudaSuccess) return e;
+  }
+  return with_gemm_tile<F64_B_K>(M, N, ks, [&](auto tile) {
+    using T = decltype(tile);
+    F64Params<FbEpi> P{};
+    if (make_tmap_f64(&P.ta, work + L.w_gpl, K, M, 1, L.Kfb, L.Kfb * M, 8, T::BM) != AFQ_OK ||
+        make_tmap_f64(&P.tb, prep + L.p_rccat, K, N, 1, L.Kfb, L.Kfb * N, 8, T::BN) != AFQ_OK)
+      return cudaErrorInvalidValue;
+    P.s.K = (int)K;
+    P.s.mt = (M + T::BM - 1) / T::BM;
+    P.s.nt = (N + T::BN - 1) / T::BN;
+    P.s.nz = ks;
+    P.s.arow_step = T::BM;
+    P.s.ksplit = kchunk;
+    P.s.err = f64_err(L, work);
+    P.epi = FbEpi{part, L.Gpad, zs, M, N};
+    ProfScope ps(K_FB, st);
+    return f64_launch<T>(P, sm_count(), st);
+  });
 }
 
 cudaError_t launch_prep_grouped(const PrepArgs* args, const BlockMap& m, int step, cudaStream_t st) {
@@ -541,17 +677,24 @@ cudaError_t launch_free_fields(const Layout& L, double* work, const double* fiel
 }
 
 cudaError_t launch_vhs_gemm(const Layout& L, const double* prep, double* work, cudaStream_t st) {
-  using Cfg = CfgBig;
   const int M = 2 * L.W, NN = L.N * L.N, K = L.G;
-  F64Operand A{work + L.w_xt, L.Gpad, 0, 0, kUnseg};
-  F64Operand B{prep + L.p_chol, L.N2pad, 0, 0, kUnseg};
-  cudaError_t err = set_smem<Cfg>((const void*)vhs_gemm_kernel<Cfg>, Cfg::SMEM);
-  if (err != cudaSuccess) return err;
-  dim3 grid((M + Cfg::BM - 1) / Cfg::BM, (NN + Cfg::BN - 1) / Cfg::BN);
-  ProfScope ps(K_VHS, st);
-  vhs_gemm_kernel<Cfg><<<grid, Cfg::NT, Cfg::SMEM, st>>>(A, B, M, NN, K, L.N, L.Npad,
-                                                         work + L.w_vhs);
-  return cudaGetLastError();
+  return with_gemm_tile<F64_B_N>(M, NN, 1, [&](auto tile) {
+    using T = decltype(tile);
+    F64Params<VhsEpi> P{};
+    if (make_tmap_f64(&P.ta, work + L.w_xt, K, M, 1, L.Gpad, L.Gpad * M, 8, T::BM) != AFQ_OK ||
+        make_tmap_f64(&P.tb, prep + L.p_chol, NN, K, 1, L.N2pad, L.N2pad * K, 16, 16) != AFQ_OK)
+      return cudaErrorInvalidValue;
+    P.s.K = K;
+    P.s.mt = (M + T::BM - 1) / T::BM;
+    P.s.nt = (NN + T::BN - 1) / T::BN;
+    P.s.nz = 1;
+    P.s.arow_step = T::BM;
+    P.s.gpw = kPlain;
+    P.s.err = f64_err(L, work);
+    P.epi = VhsEpi{work + L.w_vhs, M, NN, L.N, L.Npad};
+    ProfScope ps(K_VHS, st);
+    return f64_launch<T>(P, sm_count(), st);
+  });
 }
 
 cudaError_t launch_propagate_walkers(const Layout& L, const double* prep, double* work,
@@ -559,93 +702,42 @@ cudaError_t launch_propagate_walkers(const Layout& L, const double* prep, double
                                      cudaStream_t st) {
   const int N = L.N;
   const long long vld = 2 * L.Npad;
+  const double* vr = work + L.w_vhs;
+  const double* vi = vr + L.Npad;
   for (int s = 0; s < L.np; ++s) {
     const int nc = 2 * L.no[s];
-    const long long bs = (long long)N * nc;
     double* wk = walkers[s];
     double* y = work + L.w_y;
-    double* acc = work + L.w_acc;
-    double* ta = work + L.w_ta;
-    double* tb = work + L.w_tb;
-    F64Operand E{prep + L.p_exph1[s], L.Npad, 0, 0, kUnseg};
-    F64Operand Bw{wk, nc, bs, 0, kUnseg};
-    PropEpi ep{0, 1.0, y, nullptr, nullptr, nc, bs};
-    cudaError_t err = prop_gemm(E, E, Bw, N, nc, N, 1, L.W, ep, st);
+    const double* e1 = prep + L.p_exph1[s];
+    // y = e^{-dt h/2} w
+    cudaError_t err = prop_gemm<F64_REAL>(L, work, nc, {e1, nullptr, L.Npad, 0, wk, y, nullptr, 1.0}, st);
     if (err != cudaSuccess) return err;
+    // z_{n-1} = y + VHS z_n / n for n = T .. 1 (T = n_exp_terms - 1), z_T = y
     const double* src = y;
-    double* bufs[2] = {ta, tb};
-    if (n_exp_terms <= 1) {
-      F64Operand By{y, nc, bs, 0, kUnseg};
-      PropEpi ef{0, 1.0, wk, nullptr, nullptr, nc, bs};
-      err = prop_gemm(E, E, By, N, nc, N, 1, L.W, ef, st);
-      if (err != cudaSuccess) return err;
-      continue;
-    }
-    F64Operand Vr{work + L.w_vhs, vld, (long long)N * vld, 0, kUnseg};
-    F64Operand Vi{work + L.w_vhs + L.Npad, vld, (long long)N * vld, 0, kUnseg};
-    for (int n = 1; n < n_exp_terms; ++n) {
-      F64Operand Bt{src, nc, bs, 0, kUnseg};
-      double* dst = bufs[(n - 1) & 1];
-      const int mode = (n == 1) ? 1 : ((n == n_exp_terms - 1) ? 3 : 2);
-      PropEpi et{mode, 1.0 / n, dst, y, acc, nc, bs};
-      if (n == 1 && n_exp_terms == 2) et.mode = 1;
-      err = prop_gemm(Vr, Vi, Bt, N, nc, N, 2, L.W, et, st);
+    double* bufs[2] = {work + L.w_ta, work + L.w_tb};
+    for (int n = n_exp_terms - 1; n >= 1; --n) {
+      double* dst = bufs[n & 1];
+      err = prop_gemm<F64_COMPLEX>(L, work, nc, {vr, vi, vld, (long long)N * vld, src, dst, y, 1.0 / n}, st);
       if (err != cudaSuccess) return err;
       src = dst;
     }
-    F64Operand Ba{acc, nc, bs, 0, kUnseg};
-    PropEpi el{0, 1.0, wk, nullptr, nullptr, nc, bs};
-    err = prop_gemm(E, E, Ba, N, nc, N, 1, L.W, el, st);
+    // w' = e^{-dt h/2} z_0
+    err = prop_gemm<F64_REAL>(L, work, nc, {e1, nullptr, L.Npad, 0, src, wk, nullptr, 1.0}, st);
     if (err != cudaSuccess) return err;
   }
   return cudaSuccess;
 }
 
-template <class Cfg>
-static cudaError_t run_exch(const Layout& L, const double* prep, double* work, int s,
-                            cudaStream_t st) {
-  const ExchTile& X = L.ex[s];
-  const int no = L.no[s];
-  F64Operand A{prep + L.p_rc[s], L.Npad, 0, 0, kUnseg};
-  F64Operand B{work + L.w_theta[s], 2 * no, 0, (long long)L.N * 2 * no, 2 * no};
-  const size_t stage = size_t(Cfg::BM) * (Cfg::BN + 2) * sizeof(double) +
-                       size_t(X.gpt) * X.wpt * sizeof(double2);
-  const size_t smem = stage > Cfg::SMEM ? stage : Cfg::SMEM;
-  cudaError_t err = set_smem<Cfg>((const void*)exch_kernel<Cfg>, smem);
-  if (err != cudaSuccess) return err;
-  dim3 grid(X.mt, (L.W + X.wpt - 1) / X.wpt);
-  ProfScope ps(K_EXCH, st);
-  exch_kernel<Cfg><<<grid, Cfg::NT, smem, st>>>(A, B, L.G, no, L.N, L.W, X.gpt, X.wpt,
-                                                work + L.w_c[s], work + L.w_exc[s]);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_exchange(const Layout& L, const double* prep, double* work, int s,
                             cudaStream_t st) {
-  if (L.ex[s].bn == 80) return run_exch<CfgX80>(L, prep, work, s, st);
-  if (L.ex[s].bn == 120) return run_exch<CfgX120>(L, prep, work, s, st);
-  if (L.ex[s].bn == 160) return run_exch<CfgX160>(L, prep, work, s, st);
-  return cudaErrorInvalidValue;
-}
-
-template <class Cfg>
-static cudaError_t run_orb(const Layout& L, const double* prep, double* work, const double* prj,
-                           int nlo, cudaStream_t st) {
-  const ExchTile& X = L.ex[0];
-  const int no = L.no[0];
-  const int mt = (L.G + X.gpt - 1) / X.gpt;
-  F64Operand A{prep + L.p_rc[0], L.Npad, 0, 0, kUnseg};
-  F64Operand B{work + L.w_theta[0], 2 * no, 0, (long long)L.N * 2 * no, 2 * no};
-  const size_t stage = size_t(Cfg::BM) * (Cfg::BN + 2) * sizeof(double) +
-                       size_t(kMaxLo) * 64 * sizeof(double) + size_t(X.gpt) * X.wpt * sizeof(double2);
-  const size_t smem = stage > Cfg::SMEM ? stage : Cfg::SMEM;
-  cudaError_t err = set_smem<Cfg>((const void*)orb_kernel<Cfg>, smem);
-  if (err != cudaSuccess) return err;
-  dim3 grid(mt, (L.W + X.wpt - 1) / X.wpt);
-  ProfScope ps(K_EXCH, st);
-  orb_kernel<Cfg><<<grid, Cfg::NT, smem, st>>>(A, B, L.G, no, L.N, L.W, X.gpt, X.wpt, prj, nlo,
-                                               work + L.w_orb);
-  return cudaGetLastError();
+  const int no = L.no[s], gpt = L.ex[s].bm / no;
+  int wpt, gpw;
+  return with_exch_tile(no, wpt, gpw, [&](auto tile) {
+    using T = decltype(tile);
+    F64Params<ExchEpi> P{};
+    P.epi = ExchEpi{L.G, no, L.W, gpt, wpt, gpw, work + L.w_c[s], work + L.w_exc[s]};
+    return exch_run<T>(L, prep, work, s, P, wpt, gpw, 4 * (gpt * wpt + T::CW), st);
+  });
 }
 
 cudaError_t launch_orbenergy(const Layout& L, const double* prep, double* work, const double* prj,
@@ -658,17 +750,17 @@ cudaError_t launch_orbenergy(const Layout& L, const double* prep, double* work, 
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  if (L.ex[0].bn == 80)
-    e = run_orb<CfgX80>(L, prep, work, prj, nlo, st);
-  else if (L.ex[0].bn == 120)
-    e = run_orb<CfgX120>(L, prep, work, prj, nlo, st);
-  else if (L.ex[0].bn == 160)
-    e = run_orb<CfgX160>(L, prep, work, prj, nlo, st);
-  else
-    return cudaErrorInvalidValue;
+  const int no = L.no[0], gpt = L.ex[0].bm / no;
+  int wpt, gpw;
+  e = with_exch_tile(no, wpt, gpw, [&](auto tile) {
+    using T = decltype(tile);
+    F64Params<OrbEpi> P{};
+    P.epi = OrbEpi{L.G, no, L.W, gpt, wpt, gpw, nlo, prj, work + L.w_orb};
+    return exch_run<T>(L, prep, work, 0, P, wpt, gpw, kMaxLo * 64 + 2 * gpt * wpt, st);
+  });
   if (e != cudaSuccess) return e;
   const int wpb = 8;
-  const int mt = (L.G + L.ex[0].gpt - 1) / L.ex[0].gpt;
+  const int mt = (L.G + gpt - 1) / gpt;
   ProfScope ps(K_ECOMB, st);
   orb_combine_kernel<<<(L.W + wpb - 1) / wpb, 32 * wpb, 0, st>>>(L.W, mt, work + L.w_orb, out);
   return cudaGetLastError();
