@@ -302,6 +302,14 @@ int afq_propagate_constrained(const afq_dims* d, const void* prepared, afq_state
   const double* P = static_cast<const double*>(prepared);
   double* Wk = static_cast<double*>(work);
   cudaStream_t st = as_stream(stream);
+  if (small_step_fits(L)) {
+    const bool have = (s->flags & AFQ_STATE_GREEN_CURRENT) != 0;
+    s->flags &= ~AFQ_STATE_GREEN_CURRENT;
+    AFQ_TRY(launch_small_step(L, P, Wk, s->walkers, fields, d->dt, d->n_exp_terms, have, st));
+    s->flags |= AFQ_STATE_GREEN_CURRENT;
+    AFQ_TRY(launch_weight_update(L, P, Wk, s->weights, s->overlaps, s->scalars, d->dt, st));
+    return AFQ_OK;
+  }
   // force bias of the current walkers (the Green's function is reused when the
   // previous step on this workspace already computed it for these walkers)
   GreenArgs a = green_args(L, P, Wk, wc);

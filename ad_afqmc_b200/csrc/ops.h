@@ -58,6 +58,12 @@ cudaError_t launch_orbenergy(const Layout& L, const double* prepared, double* wo
 cudaError_t launch_energy_combine(const Layout& L, const double* prepared, double* work,
                                   double* eout, int eout_stride, cudaStream_t st);
 
+// ---- FP64 step of small systems in one kernel (small_step.cu) ---------------
+bool small_step_fits(const Layout& L);
+cudaError_t launch_small_step(const Layout& L, const double* prepared, double* work,
+                              double* const walkers[2], const double* fields, double dt,
+                              int n_exp_terms, bool have_green, cudaStream_t st);
+
 // ---- walker ops (walker_ops.cu) --------------------------------------------
 cudaError_t launch_weight_update(const Layout& L, const double* prepared, double* work,
                                  double* weights, double* overlaps, double* scalars, double dt,
