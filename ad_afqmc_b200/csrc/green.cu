@@ -278,49 +278,47 @@ __device__ __forceinline__ void green_body(const GreenArgs& a, int mode, int w, 
 }
 
 // Warp 0 of gj_kernel: the pivot among this lane's two candidate rows (lane,
-// lane + 32) and the other lanes': the largest |re|+|im|, the lowest row
-// among equal values (LAPACK izamax).  One 64-bit max-reduction over keys
-// that hold the magnitude's bits above the row number: a non-negative
-// double's bit pattern orders like its value, so the key order is the
-// magnitude order except between values within 128 ulps of each other,
-// which go to the lower row.  Non-candidates have key 0.
+// lane + 32) and the other lanes': the largest |re|+|im| to 13 bits of mantissa, the
+// lowest row among equals (LAPACK's izamax up to rows within 1.2e-4 of each other;
+// any of those is as good a pivot).  One 32-bit warp reduction over keys that
+// hold the high word of the magnitude (a non-negative double orders like its bits)
+// above the row number; a 64-bit one by shuffles took 350 cycles a step.
+// Non-candidates have key 0.
 __device__ __forceinline__ int gj_pivot(double2 v0, double2 v1, bool ok0, bool ok1, int lane) {
-  auto key = [](double2 v, int row) -> unsigned long long {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(fabs(v.x) + fabs(v.y));
-    return (b & ~127ull) | 64ull | (unsigned long long)(63 - row);
+  auto key = [](double2 v, int row) -> unsigned {
+    return ((unsigned)__double2hiint(fabs(v.x) + fabs(v.y)) & ~127u) | 64u | (unsigned)(63 - row);
   };
-  unsigned long long k = ok0 ? key(v0, lane) : 0ull;
-  const unsigned long long k1 = ok1 ? key(v1, lane + 32) : 0ull;
-  k = k1 > k ? k1 : k;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long ok = __shfl_xor_sync(0xffffffffu, k, o);
-    k = ok > k ? ok : k;
-  }
-  return 63 - (int)(k & 63ull);
+  const unsigned k0 = ok0 ? key(v0, lane) : 0u, k1 = ok1 ? key(v1, lane + 32) : 0u;
+  return 63 - (int)(__reduce_max_sync(0xffffffffu, k0 > k1 ? k0 : k1) & 63u);
 }
 
 // Gauss-Jordan inverse and det of S = C^T W held in sbuf, one CTA per
-// (walker, sector), in place in one shared-memory copy of S, with one block
-// barrier per elimination step (partial pivoting, pivot = largest |re|+|im|
-// in the column).
+// (walker, sector), in place in one shared-memory copy of S, in panels of four
+// columns (partial pivoting, pivot = largest |re|+|im| in the column).
 //  * Rows are never swapped: the pivot row r_k of step k stays in place and
 //    the inverse is unscrambled once at the end, S^-1[i][r_k] = X[r_i][k].
-//  * Pivot rows are scaled lazily: row r_k keeps its unscaled values U (the
-//    true row is U / p_k).  Every later update of that row has the same form
-//    on U (the update is linear in the row), so no thread writes row r_k
-//    during step k, and each thread reads the pivot row straight from S and
-//    scales the elements it needs.  The row scales are applied when the
-//    inverse is unscrambled.
-//  * The multipliers of step k (column k before the step) come from a copy
-//    that warp 0 wrote during step k-1, when it computed that column, so the
-//    owners of column k may overwrite it during step k.
-//  * Warp 0 computes the new column k+1, its pivot (over the rows not yet
-//    used) and the reciprocal; warps 1..7 update every other column, each
-//    thread one column and a stride of rows.  Rows are stored with an odd
-//    stride (ld = no | 1 double2), so a warp reading a column hits distinct
-//    banks.  det = product of the pivots times the permutation's sign.
-// At most 64 rows (no <= 64, checked by the caller).
+//  * Warp 0 runs a panel's steps on registers (lane l: rows l and l + 32 of the
+//    four columns), the pivot by shuffles, no block barrier.  Each step is a
+//    left multiplication that differs from the identity in column r_k only, so
+//    the finished panel holds the product T of its four: T = I outside the
+//    columns r_k, and column r_k of T is the panel's column k.
+//  * Every other column is then multiplied by T: new a[i][j] = (i a pivot row of
+//    this panel ? 0 : a[i][j]) + sum_m panel[i][m] a[r_m][j].
+// What bounds it is the chain of pivots in warp 0 while the SM's other CTAs update.
+// One barrier per column, with every step's column formed by warp 0 and the rest
+// updated beside it, took 89 us at No = 40 and 512 walkers; this takes 56 us
+// (No = 60, 58 and 1024 walkers: 940 -> 635 us; No = 39, 231 walkers: 59 -> 46 us).
+// Panels of eight spill at 128 registers (69 us).
+// Rows are stored with an odd stride (ld = no | 1 double2), so a warp reading a
+// column hits distinct banks.  det = product of the pivots times the permutation's
+// sign.  At most 64 rows (no <= 64, checked by the caller).
+constexpr int kGjThreads = 128;
+constexpr int kGjPanel = 4;
+
+__device__ __forceinline__ double2 shfl2(double2 v, int lane) {
+  return make_double2(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane));
+}
+
 __device__ __forceinline__ void gj_body(int W, int no0, int no1, double* sbuf, long long sstride,
                                         int bstride, double* wscal, int w, int sct) {
   extern __shared__ double2 gsm[];
@@ -328,12 +326,12 @@ __device__ __forceinline__ void gj_body(int W, int no0, int no1, double* sbuf, l
   const int ld = no | 1;
   const int nn = no * no;
   double2* const A = gsm;
-  double2* const pcol = gsm + bstride;  // [2][64]: multipliers of the step, by parity
-  __shared__ double2 ipks[64];          // 1 / pivot of each step (the lazy row scales)
+  double2* const P = gsm + bstride;  // the panel: [64][kGjPanel]
   __shared__ int piv[64];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  __shared__ unsigned long long rows_s;  // the panel's pivot rows
+  const int tid = threadIdx.x, lane = tid & 31;
   double2* g = reinterpret_cast<double2*>(sbuf) + ((long long)sct * W + w) * sstride;
-  for (int e = tid; e < nn; e += kGreenThreads) {
+  for (int e = tid; e < nn; e += kGjThreads) {
     const int i = e / no;
     A[i * ld + (e - i * no)] = g[e];
   }
@@ -343,87 +341,84 @@ __device__ __forceinline__ void gj_body(int W, int no0, int no1, double* sbuf, l
   const bool in0 = lane < no, in1 = lane + 32 < no;
   bool used0 = false, used1 = false;  // warp 0: rows lane, lane + 32 already pivots
   double2 det = make_double2(1.0, 0.0);
-  // warp 0: the pivot of column 0 and its value, from the column in registers
-  auto pivot = [&](double2 v0, double2 v1, int col) {
-    const int rn = gj_pivot(v0, v1, in0 && !used0, in1 && !used1, lane);
-    const double2 sel = rn < 32 ? v0 : v1;
-    const double2 p = make_double2(__shfl_sync(0xffffffffu, sel.x, rn & 31),
-                                   __shfl_sync(0xffffffffu, sel.y, rn & 31));
-    const double inv = 1.0 / (p.x * p.x + p.y * p.y);
-    if (lane == (rn & 31)) (rn < 32 ? used0 : used1) = true;
-    if (lane == 0) {
-      piv[col] = rn;
-      ipks[col] = make_double2(p.x * inv, -p.y * inv);
-      det = cmul(det, p);
-    }
-  };
-  if (warp == 0) {
-    const double2 v0 = in0 ? A[lane * ld] : zero, v1 = in1 ? A[(lane + 32) * ld] : zero;
-    if (in0) pcol[lane] = v0;
-    if (in1) pcol[lane + 32] = v1;
-    pivot(v0, v1, 0);
-  }
-  __syncthreads();
-
-  // warps 1..7: thread tid - 32 = g * no + j owns column j, rows g, g + G, ...
-  // (G = 224 / no row groups; threads beyond G * no idle)
-  constexpr int TW = kGreenThreads - 32;
-  const int nd = no > 0 ? no : 1;
-  const int G = TW / nd;
-  const int tu = tid - 32;
-  const int jc = tu % nd, g0 = tu / nd;
-  const bool upd = warp > 0 && g0 < G;
-  for (int k = 0; k < no; ++k) {
-    const int cur = k & 1;
-    const double2* pc = pcol + cur * 64;
-    const int r = piv[k];
-    const double2 ipk = ipks[k];
-    const int c = k + 1;
-    if (warp == 0) {
-      if (c < no) {
-        // the new column c (row r keeps its unscaled values), the next step's
-        // multipliers, then the pivot among the unused rows
-        const double2 prc = cmul(A[r * ld + c], ipk);
-        double2 v0 = zero, v1 = zero;
-        if (in0) {
-          const int i = lane;
-          v0 = A[i * ld + c];
-          if (i != r) {
-            v0 = csub(v0, cmul(pc[i], prc));
-            A[i * ld + c] = v0;
-          }
-          pcol[(cur ^ 1) * 64 + i] = v0;
-        }
-        if (in1) {
-          const int i = lane + 32;
-          v1 = A[i * ld + c];
-          if (i != r) {
-            v1 = csub(v1, cmul(pc[i], prc));
-            A[i * ld + c] = v1;
-          }
-          pcol[(cur ^ 1) * 64 + i] = v1;
-        }
-        pivot(v0, v1, c);
+  // trailing update: thread -> column jt of the no - b others, rows g0, g0 + RG, ...
+  for (int k0 = 0; k0 < no; k0 += kGjPanel) {
+    const int b = min(kGjPanel, no - k0);
+    if (tid < 32) {
+      double2 v0[kGjPanel], v1[kGjPanel];
+#pragma unroll
+      for (int c = 0; c < kGjPanel; ++c) {
+        v0[c] = in0 && c < b ? A[lane * ld + k0 + c] : zero;
+        v1[c] = in1 && c < b ? A[(lane + 32) * ld + k0 + c] : zero;
       }
-    } else if (upd && jc != c) {
-      const int j = jc;
-      if (j == k) {  // the pivot column: -(multiplier) / p, and 1 in the (lazy) pivot row
-        for (int i = g0; i < no; i += G) {
-          const double2 t0 = cmul(pc[i], ipk);
-          A[i * ld + j] = (i == r) ? make_double2(1.0, 0.0) : make_double2(-t0.x, -t0.y);
+      unsigned long long rows = 0ull;
+#pragma unroll
+      for (int m = 0; m < kGjPanel; ++m) {
+        if (m < b) {
+          const int rn = gj_pivot(v0[m], v1[m], in0 && !used0, in1 && !used1, lane);
+          const bool hi = rn >= 32;
+          const int owner = rn & 31;
+          const double2 p = shfl2(hi ? v1[m] : v0[m], owner);
+          const double inv = 1.0 / (p.x * p.x + p.y * p.y);
+          const double2 ip = make_double2(p.x * inv, -p.y * inv);
+          const bool mine0 = !hi && lane == owner, mine1 = hi && lane == owner;
+          const double2 f0 = v0[m], f1 = v1[m];
+#pragma unroll
+          for (int c = 0; c < kGjPanel; ++c) {
+            if (c == m) continue;
+            const double2 s = cmul(shfl2(hi ? v1[c] : v0[c], owner), ip);
+            v0[c] = mine0 ? s : csub(v0[c], cmul(f0, s));
+            v1[c] = mine1 ? s : csub(v1[c], cmul(f1, s));
+          }
+          const double2 q0 = cmul(f0, ip), q1 = cmul(f1, ip);
+          v0[m] = mine0 ? ip : make_double2(-q0.x, -q0.y);
+          v1[m] = mine1 ? ip : make_double2(-q1.x, -q1.y);
+          used0 |= mine0;
+          used1 |= mine1;
+          rows |= 1ull << rn;
+          det = cmul(det, p);
+          if (lane == 0) piv[k0 + m] = rn;
         }
-      } else {
-        const double2 prj = cmul(A[r * ld + j], ipk);
-        for (int i = g0; i < no; i += G)
-          if (i != r) A[i * ld + j] = csub(A[i * ld + j], cmul(pc[i], prj));
+      }
+      if (lane == 0) rows_s = rows;
+#pragma unroll
+      for (int c = 0; c < kGjPanel; ++c) {
+        if (c < b && in0) A[lane * ld + k0 + c] = P[lane * kGjPanel + c] = v0[c];
+        if (c < b && in1) A[(lane + 32) * ld + k0 + c] = P[(lane + 32) * kGjPanel + c] = v1[c];
       }
     }
     __syncthreads();
+    const int cols = no - b;
+    if (cols > 0) {
+      const unsigned long long rows = rows_s;
+      // column tiles of at most kGjThreads columns never occur (no <= 64)
+      const int rg = kGjThreads / cols, jt = tid % cols, r0 = tid / cols;
+      const int j = jt < k0 ? jt : jt + b;
+      double2 u[kGjPanel];
+      if (r0 < rg) {
+#pragma unroll
+        for (int m = 0; m < kGjPanel; ++m) u[m] = m < b ? A[piv[k0 + m] * ld + j] : zero;
+      }
+      __syncthreads();
+      if (r0 < rg)
+        for (int i = r0; i < no; i += rg) {
+          double2 x = (rows >> i) & 1ull ? zero : A[i * ld + j];
+          const double2* pr = P + i * kGjPanel;
+          double2 y = zero;  // two chains
+#pragma unroll
+          for (int m = 0; m < kGjPanel; m += 2) {
+            if (m < b) x = cadd(x, cmul(pr[m], u[m]));
+            if (m + 1 < b) y = cadd(y, cmul(pr[m + 1], u[m + 1]));
+          }
+          A[i * ld + j] = cadd(x, y);
+        }
+      __syncthreads();
+    }
   }
-  // unscramble with the row scales: S^-1[i][r_k] = X[r_i][k] = A[r_i][k] / p_i
-  for (int e = tid; e < nn; e += kGreenThreads) {
+  // unscramble: S^-1[i][r_k] = X[r_i][k]
+  for (int e = tid; e < nn; e += kGjThreads) {
     const int i = e / no, k = e - (e / no) * no;
-    g[i * no + piv[k]] = cmul(A[piv[i] * ld + k], ipks[i]);
+    g[i * no + piv[k]] = A[piv[i] * ld + k];
   }
   if (tid == 0) {
     // sign of the permutation k -> r_k: (-1)^(no - cycles)
@@ -454,12 +449,12 @@ __global__ void __launch_bounds__(kGreenThreads) green_kernel_grouped(const Gree
   green_body<kGreenThreads>(a, mode, local % a.W, local / a.W);
 }
 
-__global__ void __launch_bounds__(kGreenThreads, 4)
+__global__ void __launch_bounds__(kGjThreads, 4)
     gj_kernel(int W, int no0, int no1, double* sbuf, long long sstride, int bstride, double* wscal) {
   gj_body(W, no0, no1, sbuf, sstride, bstride, wscal, blockIdx.x, blockIdx.y);
 }
 
-__global__ void __launch_bounds__(kGreenThreads, 4) gj_kernel_grouped(const GjArgs* A, BlockMap m) {
+__global__ void __launch_bounds__(kGjThreads, 4) gj_kernel_grouped(const GjArgs* A, BlockMap m) {
   int local;
   const GjArgs& a = A[block_owner(m, blockIdx.x, local)];
   gj_body(a.W, a.no0, a.no1, a.sbuf, a.sstride, a.bstride, a.wscal, local % a.W, local / a.W);
@@ -500,8 +495,10 @@ size_t green_smem_bytes(int nomax) {
          2 * size_t(kRowChunk) * nomax * sizeof(double) + size_t(kRowChunk) * (nomax + 1) * sizeof(double2);
 }
 
-// S with row stride nomax | 1 and two columns of multipliers
-size_t gj_smem_bytes(int nomax) { return (size_t(nomax) * (nomax | 1) + 128) * sizeof(double2); }
+// S with row stride nomax | 1 and a panel of four columns
+size_t gj_smem_bytes(int nomax) {
+  return (size_t(nomax) * (nomax | 1) + 64 * kGjPanel) * sizeof(double2);
+}
 
 cudaError_t launch_green_grouped(const GreenArgs* args, const BlockMap& m, int mode, size_t smem,
                                  cudaStream_t st) {
@@ -518,7 +515,7 @@ cudaError_t launch_gj_grouped(const GjArgs* args, const BlockMap& m, size_t smem
                                        (int)smem);
   if (e != cudaSuccess) return e;
   ProfScope ps(K_GREEN, st);
-  gj_kernel_grouped<<<m.start[m.n], kGreenThreads, smem, st>>>(args, m);
+  gj_kernel_grouped<<<m.start[m.n], kGjThreads, smem, st>>>(args, m);
   return cudaGetLastError();
 }
 
@@ -555,7 +552,7 @@ cudaError_t launch_green(const GreenArgs& a, cudaStream_t st) {
   if ((e = cudaFuncSetAttribute(gj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsmem)) !=
       cudaSuccess)
     return e;
-  gj_kernel<<<grid, kGreenThreads, gsmem, st>>>(a.W, a.sec[0].no, a.ns > 1 ? a.sec[1].no : 0,
+  gj_kernel<<<grid, kGjThreads, gsmem, st>>>(a.W, a.sec[0].no, a.ns > 1 ? a.sec[1].no : 0,
                                                 a.sbuf, a.sstride, bstride, a.wscal);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   kernel<<<grid, threads, smem, st>>>(a, 2);
