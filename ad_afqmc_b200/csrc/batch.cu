@@ -27,7 +27,8 @@ struct afq_batch {
   OvlpArgs* ovlp = nullptr;
   WeightArgs* weight = nullptr;
   BlockMap m_green{}, m_prep{}, m_wt[2]{}, m_ovlp{};
-  size_t green_smem = 0, gj_smem = 0;
+  int green_nomax = 0;
+  size_t gj_smem = 0;
 };
 
 namespace {
@@ -128,7 +129,7 @@ int afq_batch_create(int32_t n, const afq_dims* dims, const void* const* prepare
     green[f] = a;
     b->m_green.start[f] = gb;
     gb += l.W * l.ns;
-    b->green_smem = std::max(b->green_smem, green_smem_bytes(l.nomax));
+    b->green_nomax = std::max(b->green_nomax, l.nomax);
     b->gj_smem = std::max(b->gj_smem, gj_smem_bytes(l.nomax));
     gj[f] = GjArgs{l.W, l.no[0], l.ns > 1 ? l.no[1] : 0, l.nomax * (l.nomax | 1), Wk[f] + l.w_s,
                    (long long)l.nomax * l.nomax, Wk[f] + l.w_wscal};
@@ -225,9 +226,9 @@ int afq_batch_propagate_constrained(afq_batch* b, int32_t step, int32_t green_cu
   } while (0)
   // force bias of the current walkers (Green's function unless already current)
   if (!green_current) {
-    AFQ_B(launch_green_grouped(b->green, b->m_green, 1, b->green_smem, st));
+    AFQ_B(launch_green_grouped(b->green, b->m_green, 1, b->green_nomax, st));
     AFQ_B(launch_gj_grouped(b->gj, b->m_green, b->gj_smem, st));
-    AFQ_B(launch_green_grouped(b->green, b->m_green, 2, b->green_smem, st));
+    AFQ_B(launch_green_grouped(b->green, b->m_green, 2, b->green_nomax, st));
   }
   int rc = umma_batch_fb(b->umma, st);
   if (rc != AFQ_OK) return rc;
@@ -240,9 +241,9 @@ int afq_batch_propagate_constrained(afq_batch* b, int32_t step, int32_t green_cu
       if ((rc = umma_batch_prop(b->umma, s, i, st)) != AFQ_OK) return rc;
   }
   // new overlaps, the next step's force-bias operand, weights
-  AFQ_B(launch_green_grouped(b->green, b->m_green, 1, b->green_smem, st));
+  AFQ_B(launch_green_grouped(b->green, b->m_green, 1, b->green_nomax, st));
   AFQ_B(launch_gj_grouped(b->gj, b->m_green, b->gj_smem, st));
-  AFQ_B(launch_green_grouped(b->green, b->m_green, 2, b->green_smem, st));
+  AFQ_B(launch_green_grouped(b->green, b->m_green, 2, b->green_nomax, st));
   AFQ_B(launch_ovlp_grouped(b->ovlp, b->m_ovlp, st));
   AFQ_B(launch_weight_grouped(b->weight, b->n, st));
 #undef AFQ_B

@@ -11,7 +11,7 @@ namespace afq {
 template <int T>
 __device__ double2 gauss_jordan_cta(double2* S, double2* colk, int* perm, double2* ipk_s, int no) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  constexpr int Q = 4096 / T;  // elements of a 64 x 64 S per thread
+  constexpr int Q = (4096 + T - 1) / T;  // elements of a 64 x 64 S per thread
   const int npairs = no * no;
   // Each elimination step: warp 0 alone finds the pivot (first max of
   // |re|+|im| in column k, as LAPACK izamax), swaps it into row k, keeps

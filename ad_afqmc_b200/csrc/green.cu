@@ -20,7 +20,6 @@ namespace afq {
 
 namespace {
 
-constexpr int kGreenThreads = 256;
 constexpr int kRowChunk = 32;
 
 // asynchronous global -> shared copies (Ampere-style cp.async): the next
@@ -43,15 +42,15 @@ __device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_g
 
 // mode 0: the whole computation; 1: S = C^T W only, into a.sbuf; 2: Theta
 // and its outputs from S^-1 in a.sbuf (the inverse and det by gj_kernel).
-// T threads: 256, or 512 where the staging allows one CTA per SM only (each
-// warp then owns one column tile instead of up to two).
+// T threads: one warp per column tile of 8 real columns (2 No of them), at least
+// eight (see green_threads).
 template <int T>
 __device__ __forceinline__ void green_body(const GreenArgs& a, int mode, int w, int sct) {
   extern __shared__ double2 sm[];
   const GreenSector& S_ = a.sec[sct];
   const int N = a.N, no = S_.no, tid = threadIdx.x;
   constexpr int NW = T / 32;                 // warps
-  constexpr int SL = (16 + NW - 1) / NW;     // column tiles per warp (2 No <= 128: 16 tiles)
+  constexpr int SL = 1;                      // column tiles per warp
 
   double2* S = sm;                          // no*no
   double2* colk = S + no * no;              // 64
@@ -438,15 +437,35 @@ __device__ __forceinline__ void gj_body(int W, int no0, int no1, double* sbuf, l
 }
 
 template <int T>
-__global__ void __launch_bounds__(T) green_kernel(GreenArgs a, int mode) {
+__global__ void __launch_bounds__(T, T <= 384 ? 2 : 1) green_kernel(GreenArgs a, int mode) {
   green_body<T>(a, mode, blockIdx.x, blockIdx.y);
 }
 
-__global__ void __launch_bounds__(kGreenThreads) green_kernel_grouped(const GreenArgs* A, BlockMap m,
-                                                                      int mode) {
+template <int T>
+__global__ void __launch_bounds__(T, T <= 384 ? 2 : 1) green_kernel_grouped(const GreenArgs* A, BlockMap m, int mode) {
   int local;
   const GreenArgs& a = A[block_owner(m, blockIdx.x, local)];
-  green_body<kGreenThreads>(a, mode, local % a.W, local / a.W);
+  green_body<T>(a, mode, local % a.W, local / a.W);
+}
+
+// Threads of the S / Theta kernels: a warp for each of the (2 No + 7) / 8 column
+// tiles, 8, 10, 12 or 16 of them.  With eight warps for ten tiles (No = 40) two
+// warps worked twice as long as the rest: S + Theta 216 -> 177 us at N = 200,
+// 512 walkers.
+inline int green_threads(int nomax) {
+  const int tiles = (2 * nomax + 7) / 8;
+  return tiles <= 8 ? 256 : (tiles <= 10 ? 320 : (tiles <= 12 ? 384 : 512));
+}
+
+// calls f(kernel) for the kernel template's instance of `threads`
+template <class F>
+cudaError_t with_green_kernel(int threads, F&& f) {
+  switch (threads) {
+    case 256: return f(green_kernel<256>, green_kernel_grouped<256>);
+    case 320: return f(green_kernel<320>, green_kernel_grouped<320>);
+    case 384: return f(green_kernel<384>, green_kernel_grouped<384>);
+    default: return f(green_kernel<512>, green_kernel_grouped<512>);
+  }
 }
 
 __global__ void __launch_bounds__(kGjThreads, 4)
@@ -500,14 +519,17 @@ size_t gj_smem_bytes(int nomax) {
   return (size_t(nomax) * (nomax | 1) + 64 * kGjPanel) * sizeof(double2);
 }
 
-cudaError_t launch_green_grouped(const GreenArgs* args, const BlockMap& m, int mode, size_t smem,
+cudaError_t launch_green_grouped(const GreenArgs* args, const BlockMap& m, int mode, int nomax,
                                  cudaStream_t st) {
   ProfScope ps(K_GREEN, st);
-  cudaError_t e = cudaFuncSetAttribute(green_kernel_grouped, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
-  if (e != cudaSuccess) return e;
-  green_kernel_grouped<<<m.start[m.n], kGreenThreads, smem, st>>>(args, m, mode);
-  return cudaGetLastError();
+  const int threads = green_threads(nomax);
+  const size_t smem = green_smem_bytes(nomax);
+  return with_green_kernel(threads, [&](auto, auto kernel) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    kernel<<<m.start[m.n], threads, smem, st>>>(args, m, mode);
+    return cudaGetLastError();
+  });
 }
 
 cudaError_t launch_gj_grouped(const GjArgs* args, const BlockMap& m, size_t smem, cudaStream_t st) {
@@ -529,34 +551,33 @@ cudaError_t launch_green(const GreenArgs& a, cudaStream_t st) {
   int nomax = 0;
   for (int s = 0; s < a.ns; ++s) nomax = a.sec[s].no > nomax ? a.sec[s].no : nomax;
   const size_t smem = green_smem_bytes(nomax);
-  // staging above ~113 KB leaves one CTA per SM: 16 warps instead of 8 then
-  const bool wide = smem > 113 * 1024;
-  auto kernel = wide ? green_kernel<2 * kGreenThreads> : green_kernel<kGreenThreads>;
-  const int threads = wide ? 2 * kGreenThreads : kGreenThreads;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
+  const int threads = green_threads(nomax);
   dim3 grid(a.W, a.ns);
   ProfScope ps(K_GREEN, st);
   bool need_theta = a.gpl || a.gplb[0];
   for (int s = 0; s < a.ns; ++s)
     need_theta = need_theta || a.sec[s].theta || a.sec[s].gout || a.sec[s].rh1 || a.sec[s].gtb[0];
-  if (!a.sbuf || !need_theta) {  // one kernel: S, its inverse and det, Theta and outputs
-    kernel<<<grid, threads, smem, st>>>(a, 0);
+  return with_green_kernel(threads, [&](auto kernel, auto) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    if (!a.sbuf || !need_theta) {  // one kernel: S, its inverse and det, Theta and outputs
+      kernel<<<grid, threads, smem, st>>>(a, 0);
+      return cudaGetLastError();
+    }
+    // S into a.sbuf; its inverse and det; Theta and its outputs
+    kernel<<<grid, threads, smem, st>>>(a, 1);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    const int bstride = nomax * (nomax | 1);
+    const size_t gsmem = gj_smem_bytes(nomax);
+    if ((e = cudaFuncSetAttribute(gj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsmem)) !=
+        cudaSuccess)
+      return e;
+    gj_kernel<<<grid, kGjThreads, gsmem, st>>>(a.W, a.sec[0].no, a.ns > 1 ? a.sec[1].no : 0, a.sbuf,
+                                               a.sstride, bstride, a.wscal);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    kernel<<<grid, threads, smem, st>>>(a, 2);
     return cudaGetLastError();
-  }
-  // S into a.sbuf; warp-level inverse and det; Theta and its outputs
-  kernel<<<grid, threads, smem, st>>>(a, 1);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  const int bstride = nomax * (nomax | 1);
-  const size_t gsmem = gj_smem_bytes(nomax);
-  if ((e = cudaFuncSetAttribute(gj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsmem)) !=
-      cudaSuccess)
-    return e;
-  gj_kernel<<<grid, kGjThreads, gsmem, st>>>(a.W, a.sec[0].no, a.ns > 1 ? a.sec[1].no : 0,
-                                                a.sbuf, a.sstride, bstride, a.wscal);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  kernel<<<grid, threads, smem, st>>>(a, 2);
-  return cudaGetLastError();
+  });
 }
 
 cudaError_t launch_ovlp_combine(int W, int ns, int mult, const double* wscal, double* out,

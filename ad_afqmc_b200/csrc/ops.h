@@ -203,7 +203,7 @@ struct WalkerTArgs {
 };
 size_t green_smem_bytes(int nomax);
 size_t gj_smem_bytes(int nomax);
-cudaError_t launch_green_grouped(const GreenArgs* args, const BlockMap& m, int mode, size_t smem,
+cudaError_t launch_green_grouped(const GreenArgs* args, const BlockMap& m, int mode, int nomax,
                                  cudaStream_t st);
 cudaError_t launch_gj_grouped(const GjArgs* args, const BlockMap& m, size_t smem, cudaStream_t st);
 cudaError_t launch_ovlp_grouped(const OvlpArgs* args, const BlockMap& m, cudaStream_t st);
