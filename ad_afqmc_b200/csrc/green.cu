@@ -277,18 +277,24 @@ __device__ __forceinline__ void green_body(const GreenArgs& a, int mode, int w, 
 }
 
 // Warp 0 of gj_kernel: the pivot among this lane's two candidate rows (lane,
-// lane + 32) and the other lanes': the largest |re|+|im| to 13 bits of mantissa, the
-// lowest row among equals (LAPACK's izamax up to rows within 1.2e-4 of each other;
-// any of those is as good a pivot).  One 32-bit warp reduction over keys that
-// hold the high word of the magnitude (a non-negative double orders like its bits)
-// above the row number; a 64-bit one by shuffles took 350 cycles a step.
-// Non-candidates have key 0.
+// lane + 32) and the other lanes': the largest |re|+|im|, the lowest row
+// among equal values (LAPACK izamax).  The keys hold the magnitude's bits above
+// the row number: a non-negative double's bit pattern orders like its value, so
+// the key order is the magnitude order except between values within 128 ulps of
+// each other, which go to the lower row.  Non-candidates have key 0.  The maximum
+// is two 32-bit warp reductions, the high words and then the low words under the
+// highest; a 64-bit one by shuffles took 350 cycles a step.
 __device__ __forceinline__ int gj_pivot(double2 v0, double2 v1, bool ok0, bool ok1, int lane) {
-  auto key = [](double2 v, int row) -> unsigned {
-    return ((unsigned)__double2hiint(fabs(v.x) + fabs(v.y)) & ~127u) | 64u | (unsigned)(63 - row);
+  auto key = [](double2 v, int row) -> unsigned long long {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(fabs(v.x) + fabs(v.y));
+    return (b & ~127ull) | 64ull | (unsigned long long)(63 - row);
   };
-  const unsigned k0 = ok0 ? key(v0, lane) : 0u, k1 = ok1 ? key(v1, lane + 32) : 0u;
-  return 63 - (int)(__reduce_max_sync(0xffffffffu, k0 > k1 ? k0 : k1) & 63u);
+  unsigned long long k = ok0 ? key(v0, lane) : 0ull;
+  const unsigned long long k1 = ok1 ? key(v1, lane + 32) : 0ull;
+  k = k1 > k ? k1 : k;
+  const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(k >> 32));
+  const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(k >> 32) == hi ? (unsigned)k : 0u);
+  return 63 - (int)(lo & 63u);
 }
 
 // Gauss-Jordan inverse and det of S = C^T W held in sbuf, one CTA per
@@ -296,18 +302,22 @@ __device__ __forceinline__ int gj_pivot(double2 v0, double2 v1, bool ok0, bool o
 // columns (partial pivoting, pivot = largest |re|+|im| in the column).
 //  * Rows are never swapped: the pivot row r_k of step k stays in place and
 //    the inverse is unscrambled once at the end, S^-1[i][r_k] = X[r_i][k].
+//  * Pivot rows are scaled lazily: row r_k keeps its unscaled values, the factors
+//    1 / p_k are applied where the row is used and at the end.
 //  * Warp 0 runs a panel's steps on registers (lane l: rows l and l + 32 of the
-//    four columns), the pivot by shuffles, no block barrier.  Each step is a
-//    left multiplication that differs from the identity in column r_k only, so
-//    the finished panel holds the product T of its four: T = I outside the
-//    columns r_k, and column r_k of T is the panel's column k.
-//  * Every other column is then multiplied by T: new a[i][j] = (i a pivot row of
-//    this panel ? 0 : a[i][j]) + sum_m panel[i][m] a[r_m][j].
+//    four columns) without a block barrier and leaves each step's multipliers f_m
+//    (the step's column before it) in P.
+//  * Every other column then takes the four steps at once: s_m = a[r_m] / p_m with
+//    the earlier steps applied to row r_m, a[i] -= f_m[i] s_m for i != r_m.  These
+//    are the operations of one step after the other, in their order, so the
+//    inverse has the same bits as without panels (the product of the four steps
+//    applied as one matrix saves 10 us and rounds differently, which the
+//    bf16 split of Theta then turns into differences of 1e-7 in a rare walker).
 // What bounds it is the chain of pivots in warp 0 while the SM's other CTAs update.
 // One barrier per column, with every step's column formed by warp 0 and the rest
-// updated beside it, took 89 us at No = 40 and 512 walkers; this takes 56 us
-// (No = 60, 58 and 1024 walkers: 940 -> 635 us; No = 39, 231 walkers: 59 -> 46 us).
-// Panels of eight spill at 128 registers (69 us).
+// updated beside it, took 89 us at No = 40 and 512 walkers; this takes 67 us
+// (No = 60, 58 and 1024 walkers: 940 -> 742 us; No = 39, 231 walkers: 59 -> 51 us).
+// Panels of eight spill at 128 registers.
 // Rows are stored with an odd stride (ld = no | 1 double2), so a warp reading a
 // column hits distinct banks.  det = product of the pivots times the permutation's
 // sign.  At most 64 rows (no <= 64, checked by the caller).
@@ -316,6 +326,12 @@ constexpr int kGjPanel = 4;
 
 __device__ __forceinline__ double2 shfl2(double2 v, int lane) {
   return make_double2(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane));
+}
+
+// a b, rounded in one stated way wherever it stands: left to the compiler, the product
+// that is fused in the imaginary part depends on the code around it
+__device__ __forceinline__ double2 gj_mul(double2 a, double2 b) {
+  return make_double2(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)), __fma_rn(a.x, b.y, __dmul_rn(a.y, b.x)));
 }
 
 __device__ __forceinline__ void gj_body(int W, int no0, int no1, double* sbuf, long long sstride,
@@ -327,7 +343,7 @@ __device__ __forceinline__ void gj_body(int W, int no0, int no1, double* sbuf, l
   double2* const A = gsm;
   double2* const P = gsm + bstride;  // the panel: [64][kGjPanel]
   __shared__ int piv[64];
-  __shared__ unsigned long long rows_s;  // the panel's pivot rows
+  __shared__ double2 ipks[64];  // 1 / pivot of each step (the lazy row scales)
   const int tid = threadIdx.x, lane = tid & 31;
   double2* g = reinterpret_cast<double2*>(sbuf) + ((long long)sct * W + w) * sstride;
   for (int e = tid; e < nn; e += kGjThreads) {
@@ -350,7 +366,6 @@ __device__ __forceinline__ void gj_body(int W, int no0, int no1, double* sbuf, l
         v0[c] = in0 && c < b ? A[lane * ld + k0 + c] : zero;
         v1[c] = in1 && c < b ? A[(lane + 32) * ld + k0 + c] : zero;
       }
-      unsigned long long rows = 0ull;
 #pragma unroll
       for (int m = 0; m < kGjPanel; ++m) {
         if (m < b) {
@@ -362,62 +377,78 @@ __device__ __forceinline__ void gj_body(int W, int no0, int no1, double* sbuf, l
           const double2 ip = make_double2(p.x * inv, -p.y * inv);
           const bool mine0 = !hi && lane == owner, mine1 = hi && lane == owner;
           const double2 f0 = v0[m], f1 = v1[m];
+          P[lane * kGjPanel + m] = f0;
+          P[(lane + 32) * kGjPanel + m] = f1;
 #pragma unroll
           for (int c = 0; c < kGjPanel; ++c) {
             if (c == m) continue;
-            const double2 s = cmul(shfl2(hi ? v1[c] : v0[c], owner), ip);
-            v0[c] = mine0 ? s : csub(v0[c], cmul(f0, s));
-            v1[c] = mine1 ? s : csub(v1[c], cmul(f1, s));
+            const double2 s = gj_mul(shfl2(hi ? v1[c] : v0[c], owner), ip);
+            const double2 t0 = csub(v0[c], gj_mul(f0, s)), t1 = csub(v1[c], gj_mul(f1, s));
+            v0[c] = mine0 ? v0[c] : t0;
+            v1[c] = mine1 ? v1[c] : t1;
           }
-          const double2 q0 = cmul(f0, ip), q1 = cmul(f1, ip);
-          v0[m] = mine0 ? ip : make_double2(-q0.x, -q0.y);
-          v1[m] = mine1 ? ip : make_double2(-q1.x, -q1.y);
+          const double2 q0 = gj_mul(f0, ip), q1 = gj_mul(f1, ip);
+          v0[m] = mine0 ? make_double2(1.0, 0.0) : make_double2(-q0.x, -q0.y);
+          v1[m] = mine1 ? make_double2(1.0, 0.0) : make_double2(-q1.x, -q1.y);
           used0 |= mine0;
           used1 |= mine1;
-          rows |= 1ull << rn;
-          det = cmul(det, p);
-          if (lane == 0) piv[k0 + m] = rn;
+          det = gj_mul(p, det);
+          if (lane == 0) {
+            piv[k0 + m] = rn;
+            ipks[k0 + m] = ip;
+          }
         }
       }
-      if (lane == 0) rows_s = rows;
 #pragma unroll
       for (int c = 0; c < kGjPanel; ++c) {
-        if (c < b && in0) A[lane * ld + k0 + c] = P[lane * kGjPanel + c] = v0[c];
-        if (c < b && in1) A[(lane + 32) * ld + k0 + c] = P[(lane + 32) * kGjPanel + c] = v1[c];
+        if (c < b && in0) A[lane * ld + k0 + c] = v0[c];
+        if (c < b && in1) A[(lane + 32) * ld + k0 + c] = v1[c];
       }
     }
     __syncthreads();
     const int cols = no - b;
     if (cols > 0) {
-      const unsigned long long rows = rows_s;
       // column tiles of at most kGjThreads columns never occur (no <= 64)
       const int rg = kGjThreads / cols, jt = tid % cols, r0 = tid / cols;
       const int j = jt < k0 ? jt : jt + b;
-      double2 u[kGjPanel];
+      int r[kGjPanel];
+      double2 u[kGjPanel];  // the pivot rows' entries, then s_m
       if (r0 < rg) {
 #pragma unroll
-        for (int m = 0; m < kGjPanel; ++m) u[m] = m < b ? A[piv[k0 + m] * ld + j] : zero;
+        for (int m = 0; m < kGjPanel; ++m) {
+          r[m] = m < b ? piv[k0 + m] : 0;
+          u[m] = m < b ? A[r[m] * ld + j] : zero;
+        }
+#pragma unroll
+        for (int m = 0; m < kGjPanel; ++m)
+          if (m < b) {
+            u[m] = gj_mul(u[m], ipks[k0 + m]);
+#pragma unroll
+            for (int l = m + 1; l < kGjPanel; ++l)
+              if (l < b) u[l] = csub(u[l], gj_mul(P[r[l] * kGjPanel + m], u[m]));
+          }
       }
       __syncthreads();
       if (r0 < rg)
+#pragma unroll 2
         for (int i = r0; i < no; i += rg) {
-          double2 x = (rows >> i) & 1ull ? zero : A[i * ld + j];
+          double2 x = A[i * ld + j];
           const double2* pr = P + i * kGjPanel;
-          double2 y = zero;  // two chains
 #pragma unroll
-          for (int m = 0; m < kGjPanel; m += 2) {
-            if (m < b) x = cadd(x, cmul(pr[m], u[m]));
-            if (m + 1 < b) y = cadd(y, cmul(pr[m + 1], u[m + 1]));
-          }
-          A[i * ld + j] = cadd(x, y);
+          for (int m = 0; m < kGjPanel; ++m)
+            if (m < b) {
+              const double2 t = csub(x, gj_mul(pr[m], u[m]));
+              x = i == r[m] ? x : t;
+            }
+          A[i * ld + j] = x;
         }
       __syncthreads();
     }
   }
-  // unscramble: S^-1[i][r_k] = X[r_i][k]
+  // unscramble with the row scales: S^-1[i][r_k] = X[r_i][k] = A[r_i][k] / p_i
   for (int e = tid; e < nn; e += kGjThreads) {
     const int i = e / no, k = e - (e / no) * no;
-    g[i * no + piv[k]] = A[piv[i] * ld + k];
+    g[i * no + piv[k]] = gj_mul(ipks[i], A[piv[i] * ld + k]);
   }
   if (tid == 0) {
     // sign of the permutation k -> r_k: (-1)^(no - cycles)
