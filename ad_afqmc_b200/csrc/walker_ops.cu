@@ -186,160 +186,226 @@ __device__ void qr_inplace(double2* A, int lda, int N, int no, double2* tau, dou
   __syncthreads();
 }
 
-// ---- the same factorisation with each warp's column rows in registers ----
-// Lane l holds rows r0 + l + 32 t (t < RPL) of the column it works on, where
-// r0 is the reflector's first row; N <= 32 RPL.  All RPL loads of a column are
-// in flight together and the product and update run on registers, so a
-// column step costs one round of loads, the shuffles and one round of stores.
+// ---- panels of four reflectors, columns in registers -----------------------
+// Lane l holds rows k0 + l + 32 t (t < RPL) of the column it works on, where k0
+// is the panel's first row; N <= 32 RPL.  A panel's reflectors v_m (unit entry
+// and zeros written out) sit in shared memory, with G_ml = v_m^H v_l, so a column is
+// loaded and stored once for four of them:
+//   w_m = v_m^H a (four products reduced together),
+//   c_m = conj(tau_m) (w_m - sum_{l<m} G_ml c_l),   a -= sum_m v_m c_m
+// which is the four reflectors one after the other (the same for Q, last to
+// first, with tau_m and conj(G_lm)).  Warp 0 forms a panel on its own.  One
+// reflector at a time, a block barrier, a shuffle reduction and a pass over the
+// columns for each, took 17.4 ms at N = 300 (60 + 58 columns, 1024 walkers, rows from
+// L2) and 0.76 ms at N = 157 (39 columns, 231 walkers); this takes 8.3 and 0.45 ms.
+constexpr int kQrPanel = 4;
+
 template <int RPL>
-__device__ __forceinline__ void rcol_load(const double2* A, int lda, int N, int r0, int j,
-                                          double2 (&a)[RPL]) {
+__device__ __forceinline__ void qcol_load(const double2* A, int lda, int N, int k0, int j, double2 (&a)[RPL]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int t = 0; t < RPL; ++t) {
-    const int p = r0 + lane + 32 * t;
+    const int p = k0 + lane + 32 * t;
     a[t] = p < N ? A[p * lda + j] : make_double2(0.0, 0.0);
   }
 }
 
 template <int RPL>
-__device__ __forceinline__ void rcol_store(double2* A, int lda, int N, int r0, int j,
-                                           const double2 (&a)[RPL]) {
+__device__ __forceinline__ void qcol_store(double2* A, int lda, int N, int k0, int j, const double2 (&a)[RPL]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int t = 0; t < RPL; ++t) {
-    const int p = r0 + lane + 32 * t;
+    const int p = k0 + lane + 32 * t;
     if (p < N) A[p * lda + j] = a[t];
   }
 }
 
-// a -= c v (v^H a); rows beyond N hold zeros in both
+// w[m] = v_m^H a for m < nm, in every lane; V: [kQrPanel][32 RPL] rows from k0
 template <int RPL>
-__device__ __forceinline__ void rcol_reflect(double2 (&a)[RPL], const double2 (&v)[RPL], double2 c) {
-  double2 w0 = make_double2(0.0, 0.0), w1 = make_double2(0.0, 0.0);
-#pragma unroll
-  for (int t = 0; t < RPL; ++t) {
-    if (t & 1)
-      w1 = cadd(w1, cmul(cconj(v[t]), a[t]));
-    else
-      w0 = cadd(w0, cmul(cconj(v[t]), a[t]));
-  }
-  const double2 cw = cmul(c, warp_sum2(cadd(w0, w1)));
-#pragma unroll
-  for (int t = 0; t < RPL; ++t) a[t] = csub(a[t], cmul(v[t], cw));
-}
-
-// reflector k (zlarfg) of a column held from row k - d: pivot in lane d, t = 0
-template <int RPL>
-__device__ __forceinline__ void rcol_reflector(double2 (&a)[RPL], int d, int k, double2* tau,
-                                               double* beta) {
+__device__ __forceinline__ void qcol_dots(const double2* V, const double2 (&a)[RPL], int nm,
+                                          double2 (&w)[kQrPanel]) {
   const int lane = threadIdx.x & 31;
-  double s = 0.0;
 #pragma unroll
-  for (int t = 0; t < RPL; ++t)
-    if (t > 0 || lane > d) s += a[t].x * a[t].x + a[t].y * a[t].y;
-  s = warp_sum(s);
-  const double2 al = make_double2(__shfl_sync(0xffffffffu, a[0].x, d), __shfl_sync(0xffffffffu, a[0].y, d));
-  double2 tk, sc;
-  double b;
-  if (s == 0.0 && al.y == 0.0) {
-    tk = make_double2(0.0, 0.0);
-    b = al.x;
-    sc = make_double2(1.0, 0.0);
-  } else {
-    b = -copysign(sqrt(al.x * al.x + al.y * al.y + s), al.x);
-    tk = make_double2((b - al.x) / b, -al.y / b);
-    sc = cdiv(make_double2(1.0, 0.0), make_double2(al.x - b, al.y));
+  for (int m = 0; m < kQrPanel; ++m) {
+    w[m] = make_double2(0.0, 0.0);
+    if (m < nm) {
+#pragma unroll
+      for (int t = 0; t < RPL; ++t) w[m] = cadd(w[m], cmul(cconj(V[m * 32 * RPL + lane + 32 * t]), a[t]));
+    }
   }
 #pragma unroll
-  for (int t = 0; t < RPL; ++t)
-    if (t > 0 || lane > d) a[t] = cmul(a[t], sc);
-  if (lane == d) a[0] = make_double2(b, 0.0);
-  if (lane == 0) {
-    tau[k] = tk;
-    beta[k] = b;
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int m = 0; m < kQrPanel; ++m) {
+      w[m].x += __shfl_xor_sync(0xffffffffu, w[m].x, o);
+      w[m].y += __shfl_xor_sync(0xffffffffu, w[m].y, o);
+    }
+}
+
+// a -= sum_m v_m c_m
+template <int RPL>
+__device__ __forceinline__ void qcol_update(const double2* V, double2 (&a)[RPL], int nm,
+                                            const double2 (&c)[kQrPanel]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int m = 0; m < kQrPanel; ++m)
+    if (m < nm) {
+#pragma unroll
+      for (int t = 0; t < RPL; ++t) a[t] = csub(a[t], cmul(V[m * 32 * RPL + lane + 32 * t], c[m]));
+    }
+}
+
+// c of H_{nm-1}^H ... H_0^H (geqr2's order)
+__device__ __forceinline__ void qr_coeff_fwd(const double2* tau, const double2* G, int nm,
+                                             const double2 (&w)[kQrPanel], double2 (&c)[kQrPanel]) {
+#pragma unroll
+  for (int m = 0; m < kQrPanel; ++m) {
+    c[m] = make_double2(0.0, 0.0);
+    if (m < nm) {
+      double2 r = w[m];
+#pragma unroll
+      for (int l = 0; l < m; ++l) r = csub(r, cmul(G[m * kQrPanel + l], c[l]));
+      c[m] = cmul(cconj(tau[m]), r);
+    }
   }
 }
 
-// the reflector's rows r0 + l + 32 t (v_r0 = 1) into registers
 template <int RPL>
-__device__ __forceinline__ void rcol_vector(const double2* A, int lda, int N, int r0,
-                                            double2 (&v)[RPL]) {
-  rcol_load<RPL>(A, lda, N, r0, r0, v);
-  if ((threadIdx.x & 31) == 0) v[0] = make_double2(1.0, 0.0);
-}
-
-template <int RPL>
-__device__ void qr_inplace_reg(double2* A, int lda, int N, int no, double2* tau, double* beta) {
+__device__ void qr_inplace_panel(double2* A, int lda, int N, int no, double2* tau, double* beta, double2* V,
+                                 double2* G) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  double2 v[RPL], a[RPL];
-  // ---- geqr2 ----------------------------------------------------------------
-  if (warp == 0) {
-    rcol_load<RPL>(A, lda, N, 0, 0, a);
-    rcol_reflector<RPL>(a, 0, 0, tau, beta);
-    rcol_store<RPL>(A, lda, N, 0, 0, a);
-  }
-  __syncthreads();
-  for (int k = 0; k + 1 < no; ++k) {
-    const double2 ct = cconj(tau[k]);
-    const bool active = ct.x != 0.0 || ct.y != 0.0;
-    const int j0 = qr_first_col(k, warp, nw);
-    if (j0 < no) {
-      rcol_vector<RPL>(A, lda, N, k, v);
-      for (int j = j0; j < no; j += nw) {
-        rcol_load<RPL>(A, lda, N, k, j, a);
-        if (active) rcol_reflect<RPL>(a, v, ct);
-        if (j == k + 1) rcol_reflector<RPL>(a, 1, k + 1, tau, beta);
-        rcol_store<RPL>(A, lda, N, k, j, a);
-      }
-    }
-    __syncthreads();
-  }
-  // ---- zung2r ---------------------------------------------------------------
-  for (int i = no - 2; i >= 0; --i) {
-    const double2 ti = tau[i];
-    const bool active = ti.x != 0.0 || ti.y != 0.0;
-    const int j0 = qr_first_col(i, warp, nw);
-    if (j0 < no) {
-      rcol_vector<RPL>(A, lda, N, i, v);
-      for (int j = j0; j < no; j += nw) {
-        rcol_load<RPL>(A, lda, N, i, j, a);
-        if (j == i + 1) {  // column j of Q from reflector j: window starts one row above it
-          const double2 tj = tau[j];
-#pragma unroll
-          for (int t = 0; t < RPL; ++t) {
-            if (t == 0 && lane == 0) a[t] = make_double2(0.0, 0.0);
-            else if (t == 0 && lane == 1) a[t] = make_double2(1.0 - tj.x, -tj.y);
-            else a[t] = cmul(make_double2(-tj.x, -tj.y), a[t]);
-          }
-          for (int p = lane; p < i; p += 32) A[p * lda + j] = make_double2(0.0, 0.0);
+  constexpr int NV = 32 * RPL;
+  double2 a[RPL], w[kQrPanel], c[kQrPanel];
+  // ---- geqr2: reflectors below the diagonal, R's diagonal in beta ------------
+  for (int k0 = 0; k0 < no; k0 += kQrPanel) {
+    const int b = min(kQrPanel, no - k0);
+    if (warp == 0) {
+#pragma unroll 1
+      for (int m = 0; m < b; ++m) {
+        const int k = k0 + m;
+        qcol_load<RPL>(A, lda, N, k0, k, a);
+        if (m > 0) {
+          qcol_dots<RPL>(V, a, m, w);
+          qr_coeff_fwd(tau + k0, G, m, w, c);
+          qcol_update<RPL>(V, a, m, c);
         }
-        if (active) rcol_reflect<RPL>(a, v, ti);
-        rcol_store<RPL>(A, lda, N, i, j, a);
+        // zlarfg: the pivot is lane m's first row
+        double s = 0.0;
+#pragma unroll
+        for (int t = 0; t < RPL; ++t)
+          if (t > 0 || lane > m) s += a[t].x * a[t].x + a[t].y * a[t].y;
+        s = warp_sum(s);
+        const double2 al =
+            make_double2(__shfl_sync(0xffffffffu, a[0].x, m), __shfl_sync(0xffffffffu, a[0].y, m));
+        double2 tk, sc;
+        double bt;
+        if (s == 0.0 && al.y == 0.0) {
+          tk = make_double2(0.0, 0.0);
+          bt = al.x;
+          sc = make_double2(1.0, 0.0);
+        } else {
+          bt = -copysign(sqrt(al.x * al.x + al.y * al.y + s), al.x);
+          tk = make_double2((bt - al.x) / bt, -al.y / bt);
+          sc = cdiv(make_double2(1.0, 0.0), make_double2(al.x - bt, al.y));
+        }
+#pragma unroll
+        for (int t = 0; t < RPL; ++t) {
+          const bool below = t > 0 || lane > m;
+          a[t] = below ? cmul(a[t], sc)
+                       : (lane == m ? make_double2(1.0, 0.0) : make_double2(0.0, 0.0));
+          V[m * NV + lane + 32 * t] = a[t];
+          const int p = k0 + lane + 32 * t;
+          if (below && p < N) A[p * lda + k] = a[t];
+        }
+        if (lane == 0) {
+          tau[k] = tk;
+          beta[k] = bt;
+        }
+        __syncwarp();
+        if (m > 0) {  // G_ml = v_m^H v_l = conj(v_l^H v_m)
+          qcol_dots<RPL>(V, a, m, w);
+          if (lane == 0) {
+#pragma unroll
+            for (int l = 0; l < kQrPanel; ++l)
+              if (l < m) G[m * kQrPanel + l] = cconj(w[l]);
+          }
+          __syncwarp();
+        }
       }
     }
     __syncthreads();
+    for (int j = k0 + b + warp; j < no; j += nw) {
+      qcol_load<RPL>(A, lda, N, k0, j, a);
+      qcol_dots<RPL>(V, a, b, w);
+      qr_coeff_fwd(tau + k0, G, b, w, c);
+      qcol_update<RPL>(V, a, b, c);
+      qcol_store<RPL>(A, lda, N, k0, j, a);
+    }
+    __syncthreads();
   }
-  if (warp == 0) {  // column 0 of Q
-    rcol_load<RPL>(A, lda, N, 0, 0, a);
-    const double2 t0 = tau[0];
+  // ---- zung2r: Q's columns, panels last to first -------------------------------
+  for (int k0 = (no - 1) / kQrPanel * kQrPanel; k0 >= 0; k0 -= kQrPanel) {
+    const int b = min(kQrPanel, no - k0);
+    for (int e = threadIdx.x; e < b * NV; e += blockDim.x) {
+      const int m = e / NV, r = e - m * NV, p = k0 + r;
+      V[e] = r < m || p >= N ? make_double2(0.0, 0.0)
+                             : (r == m ? make_double2(1.0, 0.0) : A[p * lda + k0 + m]);
+    }
+    __syncthreads();
+    if (warp < kQrPanel && warp < b && warp > 0) {
 #pragma unroll
-    for (int t = 0; t < RPL; ++t)
-      a[t] = (t == 0 && lane == 0) ? make_double2(1.0 - t0.x, -t0.y) : cmul(make_double2(-t0.x, -t0.y), a[t]);
-    rcol_store<RPL>(A, lda, N, 0, 0, a);
+      for (int t = 0; t < RPL; ++t) a[t] = V[warp * NV + lane + 32 * t];
+      qcol_dots<RPL>(V, a, warp, w);
+      if (lane == 0) {
+#pragma unroll
+        for (int l = 0; l < kQrPanel; ++l)
+          if (l < warp) G[warp * kQrPanel + l] = cconj(w[l]);
+      }
+    }
+    __syncthreads();
+    for (int j = k0 + warp; j < no; j += nw) {
+      const int own = j - k0;  // < b: a column of this panel, starting from e_j
+#pragma unroll
+      for (int t = 0; t < RPL; ++t) {
+        const int r = lane + 32 * t, p = k0 + r;
+        a[t] = make_double2(0.0, 0.0);
+        if (own < b) {
+          if (r == own) a[t] = make_double2(1.0, 0.0);
+        } else if (r >= b && p < N) {  // the rows above belong to R
+          a[t] = A[p * lda + j];
+        }
+      }
+      qcol_dots<RPL>(V, a, b, w);
+      const int nm = own < b ? own + 1 : b;  // H_l e_j = e_j for l > j
+#pragma unroll
+      for (int m = kQrPanel - 1; m >= 0; --m) {
+        c[m] = make_double2(0.0, 0.0);
+        if (m < nm) {
+          double2 r = w[m];
+#pragma unroll
+          for (int l = m + 1; l < kQrPanel; ++l)
+            if (l < nm) r = csub(r, cmul(cconj(G[l * kQrPanel + m]), c[l]));
+          c[m] = cmul(tau[k0 + m], r);
+        }
+      }
+      qcol_update<RPL>(V, a, nm, c);
+      qcol_store<RPL>(A, lda, N, k0, j, a);
+    }
+    __syncthreads();
   }
-  __syncthreads();
 }
 
 // grid (W, ns).  use_smem: walker copied to shared memory with row stride no+1.
-// RPL > 0: register-resident columns (N <= 32 RPL, 512 threads); 0: the loop
-// form for any N (1024 threads).
+// RPL > 0: panels, register-resident columns (N <= 32 RPL, 512 threads; four
+// reflectors of 32 RPL rows behind the walker in shared memory); 0: the loop form for
+// any N (1024 threads).
 template <int RPL>
 __device__ __forceinline__ void qr_walker(int N, int no0, int no1, double* w0, double* w1,
                                           int sign_fix, int use_smem, double* sector_norm) {
   extern __shared__ double2 qsm[];
   __shared__ double2 tau[64];
   __shared__ double beta[64];
+  __shared__ double2 G_[kQrPanel * kQrPanel];
   const int w = blockIdx.x, s = blockIdx.y;
   const int no = s ? no1 : no0;
   double2* G = reinterpret_cast<double2*>(s ? w1 : w0) + (long long)w * N * no;
@@ -355,7 +421,7 @@ __device__ __forceinline__ void qr_walker(int N, int no0, int no1, double* w0, d
     __syncthreads();
   }
   if (RPL > 0)
-    qr_inplace_reg<(RPL > 0 ? RPL : 1)>(A, lda, N, no, tau, beta);
+    qr_inplace_panel<(RPL > 0 ? RPL : 1)>(A, lda, N, no, tau, beta, qsm + (use_smem ? N * lda : 0), G_);
   else
     qr_inplace(A, lda, N, no, tau, beta);
   // prod diag R (real) and optional sign fix of column 0
@@ -602,6 +668,7 @@ cudaError_t launch_qr(const Layout& L, double* const walkers[2], double* norms, 
   const size_t smem = size_t(L.N) * (L.nomax + 1) * sizeof(double2);
   const int use_smem = smem <= 200 * 1024 && L.tune.qr_mode != 2;
   const size_t dyn = use_smem ? smem : 0;
+  auto panel = [](int rpl) { return size_t(kQrPanel) * 32 * rpl * sizeof(double2); };
   double* secn = work;  // (ns, W) doubles of scratch at the start of the workspace
   dim3 grid(L.W, L.ns);
   cudaError_t e;
@@ -609,15 +676,15 @@ cudaError_t launch_qr(const Layout& L, double* const walkers[2], double* norms, 
     ProfScope ps(K_QR, st);
     const int N = L.N, T = kQrRegThreads;
     if (N <= 32)
-      e = launch_qr_kernel(qr_reg_kernel<1>, T, grid, dyn, st, L, walkers, use_smem, secn);
+      e = launch_qr_kernel(qr_reg_kernel<1>, T, grid, dyn + panel(1), st, L, walkers, use_smem, secn);
     else if (N <= 64)
-      e = launch_qr_kernel(qr_reg_kernel<2>, T, grid, dyn, st, L, walkers, use_smem, secn);
+      e = launch_qr_kernel(qr_reg_kernel<2>, T, grid, dyn + panel(2), st, L, walkers, use_smem, secn);
     else if (N <= 128)
-      e = launch_qr_kernel(qr_reg_kernel<4>, T, grid, dyn, st, L, walkers, use_smem, secn);
+      e = launch_qr_kernel(qr_reg_kernel<4>, T, grid, dyn + panel(4), st, L, walkers, use_smem, secn);
     else if (N <= 224)
-      e = launch_qr_kernel(qr_reg_kernel<7>, T, grid, dyn, st, L, walkers, use_smem, secn);
+      e = launch_qr_kernel(qr_reg_kernel<7>, T, grid, dyn + panel(7), st, L, walkers, use_smem, secn);
     else if (N <= 320)
-      e = launch_qr_kernel(qr_reg_kernel<10>, T, grid, dyn, st, L, walkers, use_smem, secn);
+      e = launch_qr_kernel(qr_reg_kernel<10>, T, grid, dyn + panel(10), st, L, walkers, use_smem, secn);
     else
       e = launch_qr_kernel(qr_kernel, kQrThreads, grid, dyn, st, L, walkers, use_smem, secn);
   }
