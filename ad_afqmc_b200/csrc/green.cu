@@ -44,13 +44,21 @@ __device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_g
 // and its outputs from S^-1 in a.sbuf (the inverse and det by gj_kernel).
 // T threads: one warp per column tile of 8 real columns (2 No of them), at least
 // eight (see green_threads).
+// What bounds it: the FP64 tensor cores and the instructions around them (18 us for
+// S and 36 us for Theta of the former at N = 200, No = 40, 512 walkers).  The warp's tile of
+// S^-1 is laid out once in registers for all rows of Theta, and the inner loops
+// hold loads and MMAs only: entries beyond the matrices are read as they stand
+// where they reach nothing that is stored.  S + Theta there 177 -> 125 us, at N = 300,
+// No = 60 + 58, 1024 walkers 2.26 -> 1.72 ms, with every fragment rebuilt and
+// range-checked for each MMA before.
 template <int T>
 __device__ __forceinline__ void green_body(const GreenArgs& a, int mode, int w, int sct) {
   extern __shared__ double2 sm[];
   const GreenSector& S_ = a.sec[sct];
   const int N = a.N, no = S_.no, tid = threadIdx.x;
-  constexpr int NW = T / 32;                 // warps
-  constexpr int SL = 1;                      // column tiles per warp
+  // row tiles of S and k-steps of Theta at the widest No of this T (green_threads)
+  constexpr int MT = T == 256 ? 4 : (T == 320 ? 5 : (T == 384 ? 6 : 8));
+  constexpr int KS = 4 * MT;
 
   double2* S = sm;                          // no*no
   double2* colk = S + no * no;              // 64
@@ -74,7 +82,7 @@ __device__ __forceinline__ void green_body(const GreenArgs& a, int mode, int w, 
   // ---- S = C^T W on the FP64 tensor cores ----------------------------------
   // As real matrices: S (No x 2No, (re, im) interleaved) = C^T (No x N) times
   // W (N x 2No, the complex walker viewed as doubles).  mma.m8n8k4 tiles: warp
-  // w owns column tiles w and w + 8 and every row tile, so each B fragment is
+  // w owns column tile w and every row tile, so each B fragment is
   // loaded once per k-step.  Rows of W and C are staged 32 at a time.
   const int warp = tid >> 5, lane = tid & 31;
   const int nc2 = 2 * no;
@@ -96,11 +104,9 @@ __device__ __forceinline__ void green_body(const GreenArgs& a, int mode, int w, 
                        : nullptr;
   const int npairs = no * no;
   if (mode != 2) {
-  double sacc[SL][8][2];
+  double sacc[MT][2];
 #pragma unroll
-  for (int sl = 0; sl < SL; ++sl)
-#pragma unroll
-    for (int mi = 0; mi < 8; ++mi) sacc[sl][mi][0] = sacc[sl][mi][1] = 0.0;
+  for (int mi = 0; mi < MT; ++mi) sacc[mi][0] = sacc[mi][1] = 0.0;
   load_chunk(0, true);
   for (int c = 0; c < nchunks; ++c) {
     const int p0 = c * kRowChunk, rows = min(kRowChunk, N - p0);
@@ -108,45 +114,53 @@ __device__ __forceinline__ void green_body(const GreenArgs& a, int mode, int w, 
     else cp_async_commit();  // an empty group keeps the wait count uniform
     cp_async_wait1();
     __syncthreads();
-    const double* stageD = reinterpret_cast<const double*>(stage + (c & 1) * sbuf_);
-    const double* mocc = moc + (c & 1) * kRowChunk * no;
-    for (int kk = 0; kk < rows; kk += 4) {
-      const int kr = kk + (lane & 3);
-      const bool kin = kr < rows;
-      double afr[8];
+    if (warp < ntiles) {  // warp-uniform
+      // lane (r = lane / 4, q = lane % 4): A[m = 8 mi + r][k = q], B[k = q][n = 8 warp + r];
+      // entries beyond No and 2 No (what follows in shared memory) only reach rows
+      // and columns of S that are not stored
+      const double* bp = reinterpret_cast<const double*>(stage + (c & 1) * sbuf_) + (lane & 3) * sd +
+                         warp * 8 + (lane >> 2);
+      const double* ap = moc + (c & 1) * kRowChunk * no + (lane & 3) * no + (lane >> 2);
+      auto tiles = [&](auto count) {  // the first M row tiles
+        constexpr int M = decltype(count)::value;
+        const int full = rows & ~3;
+#pragma unroll 2
+        for (int kk = 0; kk < full; kk += 4) {
+          const double b = bp[kk * sd];
+          double afr[M];
 #pragma unroll
-      for (int mi = 0; mi < 8; ++mi) {
-        const int m = mi * 8 + (lane >> 2);
-        afr[mi] = (mi < mtiles && kin && m < no) ? mocc[kr * no + m] : 0.0;
-      }
+          for (int mi = 0; mi < M; ++mi) afr[mi] = ap[kk * no + mi * 8];
 #pragma unroll
-      for (int sl = 0; sl < SL; ++sl) {
-        const int ni = warp + sl * NW;
-        if (ni < ntiles) {  // warp-uniform
-          const int n = ni * 8 + (lane >> 2);
-          const double b = (kin && n < nc2) ? stageD[kr * sd + n] : 0.0;
-#pragma unroll
-          for (int mi = 0; mi < 8; ++mi)
-            if (mi < mtiles) dmma_8x8x4(sacc[sl][mi][0], sacc[sl][mi][1], afr[mi], b);
+          for (int mi = 0; mi < M; ++mi) dmma_8x8x4(sacc[mi][0], sacc[mi][1], afr[mi], b);
         }
-      }
+        if (full < rows) {
+          const bool kin = full + (lane & 3) < rows;
+          const double b = kin ? bp[full * sd] : 0.0;
+#pragma unroll
+          for (int mi = 0; mi < M; ++mi)
+            dmma_8x8x4(sacc[mi][0], sacc[mi][1], kin ? ap[full * no + mi * 8] : 0.0, b);
+        }
+      };
+      // sectors and fragments smaller than the launch's widest work on fewer tiles
+      if (mtiles <= 2)
+        tiles(std::integral_constant<int, 2>{});
+      else if (mtiles <= 4)
+        tiles(std::integral_constant<int, 4>{});
+      else
+        tiles(std::integral_constant<int, MT>{});
     }
     __syncthreads();
   }
+  if (warp < ntiles) {
 #pragma unroll
-  for (int sl = 0; sl < SL; ++sl) {
-    const int ni = warp + sl * NW;
-    if (ni < ntiles) {
-#pragma unroll
-      for (int mi = 0; mi < 8; ++mi) {
-        const int i = mi * 8 + (lane >> 2), j = ni * 4 + (lane & 3);
-        if (mi < mtiles && i < no && j < no) {
-          const double2 v = make_double2(sacc[sl][mi][0], sacc[sl][mi][1]);
-          if (mode == 1)
-            sg[i * no + j] = v;
-          else
-            S[i * no + j] = v;
-        }
+    for (int mi = 0; mi < MT; ++mi) {
+      const int i = mi * 8 + (lane >> 2), j = warp * 4 + (lane & 3);
+      if (i < no && j < no) {
+        const double2 v = make_double2(sacc[mi][0], sacc[mi][1]);
+        if (mode == 1)
+          sg[i * no + j] = v;
+        else
+          S[i * no + j] = v;
       }
     }
   }
@@ -179,6 +193,23 @@ __device__ __forceinline__ void green_body(const GreenArgs& a, int mode, int w, 
   const bool gb = a.gplb[0] != nullptr;
   const bool tb = S_.gtb[0] != nullptr;
   load_chunk(0, false);
+  // Theta rows (N x 2No real) = W rows (N x 2No) times the real form of
+  // S^-1: R[2i][2j] = R[2i+1][2j+1] = Re s_ij, R[2i][2j+1] = Im s_ij,
+  // R[2i+1][2j] = -Im s_ij.  A warp's column tile of it stays in registers for all rows.
+  const int ksteps = (nc2 + 3) >> 2;
+  double bfr[KS];
+  {
+    const int n = warp * 8 + (lane >> 2);
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      const int k = ks * 4 + (lane & 3);
+      bfr[ks] = 0.0;
+      if (k < nc2 && n < nc2) {
+        const double2 sv = S[(k >> 1) * no + (n >> 1)];
+        bfr[ks] = (k & 1) == 0 ? ((n & 1) == 0 ? sv.x : sv.y) : ((n & 1) == 0 ? -sv.y : sv.x);
+      }
+    }
+  }
   for (int c = 0; c < nchunks; ++c) {
     const int p0 = c * kRowChunk, rows = min(kRowChunk, N - p0);
     // walker rows of the next chunk stream in while this one is processed
@@ -187,57 +218,46 @@ __device__ __forceinline__ void green_body(const GreenArgs& a, int mode, int w, 
     cp_async_wait1();
     __syncthreads();
     const double* stageD = reinterpret_cast<const double*>(stage + (c & 1) * sbuf_);
-    // Theta rows (N x 2No real) = W rows (N x 2No) times the real form of
-    // S^-1: R[2i][2j] = R[2i+1][2j+1] = Re s_ij, R[2i][2j+1] = Im s_ij,
-    // R[2i+1][2j] = -Im s_ij, generated in the B fragments
-    {
+    if (warp < ntiles) {
       const int rtiles = (rows + 7) >> 3;  // <= 4
-      double tacc[SL][4][2];
+      double tacc[4][2];
 #pragma unroll
-      for (int sl = 0; sl < SL; ++sl)
+      for (int ri = 0; ri < 4; ++ri) tacc[ri][0] = tacc[ri][1] = 0.0;
+      // rows beyond the chunk's (left from another chunk) only reach rows not stored
+      const double* ap = stageD + (lane >> 2) * sd + (lane & 3);
+      if (rtiles == 4) {
 #pragma unroll
-        for (int ri = 0; ri < 4; ++ri) tacc[sl][ri][0] = tacc[sl][ri][1] = 0.0;
-      for (int kk = 0; kk < nc2; kk += 4) {
-        const int k = kk + (lane & 3);
-        const bool kin = k < nc2;
-        double afr[4];
+        for (int ks = 0; ks < KS; ++ks) {
+          if (ks >= ksteps) break;
+          const bool kin = ks * 4 + (lane & 3) < nc2;
+          double afr[4];
 #pragma unroll
-        for (int ri = 0; ri < 4; ++ri) {
-          const int r = ri * 8 + (lane >> 2);
-          afr[ri] = (ri < rtiles && kin && r < rows) ? stageD[r * sd + k] : 0.0;
+          for (int ri = 0; ri < 4; ++ri) afr[ri] = kin ? ap[ri * 8 * sd + ks * 4] : 0.0;
+#pragma unroll
+          for (int ri = 0; ri < 4; ++ri) dmma_8x8x4(tacc[ri][0], tacc[ri][1], afr[ri], bfr[ks]);
         }
+      } else {
 #pragma unroll
-        for (int sl = 0; sl < SL; ++sl) {
-          const int ni = warp + sl * NW;
-          if (ni < ntiles) {  // warp-uniform
-            const int n = ni * 8 + (lane >> 2);
-            double b = 0.0;
-            if (kin && n < nc2) {
-              const double2 sv = S[(k >> 1) * no + (n >> 1)];
-              b = (k & 1) == 0 ? ((n & 1) == 0 ? sv.x : sv.y) : ((n & 1) == 0 ? -sv.y : sv.x);
-            }
+        for (int ks = 0; ks < KS; ++ks) {
+          if (ks >= ksteps) break;
+          const bool kin = ks * 4 + (lane & 3) < nc2;
 #pragma unroll
-            for (int ri = 0; ri < 4; ++ri)
-              if (ri < rtiles) dmma_8x8x4(tacc[sl][ri][0], tacc[sl][ri][1], afr[ri], b);
-          }
+          for (int ri = 0; ri < 3; ++ri)
+            if (ri < rtiles)
+              dmma_8x8x4(tacc[ri][0], tacc[ri][1], kin ? ap[ri * 8 * sd + ks * 4] : 0.0, bfr[ks]);
         }
       }
 #pragma unroll
-      for (int sl = 0; sl < SL; ++sl) {
-        const int ni = warp + sl * NW;
-        if (ni >= ntiles) continue;
-#pragma unroll
-        for (int ri = 0; ri < 4; ++ri) {
-          const int r = ri * 8 + (lane >> 2), j = ni * 4 + (lane & 3);
-          if (ri < rtiles && r < rows && j < no) {
-            const double2 sv = make_double2(tacc[sl][ri][0], tacc[sl][ri][1]);
-            tstage[r * ts + j] = sv;
-            if (th) th[(long long)(p0 + r) * no + j] = sv;
-            if (S_.rh1) {
-              const double h = S_.rh1[(long long)j * N + p0 + r];
-              e1.x = fma(sv.x, h, e1.x);
-              e1.y = fma(sv.y, h, e1.y);
-            }
+      for (int ri = 0; ri < 4; ++ri) {
+        const int r = ri * 8 + (lane >> 2), j = warp * 4 + (lane & 3);
+        if (r < rows && j < no) {
+          const double2 sv = make_double2(tacc[ri][0], tacc[ri][1]);
+          tstage[r * ts + j] = sv;
+          if (th) th[(long long)(p0 + r) * no + j] = sv;
+          if (S_.rh1) {
+            const double h = S_.rh1[(long long)j * N + p0 + r];
+            e1.x = fma(sv.x, h, e1.x);
+            e1.y = fma(sv.y, h, e1.y);
           }
         }
       }
@@ -245,7 +265,7 @@ __device__ __forceinline__ void green_body(const GreenArgs& a, int mode, int w, 
     __syncthreads();
     if (go || gre || gb || tb) {
       for (int e = tid; e < rows * no; e += T) {
-        const int j = e / rows, r = e - (e / rows) * rows;
+        const int j = rows == kRowChunk ? e / kRowChunk : e / rows, r = e - j * rows;
         const double2 v = tstage[r * ts + j];
         if (go) go[(long long)j * N + p0 + r] = v;
         if (gre) {
@@ -468,12 +488,12 @@ __device__ __forceinline__ void gj_body(int W, int no0, int no1, double* sbuf, l
 }
 
 template <int T>
-__global__ void __launch_bounds__(T, T <= 384 ? 2 : 1) green_kernel(GreenArgs a, int mode) {
+__global__ void __launch_bounds__(T, T <= 320 ? 2 : 1) green_kernel(GreenArgs a, int mode) {
   green_body<T>(a, mode, blockIdx.x, blockIdx.y);
 }
 
 template <int T>
-__global__ void __launch_bounds__(T, T <= 384 ? 2 : 1) green_kernel_grouped(const GreenArgs* A, BlockMap m, int mode) {
+__global__ void __launch_bounds__(T, T <= 320 ? 2 : 1) green_kernel_grouped(const GreenArgs* A, BlockMap m, int mode) {
   int local;
   const GreenArgs& a = A[block_owner(m, blockIdx.x, local)];
   green_body<T>(a, mode, local % a.W, local / a.W);
