@@ -15,8 +15,8 @@ Knobs (0 = the built-in rule):
   vhs_bn, fb_bn     tensor-core column tile of the VHS / force-bias GEMMs
   fb_splitk         split-K of the force-bias GEMM
   exch_bn           tensor-core exchange column tile (walkers per tile)
-  f64_exch_bn       FP64 exchange tile (FP64 path, or spins whose tensor-core
-                    tile does not fit shared memory)
+  f64_exch_bn       row blocks of the FP64 exchange (FP64 path, or spins whose
+                    tensor-core tile does not fit shared memory)
   max_stages        cap on the tcgen05 pipeline depth
   prop_order        tile order of the tensor-core propagator launches: 0
                     alternates the direction over the walkers from one launch
