@@ -38,7 +38,7 @@ struct F64Shape {
   int mt, nt, nz;      // tiles along rows and columns, batches (or K splits)
   int arow_step;       // rows of A per tile
   int a_batched;       // A's third coordinate follows the batch
-  int gpw;             // column groups of 16 per walker (B_N with z = walker); 1 << 20: plain columns
+  int gpw;             // column groups of 16 per walker (B_N with z = walker); 1 << 30: plain columns
   int wpt;             // walkers per column tile (z advances by it), 0: z = batch
   int ksplit;          // nz splits K into chunks of this length (0: no split)
   int stages;

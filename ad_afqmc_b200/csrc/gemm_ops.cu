@@ -21,7 +21,7 @@ int sm_count();
 
 namespace {
 
-constexpr int kPlain = 1 << 20;  // column groups of a plain (not per-walker) operand
+constexpr int kPlain = 1 << 30;  // column groups of a plain (not per-walker) operand: more than any has (N^2 < 2^31)
 
 // ---------------------------------------------------------------------------
 // force bias: C[z] (2W x G) = Gpl (2W x Kfb) * RCcat^T, K split over z
