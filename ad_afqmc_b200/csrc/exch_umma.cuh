@@ -37,7 +37,7 @@ struct ExchParams {
   int gpt, wpt, mt, nt;    // tiling
   int ncw;                 // walker tiles per L2 chunk
   int arows, brows;        // box rows of A (multiple of 8) and B (multiple of 8)
-  int stages, gsub, lot;
+  int stages, gsub, wsub, lot;
   const bf16* a[2];        // row operand pieces (the TMEM kernel loads them itself), row stride lda
   long long lda;
   float4* cout;            // (W, G): tr f as pairs (re hi, re lo, im hi, im lo)
@@ -45,9 +45,9 @@ struct ExchParams {
   int* err;
 };
 
-// float2 per staged row: wpt No (re, im) pairs, odd so that consecutive rows
-// and consecutive pairs both spread over the banks
-__host__ __device__ inline int exch_row_pairs(int no, int wpt) { return (no * wpt) | 1; }
+// float2 per staged row: the (re, im) pairs of wsub walkers, odd so that consecutive
+// rows and consecutive pairs both spread over the banks
+__host__ __device__ inline int exch_row_pairs(int no, int wsub) { return (no * wsub) | 1; }
 
 // bytes behind the ring that an MMA over bn rows reads past a box of brows rows
 __host__ __device__ inline size_t exch_overread(int bn, int brows) { return size_t(bn - brows) * 128; }
@@ -55,14 +55,14 @@ __host__ __device__ inline size_t exch_overread(int bn, int brows) { return size
 // What a launch needs besides the tiling.  ts: the row operand in TMEM.
 struct ExchPlan {
   int ts, nbuf, lot;  // TMEM accumulator buffers; K blocks of the low piece that sit in TMEM
-  int stages, gsub;
+  int stages, gsub, wsub;  // Cholesky vectors and walkers staged at once
   size_t smem;
 };
 constexpr size_t kExchSums = 4 * 128 * (2 * 16 + 8);  // ring of row sums (2 x float4) and diagonals (float2)
 
-// sums and staging of the epilogue
-__host__ __device__ inline size_t exch_epi_bytes(int no, int wpt, int gsub) {
-  return (kExchSums + size_t(gsub) * no * exch_row_pairs(no, wpt) * 8 + 255) & ~size_t(255);
+// sums (several walkers per tile: a float4 for each and epilogue warp) and staging of the epilogue
+__host__ __device__ inline size_t exch_epi_bytes(int no, int wpt, int wsub, int gsub) {
+  return ((wpt == 1 ? kExchSums : size_t(wpt) * 8 * 16) + size_t(gsub) * no * exch_row_pairs(no, wsub) * 8 + 255) & ~size_t(255);
 }
 
 // Streaming kernel: [ring of A and B][barriers 256][sums][staging].
@@ -74,19 +74,25 @@ inline ExchPlan exch_plan(int npc, int no, int K, const UExchTile& X, int arows,
   const int KB = (K + kUBK - 1) / kUBK, KS = (K + 15) / 16;
   const size_t a = size_t(arows) * 128, b = size_t(brows) * 128;
   const size_t fixed = 1024 + exch_overread(X.bn, brows) + 256;
-  auto staging = [&](int gsub) { return exch_epi_bytes(no, X.wpt, gsub); };
-  ExchPlan p{0, 0, 0, 0, 0, 0};
+  ExchPlan p{0, 0, 0, 0, 0, 0, 0};
   const int cap = max_stages >= 2 ? max_stages : 6;
-  // three stages hide the load latency behind a K block's MMAs; all vectors
-  // staged at once if they fit beside them (a pass less in the epilogue)
+  // three stages hide the load latency behind a K block's MMAs; the whole tile
+  // staged at once if it fits beside them (a pass less in the epilogue), else as
+  // many of its walkers as fit, or, with one walker, Cholesky vectors.  (Several
+  // walkers are never cut by vectors: the threads of the other rows would stand idle in
+  // every pass.  Three pieces, N = 100, No = 8, 200 walkers, where three of 16 vectors
+  // fit: 197 us an energy by vectors, 86 us by walkers.)
   auto fill = [&](size_t res, size_t stage) {
+    const int most = X.wpt == 1 ? X.gpt : X.wpt;
     for (int want = cap < 3 ? cap : 3; want >= 2; --want)
-      for (int g = X.gpt; g >= 1; --g) {
-        const size_t base = fixed + res + staging(g);
+      for (int n = most; n >= 1; --n) {
+        const int g = X.wpt == 1 ? n : X.gpt, w = X.wpt == 1 ? 1 : n;
+        const size_t base = fixed + res + exch_epi_bytes(no, X.wpt, w, g);
         if (base + want * stage > kUmmaSmemBudget) continue;
         const int st = int((kUmmaSmemBudget - base) / stage);
         p.stages = st > cap ? cap : st;
         p.gsub = g;
+        p.wsub = w;
         p.smem = base + p.stages * stage;
         return true;
       }
@@ -201,20 +207,24 @@ __device__ __forceinline__ void exch_tile(const ExchParams& P, uint32_t taddr, u
                                           int nti, int ew, int it, float2* Fs, float4* xs, float2* dg,
                                           uint64_t* xempty, uint64_t* xfull, volatile int* abort_s) {
   const int lane = threadIdx.x & 31, h = ew >> 2, row = ((threadIdx.x >> 5) & 3) * 32 + lane;
-  const int no = P.no, no4 = no & ~3, npair = P.wpt * no;
+  const int no = P.no, no4 = no & ~3;
   const int gl = row / no, i = row - gl * no;
-  const int fs = exch_row_pairs(no, P.wpt);
+  const int fs = exch_row_pairs(no, P.wsub);
   const bool one = P.wpt == 1;
   const int g0 = mti * P.gpt, w0 = nti * P.wpt;
   const int gcount = min(P.gpt, P.G - g0), wcount = min(P.wpt, P.W - w0);
   if (one) mbar_wait_or_abort(xempty, ((it / kExchRing) & 1) ^ 1, abort_s, P.err);
-  for (int gs = 0; gs < gcount; gs += P.gsub) {
-    const int gn = min(P.gsub, gcount - gs);
+  const int nall = one ? gcount : wcount, nsub = one ? P.gsub : P.wsub;
+  for (int s = 0; s < nall; s += nsub) {  // Cholesky vectors (one walker) or walkers staged together
+    const int n = min(nsub, nall - s);
+    const int gs = one ? s : 0, gn = one ? n : gcount, ws = one ? 0 : s, wn = one ? 1 : n;
     const bool mine = gl >= gs && gl < gs + gn;
+    const int plo = ws * no, phi = (ws + wn) * no;  // (re, im) pairs of the row
     float2* const fr = Fs + (row - gs * no) * fs;
     constexpr int NCH = BN / 16, CU = NCH == 5 ? 5 : (NCH == 6 ? 3 : (NCH >= 4 ? 4 : NCH));
 #pragma unroll 1
     for (int c = 0; c < NCH; c += CU) {
+      if ((c + CU) * 8 <= plo || c * 8 >= phi) continue;
       uint32_t x[2 * CU][4], y[2 * CU][4];
 #pragma unroll
       for (int k = 0; k < 2 * CU; ++k) {
@@ -227,21 +237,21 @@ __device__ __forceinline__ void exch_tile(const ExchParams& P, uint32_t taddr, u
       for (int k = 0; k < 2 * CU; ++k) {
         tmem_tie(x[k], y[k]);
         const int pr = c * 8 + k * 4 + 2 * h;
-        if (mine && pr < npair)
-          fr[pr] = make_float2(__uint_as_float(x[k][0]) + __uint_as_float(y[k][0]),
+        if (mine && pr >= plo && pr < phi)
+          fr[pr - plo] = make_float2(__uint_as_float(x[k][0]) + __uint_as_float(y[k][0]),
                                __uint_as_float(x[k][1]) + __uint_as_float(y[k][1]));
-        if (mine && pr + 1 < npair)
-          fr[pr + 1] = make_float2(__uint_as_float(x[k][2]) + __uint_as_float(y[k][2]),
+        if (mine && pr + 1 >= plo && pr + 1 < phi)
+          fr[pr + 1 - plo] = make_float2(__uint_as_float(x[k][2]) + __uint_as_float(y[k][2]),
                                    __uint_as_float(x[k][3]) + __uint_as_float(y[k][3]));
       }
     }
-    if (gs + P.gsub >= gcount) {  // the accumulators are in shared memory
+    if (s + nsub >= nall) {  // the accumulators are in shared memory
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(release);
     }
     exch_sync();
-    for (int wl = 0; wl < wcount; ++wl) {
+    for (int wl = 0; wl < wn; ++wl) {
       ff xr = {0.f, 0.f}, xi = {0.f, 0.f};
       if (mine) {
         const float2* fc = Fs + (gl - gs) * no * fs + wl * no + i;
@@ -270,19 +280,12 @@ __device__ __forceinline__ void exch_tile(const ExchParams& P, uint32_t taddr, u
       }
       if (!one) {
         ff_lane_sum<32>(xr, xi);
-        if (lane == 0) {
-          float4* p = &xs[wl * 8 + ew];
-          if (gs) {
-            xr = ff_add(xr, {p->x, p->y});
-            xi = ff_add(xi, {p->z, p->w});
-          }
-          *p = ff_pack(xr, xi);
-        }
+        if (lane == 0) xs[(ws + wl) * 8 + ew] = ff_pack(xr, xi);
       }
     }
     if (!one) {
       // traces of several walkers: one thread per (Cholesky vector, walker)
-      for (int e = ew * 32 + lane; e < gn * wcount; e += 256) {
+      for (int e = ew * 32 + lane; e < gn * wn; e += 256) {
         const int wl = e / gn, g = e - wl * gn;
         const float2* d = Fs + g * no * fs + wl * no;
         ff cr = {0.f, 0.f}, ci = {0.f, 0.f};
@@ -291,7 +294,7 @@ __device__ __forceinline__ void exch_tile(const ExchParams& P, uint32_t taddr, u
           cr = ff_add(cr, {z.x, 0.f});
           ci = ff_add(ci, {z.y, 0.f});
         }
-        P.cout[(long long)(w0 + wl) * P.G + g0 + gs + g] = ff_pack(cr, ci);
+        P.cout[(long long)(w0 + ws + wl) * P.G + g0 + g] = ff_pack(cr, ci);
       }
     }
     exch_sync();
@@ -371,7 +374,7 @@ __global__ void __launch_bounds__(kExchThreads, 1) umma_exch_kernel(const __grid
   volatile int* abort_s = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float4* xsum = reinterpret_cast<float4*>(reinterpret_cast<uint8_t*>(full) + 256);
   float2* diag = reinterpret_cast<float2*>(xsum + kExchRing * 256);
-  float2* Fs = diag + kExchRing * 128;
+  float2* Fs = P.wpt == 1 ? diag + kExchRing * 128 : reinterpret_cast<float2*>(xsum + P.wpt * 8);
 
   constexpr uint32_t kCols = umma_tmem_cols(BN, 2, 2);
   constexpr uint32_t acc_stride = 2 * BN;
@@ -553,7 +556,7 @@ __global__ void __launch_bounds__(kExchThreads, 1)
   volatile int* abort_s = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float4* xsum = reinterpret_cast<float4*>(reinterpret_cast<uint8_t*>(full) + 256);
   float2* diag = reinterpret_cast<float2*>(xsum + kExchRing * 256);
-  float2* Fs = diag + kExchRing * 128;
+  float2* Fs = P.wpt == 1 ? diag + kExchRing * 128 : reinterpret_cast<float2*>(xsum + P.wpt * 8);
 
   constexpr uint32_t kACol = NBUF * 2 * BN;  // first column of the row operand
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -468,6 +468,7 @@ int exch_launch(const Layout& L, const double* prep, double* work, int s, cudaSt
   if (plan.stages < 2) return AFQ_ERR_SHAPE;
   P.stages = plan.stages;
   P.gsub = plan.gsub;
+  P.wsub = plan.wsub;
   P.lot = plan.lot;
   for (int i = 0; i < 2; ++i) P.a[i] = a[i];
   P.lda = L.Nb;
