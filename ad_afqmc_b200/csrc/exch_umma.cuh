@@ -38,10 +38,11 @@ struct ExchParams {
   int ncw;                 // walker tiles per L2 chunk
   int arows, brows;        // box rows of A (multiple of 8) and B (multiple of 8)
   int stages, gsub, wsub, lot;
+  int ring;                // slots between the epilogue and the reducing warps (4 or 2)
   const bf16* a[2];        // row operand pieces (the TMEM kernel loads them itself), row stride lda
   long long lda;
-  float4* cout;            // (W, G): tr f as pairs (re hi, re lo, im hi, im lo)
-  float4* excout;          // (mt, W): sum f o f^T, the same
+  double* cout;            // (W, G) complex: tr f
+  double* excout;          // (mt, W) complex: sum f o f^T
   int* err;
 };
 
@@ -52,17 +53,18 @@ __host__ __device__ inline int exch_row_pairs(int no, int wsub) { return (no * w
 // bytes behind the ring that an MMA over bn rows reads past a box of brows rows
 __host__ __device__ inline size_t exch_overread(int bn, int brows) { return size_t(bn - brows) * 128; }
 
+constexpr int kExchRing = 4;  // most walkers between the epilogue and the reducing warps
+
 // What a launch needs besides the tiling.  ts: the row operand in TMEM.
 struct ExchPlan {
   int ts, nbuf, lot;  // TMEM accumulator buffers; K blocks of the low piece that sit in TMEM
   int stages, gsub, wsub;  // Cholesky vectors and walkers staged at once
+  int ring;
   size_t smem;
 };
-constexpr size_t kExchSums = 4 * 128 * (2 * 16 + 8);  // ring of row sums (2 x float4) and diagonals (float2)
-
-// sums (several walkers per tile: a float4 for each and epilogue warp) and staging of the epilogue
-__host__ __device__ inline size_t exch_epi_bytes(int no, int wpt, int wsub, int gsub) {
-  return ((wpt == 1 ? kExchSums : size_t(wpt) * 8 * 16) + size_t(gsub) * no * exch_row_pairs(no, wsub) * 8 + 255) & ~size_t(255);
+// ring of a walker's row chains (2 x float4) and diagonals (float2), and staging of the epilogue
+__host__ __device__ inline size_t exch_epi_bytes(int no, int wsub, int gsub, int ring) {
+  return (size_t(ring) * 128 * (2 * 16 + 8) + size_t(gsub) * no * exch_row_pairs(no, wsub) * 8 + 255) & ~size_t(255);
 }
 
 // Streaming kernel: [ring of A and B][barriers 256][sums][staging].
@@ -74,28 +76,30 @@ inline ExchPlan exch_plan(int npc, int no, int K, const UExchTile& X, int arows,
   const int KB = (K + kUBK - 1) / kUBK, KS = (K + 15) / 16;
   const size_t a = size_t(arows) * 128, b = size_t(brows) * 128;
   const size_t fixed = 1024 + exch_overread(X.bn, brows) + 256;
-  ExchPlan p{0, 0, 0, 0, 0, 0, 0};
+  ExchPlan p{};
   const int cap = max_stages >= 2 ? max_stages : 6;
   // three stages hide the load latency behind a K block's MMAs; the whole tile
   // staged at once if it fits beside them (a pass less in the epilogue), else as
   // many of its walkers as fit, or, with one walker, Cholesky vectors.  (Several
   // walkers are never cut by vectors: the threads of the other rows would stand idle in
   // every pass.  Three pieces, N = 100, No = 8, 200 walkers, where three of 16 vectors
-  // fit: 197 us an energy by vectors, 86 us by walkers.)
+  // fit: 197 us an energy by vectors, 94 us by walkers.)
   auto fill = [&](size_t res, size_t stage) {
     const int most = X.wpt == 1 ? X.gpt : X.wpt;
-    for (int want = cap < 3 ? cap : 3; want >= 2; --want)
-      for (int n = most; n >= 1; --n) {
-        const int g = X.wpt == 1 ? n : X.gpt, w = X.wpt == 1 ? 1 : n;
-        const size_t base = fixed + res + exch_epi_bytes(no, X.wpt, w, g);
-        if (base + want * stage > kUmmaSmemBudget) continue;
-        const int st = int((kUmmaSmemBudget - base) / stage);
-        p.stages = st > cap ? cap : st;
-        p.gsub = g;
-        p.wsub = w;
-        p.smem = base + p.stages * stage;
-        return true;
-      }
+    for (int ring = kExchRing; ring >= 2; ring >>= 1)
+      for (int want = cap < 3 ? cap : 3; want >= 2; --want)
+        for (int n = most; n >= 1; --n) {
+          const int g = X.wpt == 1 ? n : X.gpt, w = X.wpt == 1 ? 1 : n;
+          const size_t base = fixed + res + exch_epi_bytes(no, w, g, ring);
+          if (base + want * stage > kUmmaSmemBudget) continue;
+          const int st = int((kUmmaSmemBudget - base) / stage);
+          p.stages = st > cap ? cap : st;
+          p.gsub = g;
+          p.wsub = w;
+          p.ring = ring;
+          p.smem = base + p.stages * stage;
+          return true;
+        }
     return false;
   };
   // two accumulator buffers if the high piece's K fits the columns beside them, else one
@@ -115,7 +119,6 @@ inline ExchPlan exch_plan(int npc, int no, int K, const UExchTile& X, int arows,
 // the eight epilogue warps (four more reduce)
 __device__ __forceinline__ void exch_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 constexpr int kExchThreads = 64 + 256 + 128;
-constexpr int kExchRing = 4;  // tiles between the epilogue and the reducing warps
 
 // position of a tile: walker chunk [c0, c0 + width), row tile, walker tile;
 // stepped without divisions (a 64-bit division costs the MMA thread 500 cycles)
@@ -161,62 +164,64 @@ __device__ __forceinline__ void tmem_tie(uint32_t (&r)[4], uint32_t (&q)[4]) {
                     "+r"(q[2]), "+r"(q[3]));
 }
 
-// Sums of FP32 values as unevaluated pairs hi + lo (Knuth's two-sum; about 48
-// bits).  A dependent DADD takes 400 cycles while tcgen05.mma runs (the FP64 unit
-// waits for the tensor core), an FADD about 14; the consumer adds hi and lo in FP64.
-struct ff {
-  float hi, lo;
+// Sums of FP32 values.  The FP64 unit waits for the tensor core while tcgen05.mma
+// runs (110 to 170 cycles an instruction and scheduler, a dependent DADD 405, an FADD 14), so a
+// lane adds its values up in FP32 with the rounding errors carried along twice
+// (Knuth's two-sum): a + b + c holds about 70 bits of the sum, and becomes one FP64 number.
+struct ExchSum {
+  float a, b, c;
 };
-__device__ __forceinline__ ff ff_two_sum(float a, float b) {
-  const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
-  return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t))};
+__device__ __forceinline__ float exch_two_sum(float& s, float x) {  // s += x, returns what was rounded off
+  const float t = __fadd_rn(s, x), v = __fsub_rn(t, s);
+  const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, v)), __fsub_rn(x, v));
+  s = t;
+  return e;
 }
-__device__ __forceinline__ ff ff_add(ff a, ff b) {
-  const ff s = ff_two_sum(a.hi, b.hi);
-  const float e = __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo));
-  const float h = __fadd_rn(s.hi, e);
-  return {h, __fsub_rn(e, __fsub_rn(h, s.hi))};
+__device__ __forceinline__ void exch_add(ExchSum& s, float x) {
+  s.c = __fadd_rn(s.c, exch_two_sum(s.b, exch_two_sum(s.a, x)));
 }
-// sums of r and i over groups of WIDTH lanes, valid in the first lane of each
-template <int WIDTH>
-__device__ __forceinline__ void ff_lane_sum(ff& r, ff& i) {
-#pragma unroll
-  for (int o = WIDTH >> 1; o > 0; o >>= 1) {
-    const ff a = {__shfl_down_sync(0xffffffffu, r.hi, o), __shfl_down_sync(0xffffffffu, r.lo, o)};
-    const ff b = {__shfl_down_sync(0xffffffffu, i.hi, o), __shfl_down_sync(0xffffffffu, i.lo, o)};
-    r = ff_add(r, a);
-    i = ff_add(i, b);
-  }
+__device__ __forceinline__ double exch_value(const ExchSum& s) { return (double)s.a + ((double)s.b + (double)s.c); }
+
+// x of half the lanes (those with lane & o) exchanged for y of the others: lanes without
+// the bit then hold the sum of two lanes' x, those with it of two lanes' y
+__device__ __forceinline__ ExchSum exch_halve(const ExchSum& x, const ExchSum& y, int o) {
+  const bool up = (threadIdx.x & o) != 0;
+  ExchSum m = up ? y : x;
+  const ExchSum t = up ? x : y;
+  const float a = __shfl_xor_sync(0xffffffffu, t.a, o), b = __shfl_xor_sync(0xffffffffu, t.b, o),
+              c = __shfl_xor_sync(0xffffffffu, t.c, o);
+  exch_add(m, a);
+  exch_add(m, b);
+  exch_add(m, c);
+  return m;
 }
-// (re, im) pairs of such sums as they are stored
-__device__ __forceinline__ float4 ff_pack(ff r, ff i) { return make_float4(r.hi, r.lo, i.hi, i.lo); }
 
 // One tile's epilogue by eight warps: f from the accumulators (both groups
 // summed in FP32) to shared memory, then per row (g, i) and walker
 // sum_j f[i][j] f[j][i] in four FP32 chains (j mod 4; the last no mod 4 terms in
-// chain 0), combined as pairs.  Half h of the warps moves the pairs j = 2h, 2h + 1
-// (mod 4) and runs chains 2h, 2h + 1 of all 128 rows.  The loops stay rolled: the
-// warps share an instruction cache with the MMA warp, and a fully unrolled form
-// with the row in registers ran slower.  Everything after the chains is summed
-// in pairs in a fixed order, so results are reproducible.
-// One walker per tile: the row sums (xs: [2 halves][128]) and diagonals (dg: [128])
-// go to the reducing warps through a ring of kExchRing tiles; several: xs holds a
-// partial per (walker, warp) and the tile is finished here.
+// chain 0).  Half h of the warps moves the pairs j = 2h, 2h + 1 (mod 4) and runs
+// chains 2h, 2h + 1 of all 128 rows.  The loops stay rolled: the warps share an
+// instruction cache with the MMA warp, and a fully unrolled form with the row in
+// registers ran slower.  A walker's chains (xs: [2 halves][128], re re im im) and
+// diagonals (dg: [128]) go to the reducing warps through a ring of P.ring slots;
+// `slot` counts them over the CTA's tiles.
+// times the ring has gone round before this slot
+__device__ __forceinline__ int exch_lap(const ExchParams& P, int slot) { return slot >> (P.ring == 4 ? 2 : 1); }
+
 template <int BN>
 __device__ __forceinline__ void exch_tile(const ExchParams& P, uint32_t taddr, uint64_t* release, int mti,
-                                          int nti, int ew, int it, float2* Fs, float4* xs, float2* dg,
+                                          int nti, int ew, int& slot, float2* Fs, float4* xsum, float2* diag,
                                           uint64_t* xempty, uint64_t* xfull, volatile int* abort_s) {
   const int lane = threadIdx.x & 31, h = ew >> 2, row = ((threadIdx.x >> 5) & 3) * 32 + lane;
   const int no = P.no, no4 = no & ~3;
   const int gl = row / no, i = row - gl * no;
   const int fs = exch_row_pairs(no, P.wsub);
   const bool one = P.wpt == 1;
-  const int g0 = mti * P.gpt, w0 = nti * P.wpt;
-  const int gcount = min(P.gpt, P.G - g0), wcount = min(P.wpt, P.W - w0);
-  if (one) mbar_wait_or_abort(xempty, ((it / kExchRing) & 1) ^ 1, abort_s, P.err);
+  const int gcount = min(P.gpt, P.G - mti * P.gpt), wcount = min(P.wpt, P.W - nti * P.wpt);
   const int nall = one ? gcount : wcount, nsub = one ? P.gsub : P.wsub;
   for (int s = 0; s < nall; s += nsub) {  // Cholesky vectors (one walker) or walkers staged together
     const int n = min(nsub, nall - s);
+    const bool last = s + nsub >= nall;
     const int gs = one ? s : 0, gn = one ? n : gcount, ws = one ? 0 : s, wn = one ? 1 : n;
     const bool mine = gl >= gs && gl < gs + gn;
     const int plo = ws * no, phi = (ws + wn) * no;  // (re, im) pairs of the row
@@ -239,20 +244,21 @@ __device__ __forceinline__ void exch_tile(const ExchParams& P, uint32_t taddr, u
         const int pr = c * 8 + k * 4 + 2 * h;
         if (mine && pr >= plo && pr < phi)
           fr[pr - plo] = make_float2(__uint_as_float(x[k][0]) + __uint_as_float(y[k][0]),
-                               __uint_as_float(x[k][1]) + __uint_as_float(y[k][1]));
+                                     __uint_as_float(x[k][1]) + __uint_as_float(y[k][1]));
         if (mine && pr + 1 >= plo && pr + 1 < phi)
           fr[pr + 1 - plo] = make_float2(__uint_as_float(x[k][2]) + __uint_as_float(y[k][2]),
-                                   __uint_as_float(x[k][3]) + __uint_as_float(y[k][3]));
+                                         __uint_as_float(x[k][3]) + __uint_as_float(y[k][3]));
       }
     }
-    if (s + nsub >= nall) {  // the accumulators are in shared memory
+    if (last) {  // the accumulators are in shared memory
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(release);
     }
     exch_sync();
     for (int wl = 0; wl < wn; ++wl) {
-      ff xr = {0.f, 0.f}, xi = {0.f, 0.f};
+      const int q = slot & (P.ring - 1);
+      if (!one || s == 0) mbar_wait_or_abort(&xempty[q], (exch_lap(P, slot) & 1) ^ 1, abort_s, P.err);
       if (mine) {
         const float2* fc = Fs + (gl - gs) * no * fs + wl * no + i;
         const float2* fw = fr + wl * no;
@@ -271,86 +277,137 @@ __device__ __forceinline__ void exch_tile(const ExchParams& P, uint32_t taddr, u
             ar0 = fmaf(a.x, b.x, fmaf(-a.y, b.y, ar0));
             ai0 = fmaf(a.x, b.y, fmaf(a.y, b.x, ai0));
           }
-        xr = ff_two_sum(ar0, ar1);
-        xi = ff_two_sum(ai0, ai1);
-        if (one) {
-          xs[h * 128 + row] = ff_pack(xr, xi);
-          if (h == 0) dg[row] = fw[i];
-        }
+        xsum[q * 256 + h * 128 + row] = make_float4(ar0, ar1, ai0, ai1);
+        if (h == 0) diag[q * 128 + row] = fw[i];
       }
-      if (!one) {
-        ff_lane_sum<32>(xr, xi);
-        if (lane == 0) xs[(ws + wl) * 8 + ew] = ff_pack(xr, xi);
-      }
-    }
-    if (!one) {
-      // traces of several walkers: one thread per (Cholesky vector, walker)
-      for (int e = ew * 32 + lane; e < gn * wn; e += 256) {
-        const int wl = e / gn, g = e - wl * gn;
-        const float2* d = Fs + g * no * fs + wl * no;
-        ff cr = {0.f, 0.f}, ci = {0.f, 0.f};
-        for (int r = 0; r < no; ++r) {
-          const float2 z = d[r * fs + r];
-          cr = ff_add(cr, {z.x, 0.f});
-          ci = ff_add(ci, {z.y, 0.f});
-        }
-        P.cout[(long long)(w0 + ws + wl) * P.G + g0 + g] = ff_pack(cr, ci);
+      if (!one || last) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&xfull[q]);
+        ++slot;
       }
     }
     exch_sync();
   }
-  if (one && lane == 0) mbar_arrive(xfull);  // every row is written (the barrier above)
-  if (!one) {
-    for (int wl = ew * 32 + lane; wl < wcount; wl += 256) {
-      ff xr = {0.f, 0.f}, xi = {0.f, 0.f};
-      for (int k = 0; k < 8; ++k) {
-        const float4 p = xs[wl * 8 + k];
-        xr = ff_add(xr, {p.x, p.y});
-        xi = ff_add(xi, {p.z, p.w});
-      }
-      P.excout[(long long)mti * P.W + w0 + wl] = ff_pack(xr, xi);
+}
+
+// The same sums in FP64 throughout: a walker some of whose FP32 sums leave FP32's range (an
+// overflowed row, an infinite or undefined one).  +-inf stays +-inf.
+__device__ __noinline__ void exch_finish_f64(const ExchParams& P, int mti, int w, const float4* xs,
+                                             const float2* dg) {
+  const int lane = threadIdx.x & 31, no = P.no;
+  const int g0 = mti * P.gpt, gcount = min(P.gpt, P.G - g0), rows = gcount * no;
+  double x = 0.0, y = 0.0;
+  for (int k = lane; k < rows; k += 32) {
+    const float4 u = xs[k], v = xs[128 + k];
+    x += ((double)u.x + (double)u.y) + ((double)v.x + (double)v.y);
+    y += ((double)u.z + (double)u.w) + ((double)v.z + (double)v.w);
+  }
+  __syncwarp();
+  x = warp_sum(x);
+  y = warp_sum(y);
+  if (lane == 0) {
+    P.excout[2 * ((long long)mti * P.W + w)] = x;
+    P.excout[2 * ((long long)mti * P.W + w) + 1] = y;
+  }
+  double* const c = P.cout + 2 * ((long long)w * P.G + g0);
+  for (int g = lane; g < gcount; g += 32) {
+    double cr = 0.0, ci = 0.0;
+    for (int q = 0; q < no; ++q) {
+      const float2 z = dg[g * no + q];
+      cr += (double)z.x;
+      ci += (double)z.y;
     }
+    c[2 * g] = cr;
+    c[2 * g + 1] = ci;
   }
 }
 
-// The reducing warps (one walker per tile): a tile's row sums and diagonals to
-// its exchange partial and its Cholesky vectors' traces.  Four warps take the tiles in
-// turn, off the epilogue's path: the chain of pair additions takes longer than a
-// tile.
-__device__ __forceinline__ void exch_finish(const ExchParams& P, int mti, int nti, int it, const float4* xs,
-                                            const float2* dg, uint64_t* xempty, uint64_t* xfull,
+// The reducing warps: a walker's chains and diagonals to its exchange partial and its
+// Cholesky vectors' traces, FP64 numbers.  Four warps take the slots in turn, off the
+// epilogue's path: the sums take longer than a tile.  The FP32 sums come first, so
+// that the FP64 instructions of all of them overlap.
+__device__ __forceinline__ void exch_finish(const ExchParams& P, int mti, int w, const float4* xs,
+                                            const float2* dg, uint64_t* xempty, uint64_t* xfull, uint32_t parity,
                                             volatile int* abort_s) {
   const int lane = threadIdx.x & 31, no = P.no;
   const int g0 = mti * P.gpt, gcount = min(P.gpt, P.G - g0), rows = gcount * no;
-  mbar_wait_or_abort(xfull, (it / kExchRing) & 1, abort_s, P.err);
-  ff r[4], i[4];
+  mbar_wait_or_abort(xfull, parity, abort_s, P.err);
+  const ExchSum zero = {0.f, 0.f, 0.f};
+  ExchSum r = zero, i = zero;
+#pragma unroll 1
+  for (int k = 0; k < 4; ++k)
+    if (lane + 32 * k < rows) {
+      const float4 u = xs[lane + 32 * k], v = xs[128 + lane + 32 * k];
+      exch_add(r, u.x);
+      exch_add(i, u.z);
+      exch_add(r, u.y);
+      exch_add(i, u.w);
+      exch_add(r, v.x);
+      exch_add(i, v.z);
+      exch_add(r, v.y);
+      exch_add(i, v.w);
+    }
+  __syncwarp();
+  const ExchSum m = exch_halve(r, i, 16);  // lanes 0-15: re, 16-31: im
+  double x = exch_value(m);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const bool in = lane + 32 * k < rows;
-    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 u = in ? xs[lane + 32 * k] : z, v = in ? xs[128 + lane + 32 * k] : z;
-    r[k] = ff_add({u.x, u.y}, {v.x, v.y});
-    i[k] = ff_add({u.z, u.w}, {v.z, v.w});
+  for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  if ((lane & 15) == 0) P.excout[2 * ((long long)mti * P.W + w) + (lane >> 4)] = x;
+  // traces: a lane each of up to 128 Cholesky vectors (no <= 14), or eight lanes each
+  // of up to eight, four of them re and four im
+  double* const c = P.cout + 2 * ((long long)w * P.G + g0);
+  bool fin = isfinite(m.a);
+  if (gcount > 8) {
+#pragma unroll 1
+    for (int gb = 0; gb < gcount; gb += 32) {
+      const int g = gb + lane;
+      ExchSum tr = zero, ti = zero;
+      if (g < gcount)
+#pragma unroll 1
+        for (int q = 0; q < no; ++q) {
+          const float2 z = dg[g * no + q];
+          exch_add(tr, z.x);
+          exch_add(ti, z.y);
+        }
+      __syncwarp();
+      fin = fin && isfinite(tr.a) && isfinite(ti.a);
+      if (g < gcount) *reinterpret_cast<double2*>(c + 2 * g) = make_double2(exch_value(tr), exch_value(ti));
+    }
+  } else {
+#pragma unroll 1
+    for (int gb = 0; gb < gcount; gb += 4) {
+      const int g = gb + (lane >> 3);
+      ExchSum tr = zero, ti = zero;
+      if (g < gcount)
+#pragma unroll 1
+        for (int q = lane & 7; q < no; q += 8) {
+          const float2 z = dg[g * no + q];
+          exch_add(tr, z.x);
+          exch_add(ti, z.y);
+        }
+      __syncwarp();
+      const ExchSum mt = exch_halve(tr, ti, 4);
+      fin = fin && isfinite(mt.a);
+      double y = exch_value(mt);
+      y += __shfl_xor_sync(0xffffffffu, y, 2);
+      y += __shfl_xor_sync(0xffffffffu, y, 1);
+      if (g < gcount && (lane & 3) == 0) c[2 * g + ((lane >> 2) & 1)] = y;
+    }
   }
-  ff xr = ff_add(ff_add(r[0], r[1]), ff_add(r[2], r[3]));
-  ff xi = ff_add(ff_add(i[0], i[1]), ff_add(i[2], i[3]));
-  ff_lane_sum<32>(xr, xi);
-  if (lane == 0) P.excout[(long long)mti * P.W + nti] = ff_pack(xr, xi);
-  for (int gb = 0; gb < gcount; gb += 4) {  // eight lanes per Cholesky vector
-    const int g = gb + (lane >> 3);
-    ff cr = {0.f, 0.f}, ci = {0.f, 0.f};
-    if (g < gcount)
-      for (int q = lane & 7; q < no; q += 8) {
-        const float2 z = dg[g * no + q];
-        cr = ff_add(cr, {z.x, 0.f});
-        ci = ff_add(ci, {z.y, 0.f});
-      }
-    __syncwarp();
-    ff_lane_sum<8>(cr, ci);
-    if (g < gcount && (lane & 7) == 0) P.cout[(long long)nti * P.G + g0 + g] = ff_pack(cr, ci);
-  }
+  if (!__all_sync(0xffffffffu, fin)) exch_finish_f64(P, mti, w, xs, dg);
   __syncwarp();
   if (lane == 0) mbar_arrive(xempty);
+}
+
+// The reducing warps' part of one tile: every P.ring-th slot each.
+__device__ __forceinline__ void exch_reduce(const ExchParams& P, int mti, int nti, int rw, int& slot,
+                                            const float4* xsum, const float2* diag, uint64_t* xempty,
+                                            uint64_t* xfull, volatile int* abort_s) {
+  const int w0 = nti * P.wpt, wcount = min(P.wpt, P.W - w0);
+  for (int wl = 0; wl < wcount; ++wl, ++slot)
+    if ((slot & (P.ring - 1)) == rw)
+      exch_finish(P, mti, w0 + wl, xsum + rw * 256, diag + rw * 128, &xempty[rw], &xfull[rw],
+                  exch_lap(P, slot) & 1, abort_s);
 }
 
 // Streaming form: three-piece operands, or K too long for TMEM.
@@ -373,8 +430,8 @@ __global__ void __launch_bounds__(kExchThreads, 1) umma_exch_kernel(const __grid
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xempty + kExchRing);
   volatile int* abort_s = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float4* xsum = reinterpret_cast<float4*>(reinterpret_cast<uint8_t*>(full) + 256);
-  float2* diag = reinterpret_cast<float2*>(xsum + kExchRing * 256);
-  float2* Fs = P.wpt == 1 ? diag + kExchRing * 128 : reinterpret_cast<float2*>(xsum + P.wpt * 8);
+  float2* diag = reinterpret_cast<float2*>(xsum + P.ring * 256);
+  float2* Fs = diag + P.ring * 128;
 
   constexpr uint32_t kCols = umma_tmem_cols(BN, 2, 2);
   constexpr uint32_t acc_stride = 2 * BN;
@@ -457,23 +514,20 @@ __global__ void __launch_bounds__(kExchThreads, 1) umma_exch_kernel(const __grid
     }
   } else if (warp < 10) {
     const uint32_t lane_t = tbase + ((uint32_t)((warp & 3) * 32) << 16);
-    int it = 0;
+    int it = 0, slot = 0;
     ExchWalk wk = exch_locate(P, t_lo);
     for (int t = t_lo; t < T; t += t_step, ++it, exch_advance(P, wk, t_step)) {
       const int buf = it & 1;
       mbar_wait_or_abort(&accf[buf], (it >> 1) & 1, abort_s, P.err);
       tc_fence_after();
-      exch_tile<BN>(P, lane_t + buf * acc_stride, &acce[buf], wk.mti, wk.nti, warp - 2, it, Fs, xsum + (P.wpt == 1 ? (it % kExchRing) * 256 : 0),
-                    diag + (it % kExchRing) * 128, &xempty[it % kExchRing], &xfull[it % kExchRing], abort_s);
+      exch_tile<BN>(P, lane_t + buf * acc_stride, &acce[buf], wk.mti, wk.nti, warp - 2, slot, Fs,
+                    xsum, diag, xempty, xfull, abort_s);
     }
-  } else if (P.wpt == 1) {
-    int it = 0;
+  } else {
+    int slot = 0;
     ExchWalk wk = exch_locate(P, t_lo);
-    for (int t = t_lo; t < T; t += t_step, ++it, exch_advance(P, wk, t_step)) {
-      const int q = it % kExchRing;
-      if (q == warp - 10)
-        exch_finish(P, wk.mti, wk.nti, it, xsum + q * 256, diag + q * 128, &xempty[q], &xfull[q], abort_s);
-    }
+    for (int t = t_lo; t < T; t += t_step, exch_advance(P, wk, t_step))
+      exch_reduce(P, wk.mti, wk.nti, warp - 10, slot, xsum, diag, xempty, xfull, abort_s);
   }
   tc_fence_before();
   __syncthreads();
@@ -555,8 +609,8 @@ __global__ void __launch_bounds__(kExchThreads, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(xempty + kExchRing);
   volatile int* abort_s = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float4* xsum = reinterpret_cast<float4*>(reinterpret_cast<uint8_t*>(full) + 256);
-  float2* diag = reinterpret_cast<float2*>(xsum + kExchRing * 256);
-  float2* Fs = P.wpt == 1 ? diag + kExchRing * 128 : reinterpret_cast<float2*>(xsum + P.wpt * 8);
+  float2* diag = reinterpret_cast<float2*>(xsum + P.ring * 256);
+  float2* Fs = diag + P.ring * 128;
 
   constexpr uint32_t kACol = NBUF * 2 * BN;  // first column of the row operand
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -672,7 +726,7 @@ __global__ void __launch_bounds__(kExchThreads, 1)
     __syncwarp();
   } else if (warp < 10) {
     const uint32_t lane_t = tbase + ((uint32_t)((warp & 3) * 32) << 16);
-    int it = 0, have = -1;
+    int it = 0, have = -1, slot = 0;
     ExchWalk wk = exch_locate(P, t_lo);
     for (int t = t_lo; t < t_hi; ++t, ++it, exch_advance(P, wk, 1)) {
       if (wk.mti != have) {
@@ -704,17 +758,14 @@ __global__ void __launch_bounds__(kExchThreads, 1)
       const int buf = NBUF == 2 ? it & 1 : 0;
       mbar_wait_or_abort(&accf[buf], (it / NBUF) & 1, abort_s, P.err);
       tc_fence_after();
-      exch_tile<BN>(P, lane_t + buf * 2 * BN, &acce[buf], wk.mti, wk.nti, warp - 2, it, Fs, xsum + (P.wpt == 1 ? (it % kExchRing) * 256 : 0),
-                    diag + (it % kExchRing) * 128, &xempty[it % kExchRing], &xfull[it % kExchRing], abort_s);
+      exch_tile<BN>(P, lane_t + buf * 2 * BN, &acce[buf], wk.mti, wk.nti, warp - 2, slot, Fs,
+                    xsum, diag, xempty, xfull, abort_s);
     }
-  } else if (P.wpt == 1) {
-    int it = 0;
+  } else {
+    int slot = 0;
     ExchWalk wk = exch_locate(P, t_lo);
-    for (int t = t_lo; t < t_hi; t += 1, ++it, exch_advance(P, wk, 1)) {
-      const int q = it % kExchRing;
-      if (q == warp - 10)
-        exch_finish(P, wk.mti, wk.nti, it, xsum + q * 256, diag + q * 128, &xempty[q], &xfull[q], abort_s);
-    }
+    for (int t = t_lo; t < t_hi; ++t, exch_advance(P, wk, 1))
+      exch_reduce(P, wk.mti, wk.nti, warp - 10, slot, xsum, diag, xempty, xfull, abort_s);
   }
   tc_fence_before();
   __syncthreads();

@@ -432,36 +432,28 @@ __global__ void orb_combine_kernel(int W, int mt, const double* part, double* ou
 // ---------------------------------------------------------------------------
 // local energy from the pieces (one warp per walker)
 // ---------------------------------------------------------------------------
-// a complex value of the exchange: FP64, or (pairs) the tensor-core kernel's
-// unevaluated FP32 pairs (re hi, re lo, im hi, im lo) in the same 16 bytes
-__device__ __forceinline__ double2 exch_value(const double* p, long long i, int pairs) {
-  if (!pairs) return make_double2(p[2 * i], p[2 * i + 1]);
-  const float4 v = reinterpret_cast<const float4*>(p)[i];
-  return make_double2((double)v.x + (double)v.y, (double)v.z + (double)v.w);
-}
-
 __global__ void energy_combine_kernel(int W, int G, int ns, int restricted, const double* scal,
                                       const double* c0, const double* c1, const double* x0,
-                                      int mt0, const double* x1, int mt1, int pairs0, int pairs1,
-                                      const double* wscal, double* eout, int eout_stride) {
+                                      int mt0, const double* x1, int mt1, const double* wscal,
+                                      double* eout, int eout_stride) {
   const int lane = threadIdx.x & 31;
   const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= W) return;
   double jr = 0, ji = 0, xr = 0, xi = 0;
   for (int g = lane; g < G; g += 32) {
-    double2 a = exch_value(c0, (long long)w * G + g, pairs0);
-    if (ns == 2) a = cadd(a, exch_value(c1, (long long)w * G + g, pairs1));
+    double2 a = reinterpret_cast<const double2*>(c0)[(long long)w * G + g];
+    if (ns == 2) a = cadd(a, reinterpret_cast<const double2*>(c1)[(long long)w * G + g]);
     jr += a.x * a.x - a.y * a.y;
     ji += 2.0 * a.x * a.y;
   }
   for (int m = lane; m < mt0; m += 32) {
-    const double2 x = exch_value(x0, (long long)m * W + w, pairs0);
+    const double2 x = reinterpret_cast<const double2*>(x0)[(long long)m * W + w];
     xr += x.x;
     xi += x.y;
   }
   if (ns == 2)
     for (int m = lane; m < mt1; m += 32) {
-      const double2 x = exch_value(x1, (long long)m * W + w, pairs1);
+      const double2 x = reinterpret_cast<const double2*>(x1)[(long long)m * W + w];
       xr += x.x;
       xi += x.y;
     }
@@ -806,7 +798,7 @@ cudaError_t launch_energy_combine(const Layout& L, const double* prep, double* w
   energy_combine_kernel<<<(L.W + wpb - 1) / wpb, 32 * wpb, 0, st>>>(
       L.W, L.G, L.ns, L.restricted, prep + L.p_scal, work + L.w_c[0], L.ns == 2 ? work + L.w_c[1] : nullptr,
       work + L.w_exc[0], L.ex[0].mt, L.ns == 2 ? work + L.w_exc[1] : nullptr,
-      L.ns == 2 ? L.ex[1].mt : 0, !L.exch_f64[0], !L.exch_f64[1], work + L.w_wscal, eout, eout_stride);
+      L.ns == 2 ? L.ex[1].mt : 0, work + L.w_wscal, eout, eout_stride);
   return cudaGetLastError();
 }
 

@@ -469,11 +469,12 @@ int exch_launch(const Layout& L, const double* prep, double* work, int s, cudaSt
   P.stages = plan.stages;
   P.gsub = plan.gsub;
   P.wsub = plan.wsub;
+  P.ring = plan.ring;
   P.lot = plan.lot;
   for (int i = 0; i < 2; ++i) P.a[i] = a[i];
   P.lda = L.Nb;
-  P.cout = reinterpret_cast<float4*>(work + L.w_c[s]);
-  P.excout = reinterpret_cast<float4*>(work + L.w_exc[s]);
+  P.cout = work + L.w_c[s];
+  P.excout = work + L.w_exc[s];
   P.err = err_flag(L, work);
   int ctas = sm_count();
   if (L.tune.grid_cap > 0 && L.tune.grid_cap < ctas) ctas = L.tune.grid_cap;
