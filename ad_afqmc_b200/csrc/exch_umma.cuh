@@ -258,7 +258,7 @@ __device__ __forceinline__ void exch_tile(const ExchParams& P, uint32_t taddr, u
     exch_sync();
     for (int wl = 0; wl < wn; ++wl) {
       const int q = slot & (P.ring - 1);
-      if (!one || s == 0) mbar_wait_or_abort(&xempty[q], (exch_lap(P, slot) & 1) ^ 1, abort_s, P.err);
+      if (!one || s == 0) mbar_wait_run_on(&xempty[q], (exch_lap(P, slot) & 1) ^ 1, abort_s, P.err);
       if (mine) {
         const float2* fc = Fs + (gl - gs) * no * fs + wl * no + i;
         const float2* fw = fr + wl * no;
@@ -331,7 +331,7 @@ __device__ __forceinline__ void exch_finish(const ExchParams& P, int mti, int w,
                                             volatile int* abort_s) {
   const int lane = threadIdx.x & 31, no = P.no;
   const int g0 = mti * P.gpt, gcount = min(P.gpt, P.G - g0), rows = gcount * no;
-  mbar_wait_or_abort(xfull, parity, abort_s, P.err);
+  mbar_wait_run_on(xfull, parity, abort_s, P.err);
   const ExchSum zero = {0.f, 0.f, 0.f};
   ExchSum r = zero, i = zero;
 #pragma unroll 1
@@ -463,62 +463,54 @@ __global__ void __launch_bounds__(kExchThreads, 1) umma_exch_kernel(const __grid
   const int t_lo = blockIdx.x, t_step = gridDim.x;
   const int tail = (P.K - (KB - 1) * kUBK + 15) >> 4;  // 16-wide K steps with data in the last block
 
+  Ring rg{full, empty, ST};
   if (warp == 0) {
-    int stage = 0;
-    uint32_t phase = 0;
     ExchWalk wk = exch_locate(P, t_lo);
     for (int t = t_lo; t < T; t += t_step, exch_advance(P, wk, t_step)) {
       const int arow = wk.mti * P.gpt * no, brow = wk.nti * P.wpt * 2 * no;
-      for (int kb = 0; kb < KB; ++kb) {
-        mbar_wait_or_abort(&empty[stage], phase ^ 1, abort_s, P.err);
-        if (elect_one()) {
-          mbar_arrive_expect_tx(&full[stage], stage_bytes);
-          uint8_t* sa = ring + stage * stage_bytes;
-          uint8_t* sb = sa + NPC * a_bytes;
-          for (int i = 0; i < NPC; ++i)
-            tma_load_3d(sa + i * a_bytes, &P.ta[i], &full[stage], kb * kUBK, arow, 0);
-          for (int j = 0; j < NPC; ++j)
-            tma_load_3d(sb + j * b_bytes, &P.tb[j], &full[stage], kb * kUBK, brow, 0);
-        }
-        __syncwarp();
-        if (++stage == ST) { stage = 0; phase ^= 1; }
-      }
+      const bool ok = ring_fill(rg, KB, abort_s, P.err, [&](int stage, int kb) {
+        mbar_arrive_expect_tx(&full[stage], stage_bytes);
+        uint8_t* sa = ring + stage * stage_bytes;
+        uint8_t* sb = sa + NPC * a_bytes;
+        for (int i = 0; i < NPC; ++i)
+          tma_load_3d(sa + i * a_bytes, &P.ta[i], &full[stage], kb * kUBK, arow, 0);
+        for (int j = 0; j < NPC; ++j)
+          tma_load_3d(sb + j * b_bytes, &P.tb[j], &full[stage], kb * kUBK, brow, 0);
+      });
+      if (!ok) break;
     }
-    // drain (bounded): every stage that was filled has been released
-    for (int s = 0; s < ST; ++s) {
-      mbar_wait_or_abort(&empty[stage], phase ^ 1, abort_s, P.err);
-      if (++stage == ST) { stage = 0; phase ^= 1; }
-    }
+    ring_drain(rg, full);
   } else if (warp == 1) {
     const uint32_t ring_base = su32(ring);
-    int stage = 0, it = 0;
-    uint32_t phase = 0;
+    int it = 0;
     for (int t = t_lo; t < T; t += t_step, ++it) {
       const int buf = it & 1;
-      mbar_wait_or_abort(&acce[buf], ((it >> 1) & 1) ^ 1, abort_s, P.err);
+      const bool ok = mbar_wait_or_abort(&acce[buf], ((it >> 1) & 1) ^ 1, abort_s, P.err);
       tc_fence_after();
       const uint32_t dt = tbase + buf * acc_stride;
+      if (!ok) break;
       for (int kb = 0; kb < KB; ++kb) {
-        mbar_wait_or_abort(&full[stage], phase, abort_s, P.err);
+        mbar_wait_run_on(&full[rg.stage], rg.phase, abort_s, P.err);
         tc_fence_after();
-        const uint32_t sa = ring_base + stage * stage_bytes;
+        const uint32_t sa = ring_base + rg.stage * stage_bytes;
         if (elect_one()) {
           issue_pairs<BN, NPC>(dt, sa, sa + NPC * a_bytes, a_bytes, b_bytes, kb + 1 < KB ? 4 : tail, kb != 0);
-          umma_commit(&empty[stage]);
+          umma_commit(&empty[rg.stage]);
         }
         __syncwarp();
-        if (++stage == ST) { stage = 0; phase ^= 1; }
+        rg.advance();
       }
       if (elect_one()) umma_commit(&accf[buf]);
       __syncwarp();
     }
+    ring_drain(rg, empty);
   } else if (warp < 10) {
     const uint32_t lane_t = tbase + ((uint32_t)((warp & 3) * 32) << 16);
     int it = 0, slot = 0;
     ExchWalk wk = exch_locate(P, t_lo);
     for (int t = t_lo; t < T; t += t_step, ++it, exch_advance(P, wk, t_step)) {
       const int buf = it & 1;
-      mbar_wait_or_abort(&accf[buf], (it >> 1) & 1, abort_s, P.err);
+      mbar_wait_run_on(&accf[buf], (it >> 1) & 1, abort_s, P.err);
       tc_fence_after();
       exch_tile<BN>(P, lane_t + buf * acc_stride, &acce[buf], wk.mti, wk.nti, warp - 2, slot, Fs,
                     xsum, diag, xempty, xfull, abort_s);
@@ -644,14 +636,15 @@ __global__ void __launch_bounds__(kExchThreads, 1)
   const int t_hi = (int)((long long)T * (blockIdx.x + 1) / gridDim.x);
   const int tail = (P.K - (KB - 1) * kUBK + 15) >> 4;
 
+  Ring rg{full, empty, ST};
   if (warp == 0) {
-    int stage = 0, have = -1;
-    uint32_t phase = 0, aphase = 0;
+    int have = -1;
+    uint32_t aphase = 0;
     ExchWalk wk = exch_locate(P, t_lo);
     for (int t = t_lo; t < t_hi; ++t, exch_advance(P, wk, 1)) {
       if (wk.mti != have) {
         // the blocks of the low piece that stay in shared memory
-        mbar_wait_or_abort(aempty, aphase ^ 1, abort_s, P.err);
+        if (!mbar_wait_or_abort(aempty, aphase ^ 1, abort_s, P.err)) break;
         if (nlo && elect_one()) {
           mbar_arrive_expect_tx(sfull, nlo * a_bytes);
           for (int k = 0; k < nlo; ++k)
@@ -662,49 +655,42 @@ __global__ void __launch_bounds__(kExchThreads, 1)
         aphase ^= 1;
       }
       const int brow = wk.nti * P.wpt * 2 * no;
-      for (int kb = 0; kb < KB; ++kb) {
-        mbar_wait_or_abort(&empty[stage], phase ^ 1, abort_s, P.err);
-        if (elect_one()) {
-          mbar_arrive_expect_tx(&full[stage], stage_bytes);
-          uint8_t* sb = ring + stage * stage_bytes;
-          tma_load_3d(sb, &P.tb[0], &full[stage], kb * kUBK, brow, 0);
-          tma_load_3d(sb + b_bytes, &P.tb[1], &full[stage], kb * kUBK, brow, 0);
-        }
-        __syncwarp();
-        if (++stage == ST) { stage = 0; phase ^= 1; }
-      }
+      const bool ok = ring_fill(rg, KB, abort_s, P.err, [&](int stage, int kb) {
+        mbar_arrive_expect_tx(&full[stage], stage_bytes);
+        uint8_t* sb = ring + stage * stage_bytes;
+        tma_load_3d(sb, &P.tb[0], &full[stage], kb * kUBK, brow, 0);
+        tma_load_3d(sb + b_bytes, &P.tb[1], &full[stage], kb * kUBK, brow, 0);
+      });
+      if (!ok) break;
     }
-    // drain (bounded): every stage that was filled has been released, and
-    // the low piece's last blocks have landed and been read
-    for (int s = 0; s < ST; ++s) {
-      mbar_wait_or_abort(&empty[stage], phase ^ 1, abort_s, P.err);
-      if (++stage == ST) { stage = 0; phase ^= 1; }
-    }
-    mbar_wait_or_abort(aempty, aphase ^ 1, abort_s, P.err);
+    ring_drain(rg, full);
+    if (nlo && have >= 0) mbar_wait(sfull, aphase ^ 1);  // the low piece's last blocks have landed
+    __syncwarp();
   } else if (warp == 1) {
     const uint32_t ring_base = su32(ring), alo_base = su32(alo_s), bs = b_bytes >> 4;
     const uint32_t ahi_t = tbase + kACol, alo_t = ahi_t + 8 * KS;
-    int stage = 0, have = -1, it = 0;
-    uint32_t phase = 0, aphase = 0;
+    int have = -1, it = 0;
+    uint32_t aphase = 0;
     ExchWalk wk = exch_locate(P, t_lo);
     for (int t = t_lo; t < t_hi; ++t, ++it, exch_advance(P, wk, 1)) {
       if (wk.mti != have) {
         if (have >= 0 && elect_one()) umma_commit(aempty);  // every MMA on the previous rows
         __syncwarp();
-        mbar_wait_or_abort(afull, aphase, abort_s, P.err);
-        if (nlo) mbar_wait_or_abort(sfull, aphase, abort_s, P.err);
+        mbar_wait_run_on(afull, aphase, abort_s, P.err);
+        if (nlo) mbar_wait_run_on(sfull, aphase, abort_s, P.err);
         tc_fence_after();
         aphase ^= 1;
         have = wk.mti;
       }
       const int buf = NBUF == 2 ? it & 1 : 0;
-      mbar_wait_or_abort(&acce[buf], ((it / NBUF) & 1) ^ 1, abort_s, P.err);
+      const bool ok = mbar_wait_or_abort(&acce[buf], ((it / NBUF) & 1) ^ 1, abort_s, P.err);
       tc_fence_after();
       const uint32_t dt = tbase + buf * 2 * BN;
+      if (!ok) break;
       for (int kb = 0; kb < KB; ++kb) {
-        mbar_wait_or_abort(&full[stage], phase, abort_s, P.err);
+        mbar_wait_run_on(&full[rg.stage], rg.phase, abort_s, P.err);
         tc_fence_after();
-        const uint32_t blo = smem_desc_lo(ring_base + stage * stage_bytes);
+        const uint32_t blo = smem_desc_lo(ring_base + rg.stage * stage_bytes);
         const uint32_t ahi = ahi_t + kb * 32, alo = alo_t + kb * 32;
         const uint32_t as = kb < lot ? 0u : smem_desc_lo(alo_base + (kb - lot) * a_bytes);
         const uint32_t acc = kb != 0;
@@ -714,16 +700,15 @@ __global__ void __launch_bounds__(kExchThreads, 1)
           else if (nks == 3) exch_issue_ts<BN, 3>(dt, ahi, alo, as, blo, bs, acc);
           else if (nks == 2) exch_issue_ts<BN, 2>(dt, ahi, alo, as, blo, bs, acc);
           else exch_issue_ts<BN, 1>(dt, ahi, alo, as, blo, bs, acc);
-          umma_commit(&empty[stage]);
+          umma_commit(&empty[rg.stage]);
         }
         __syncwarp();
-        if (++stage == ST) { stage = 0; phase ^= 1; }
+        rg.advance();
       }
       if (elect_one()) umma_commit(&accf[buf]);
       __syncwarp();
     }
-    if (have >= 0 && elect_one()) umma_commit(aempty);
-    __syncwarp();
+    ring_drain(rg, empty);
   } else if (warp < 10) {
     const uint32_t lane_t = tbase + ((uint32_t)((warp & 3) * 32) << 16);
     int it = 0, have = -1, slot = 0;
@@ -756,7 +741,7 @@ __global__ void __launch_bounds__(kExchThreads, 1)
         __syncwarp();
       }
       const int buf = NBUF == 2 ? it & 1 : 0;
-      mbar_wait_or_abort(&accf[buf], (it / NBUF) & 1, abort_s, P.err);
+      mbar_wait_run_on(&accf[buf], (it / NBUF) & 1, abort_s, P.err);
       tc_fence_after();
       exch_tile<BN>(P, lane_t + buf * 2 * BN, &acce[buf], wk.mti, wk.nti, warp - 2, slot, Fs,
                     xsum, diag, xempty, xfull, abort_s);

@@ -105,8 +105,7 @@ __global__ void __launch_bounds__(T::NT, 1) f64_gemm_kernel(const __grid_constan
   };
 
   if (warp == T::CW) {
-    int stage = 0;
-    uint32_t phase = 0;
+    Ring ring{full, empty, ST};
     for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
       const F64At a = locate(t);
       int k0, kt;
@@ -115,40 +114,33 @@ __global__ void __launch_bounds__(T::NT, 1) f64_gemm_kernel(const __grid_constan
       const int zb = P.s.wpt ? a.nti * P.s.wpt : (P.s.ksplit ? 0 : a.z);
       const int az = P.s.a_batched ? a.z : 0;
       const int cg0 = P.s.wpt ? 0 : a.nti * T::GROUPS;
-      for (int kb = 0; kb < kt; ++kb) {
-        mbar_wait_or_abort(&empty[stage], phase ^ 1, abort_s, P.s.err);
-        if (elect_one()) {
-          mbar_arrive_expect_tx(&full[stage], T::STAGE);
-          uint8_t* sa = smem + stage * T::STAGE;
-          const int k = k0 + kb * 16;
+      const bool ok = ring_fill(ring, kt, abort_s, P.s.err, [&](int stage, int kb) {
+        mbar_arrive_expect_tx(&full[stage], T::STAGE);
+        uint8_t* sa = smem + stage * T::STAGE;
+        const int k = k0 + kb * 16;
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            tma_load_3d(sa + h * (T::A_BYTES / 2), &P.ta, &full[stage], k + 8 * h, arow, az);
-            if (T::KIND == F64_COMPLEX)
-              tma_load_3d(sa + T::A_BYTES + h * (T::A_BYTES / 2), &P.ta2, &full[stage], k + 8 * h, arow, az);
-          }
-          uint8_t* sb = sa + T::STAGE - T::B_BYTES;
-          if (T::BMODE == F64_B_K) {
+        for (int h = 0; h < 2; ++h) {
+          tma_load_3d(sa + h * (T::A_BYTES / 2), &P.ta, &full[stage], k + 8 * h, arow, az);
+          if (T::KIND == F64_COMPLEX)
+            tma_load_3d(sa + T::A_BYTES + h * (T::A_BYTES / 2), &P.ta2, &full[stage], k + 8 * h, arow, az);
+        }
+        uint8_t* sb = sa + T::STAGE - T::B_BYTES;
+        if (T::BMODE == F64_B_K) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
-              tma_load_3d(sb + h * (T::B_BYTES / 2), &P.tb, &full[stage], k + 8 * h, a.nti * T::BN, 0);
-          } else {
-            int w = 0, c = cg0;
-            for (int q = 0; q < T::GROUPS; ++q) {
-              if (c == P.s.gpw) { c = 0; ++w; }
-              tma_load_3d(sb + q * 2048, &P.tb, &full[stage], c * 16, k, zb + w);
-              ++c;
-            }
+          for (int h = 0; h < 2; ++h)
+            tma_load_3d(sb + h * (T::B_BYTES / 2), &P.tb, &full[stage], k + 8 * h, a.nti * T::BN, 0);
+        } else {
+          int w = 0, c = cg0;
+          for (int q = 0; q < T::GROUPS; ++q) {
+            if (c == P.s.gpw) { c = 0; ++w; }
+            tma_load_3d(sb + q * 2048, &P.tb, &full[stage], c * 16, k, zb + w);
+            ++c;
           }
         }
-        __syncwarp();
-        if (++stage == ST) { stage = 0; phase ^= 1; }
-      }
+      });
+      if (!ok) break;
     }
-    for (int s = 0; s < ST; ++s) {  // drain: every stage filled has been read
-      mbar_wait_or_abort(&empty[stage], phase ^ 1, abort_s, P.s.err);
-      if (++stage == ST) { stage = 0; phase ^= 1; }
-    }
+    ring_drain(ring, full);
   } else {
     const int wm = warp & 3, wn = warp >> 2;
     const int g = lane >> 2, t4 = lane & 3;
@@ -156,8 +148,7 @@ __global__ void __launch_bounds__(T::NT, 1) f64_gemm_kernel(const __grid_constan
     const uint32_t a_off = (wm * T::FM * 8 + g) * 64 + t4 * 16;
     const uint32_t b_off0 = T::BMODE == F64_B_N ? (2 * t4) * 128 + ((g ^ (2 * t4)) << 4) : g * 64 + t4 * 16;
     const uint32_t b_off1 = (2 * t4 + 1) * 128 + ((g ^ (2 * t4 + 1)) << 4);
-    int stage = 0;
-    uint32_t phase = 0;
+    Ring ring{full, empty, ST};
     for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
       const F64At at = locate(t);
       int k0, kt;
@@ -170,8 +161,8 @@ __global__ void __launch_bounds__(T::NT, 1) f64_gemm_kernel(const __grid_constan
           acc[i][n][0][0] = acc[i][n][0][1] = acc[i][n][1][0] = acc[i][n][1][1] = 0.0;
 #pragma unroll 1
       for (int kb = 0; kb < kt; ++kb) {
-        mbar_wait_or_abort(&full[stage], phase, abort_s, P.s.err);
-        const uint8_t* sa = smem + stage * T::STAGE;
+        mbar_wait_run_on(&full[ring.stage], ring.phase, abort_s, P.s.err);
+        const uint8_t* sa = smem + ring.stage * T::STAGE;
         const uint8_t* sb = sa + T::STAGE - T::B_BYTES;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -230,8 +221,8 @@ __global__ void __launch_bounds__(T::NT, 1) f64_gemm_kernel(const __grid_constan
         // overwritten under a warp's last loads)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[stage]);
-        if (++stage == ST) { stage = 0; phase ^= 1; }
+        if (lane == 0) mbar_arrive(&empty[ring.stage]);
+        ring.advance();
       }
       P.epi.template tile<T>(at, acc, wm, wn, g, t4, epi_smem);
     }

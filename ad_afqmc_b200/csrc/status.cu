@@ -2,15 +2,15 @@
 //
 // The tensor-core kernels never spin without bound: every mbarrier wait polls
 // a limited number of times (umma.cuh), and a wait that runs out sets an int
-// flag in the caller's workspace, unwinds its CTA (drains its pipeline with
-// bounded waits, frees TMEM) and returns.  The launching call has returned
+// flag in the caller's workspace and ends its CTA: nothing more is issued, what is in flight
+// is waited for (bounded), TMEM is freed.  The launching call has returned
 // AFQ_OK long before, since every entry point is asynchronous, so the walkers
 // or energies of that call are garbage and the flag is the only record.
 // afq_check_status reads and clears it (once per block is enough: the flag
 // stays set until read); afq_status_flag gives its device address to code that
-// copies it out inside a CUDA graph.  afq_test_wait_timeout makes one bounded
-// wait run out on purpose, on an mbarrier that nothing arrives at and with no
-// copy or MMA in flight, so tests can exercise this path without a fault.
+// copies it out inside a CUDA graph.  afq_test_wait_timeout makes a producer's
+// wait run out on purpose, on a stage that nobody reads and with no copy or MMA in
+// flight, so tests can exercise this path without a fault.
 #include <cuda_runtime.h>
 
 #include "afqmc_b200.h"
@@ -31,14 +31,32 @@ int flag_ptr(const afq_dims* d, void* work, size_t work_bytes, int** out) {
   return AFQ_OK;
 }
 
-// One thread waits, with the same bounded poll loop as the GEMM pipelines,
-// for phase 0 of a fresh mbarrier whose single expected arrival never comes.
+// The producer side of a ring of two stages that nobody reads, with the GEMM
+// pipelines' own wait and fill loop; a plain arrival stands for a copy that has landed.
+// The third stage's wait runs out, which sets the flag.  Anything else than two
+// stages issued, the second fill refused at its first wait and a drain of what was
+// issued is reported as flag value 2.
 __global__ void wait_timeout_kernel(int* flag, uint32_t polls) {
-  __shared__ __align__(8) uint64_t bar;
-  if (threadIdx.x != 0) return;
-  mbar_init(&bar, 1);
-  fence_barrier_init();
-  if (!mbar_wait(&bar, 0, polls)) atomicExch(flag, 1);
+  __shared__ __align__(8) uint64_t full[2], empty[2];
+  __shared__ int abort_s, issued;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    abort_s = issued = 0;
+    fence_barrier_init();
+  }
+  __syncwarp();
+  Ring ring{full, empty, 2};
+  auto issue = [&](int stage, int) {
+    ++issued;
+    mbar_arrive(&full[stage]);
+  };
+  const bool first = ring_fill(ring, 5, &abort_s, flag, issue, polls);
+  const bool second = ring_fill(ring, 5, &abort_s, flag, issue, polls);
+  ring_drain(ring, full);
+  if (threadIdx.x == 0 && (first || second || issued != 2 || abort_s != 1)) atomicExch(flag, 2);
 }
 
 }  // namespace

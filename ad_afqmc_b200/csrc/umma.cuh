@@ -67,27 +67,38 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   return false;
 }
 
-// The waits of the GEMM kernels.  A wait that runs out sets the error flag and
-// the CTA's abort word and returns like any other; from then on every wait of
-// the CTA that is not complete at once returns too, so all roles run on to
-// their end (over data that nobody uses) and meet at the same barriers.  The
-// caller's control flow therefore does not depend on the outcome: it stays
-// uniform over the warp, and the operands of tcgen05.mma and of the TMA loads
-// stay in uniform registers.  With waits that returned a status and a single
-// branching thread, an MMA took 100-150 cycles to issue.
-static __device__ __noinline__ void mbar_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort, int* err) {
-  for (uint32_t i = 0; i < kMaxPolls; ++i) {
-    if ((i & 1023) == 0 && *abort) return;
-    if (mbar_try_wait(bar, parity)) return;
+// The waits of the GEMM kernels, called by whole warps.  A wait that runs out sets the
+// error flag and the CTA's abort word; from then on every wait of the CTA that is
+// not complete at once gives up too.
+//  * mbar_wait_or_abort returns whether the barrier completed, the same in every lane (a
+//    lane may see it complete while its neighbour polls on), so that the branch on it is
+//    uniform.  The producers test it for every stage and stop at the first failure: a
+//    barrier may not be armed again before its phase is over, nor a stage filled while
+//    it is read.  The MMA warps test it once per accumulator.
+//  * mbar_wait_run_on returns nothing.  The MMA warps use it per K block: an MMA on a stage that
+//    was not filled harms nothing, and the test there cost the exchange 10 % and
+//    a step 1 % (N = 200 and 300); the epilogue and FP64 consumer warps use it because
+//    they meet at named barriers: they run on to their end over data that nobody uses.
+// A role that issues ends with ring_drain, so that nothing lands in shared memory or
+// TMEM that the CTA no longer owns.
+static __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort, int* err,
+                                                   uint32_t max_polls) {
+  for (uint32_t i = 0; i < max_polls; ++i) {
+    if ((i & 1023) == 0 && *abort) return false;
+    if (mbar_try_wait(bar, parity)) return true;
   }
   atomicExch(err, 1);
   *abort = 1;
+  return false;
 }
-// Called by whole warps: the lanes meet again before the .aligned instructions
-// that follow (a lane may see the barrier complete while its neighbour polls on).
-__device__ __forceinline__ void mbar_wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort,
-                                                   int* err) {
-  if (!mbar_try_wait(bar, parity)) mbar_wait_slow(bar, parity, abort, err);
+__device__ __forceinline__ bool mbar_wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort, int* err,
+                                                   uint32_t max_polls = kMaxPolls) {
+  bool ok = mbar_try_wait(bar, parity);
+  if (!ok) ok = mbar_wait_slow(bar, parity, abort, err, max_polls);
+  return __all_sync(0xffffffffu, ok);
+}
+__device__ __forceinline__ void mbar_wait_run_on(uint64_t* bar, uint32_t parity, volatile int* abort, int* err) {
+  if (!mbar_try_wait(bar, parity)) mbar_wait_slow(bar, parity, abort, err, kMaxPolls);
   __syncwarp();
 }
 
@@ -96,6 +107,42 @@ __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n .reg .pred P;\n elect.sync _|P, 0xffffffff;\n selp.u32 %0, 1, 0, P;\n}" : "=r"(p));
   return p != 0;
+}
+
+// A role's place in a ring of shared-memory stages.
+struct Ring {
+  uint64_t *full, *empty;  // per stage: filled, read
+  int stages, stage = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void advance() {
+    if (++stage == stages) {
+      stage = 0;
+      phase ^= 1;
+    }
+  }
+};
+
+// The producer's n next stages: one lane calls issue(stage, i) once the stage has been
+// read.  False, with nothing more issued, once a wait fails.
+template <class Issue>
+__device__ __forceinline__ bool ring_fill(Ring& r, int n, volatile int* abort, int* err, Issue&& issue,
+                                          uint32_t max_polls = kMaxPolls) {
+  for (int i = 0; i < n; ++i) {
+    if (!mbar_wait_or_abort(&r.empty[r.stage], r.phase ^ 1, abort, err, max_polls)) return false;
+    if (elect_one()) issue(r.stage, i);
+    __syncwarp();
+    r.advance();
+  }
+  return true;
+}
+
+// The end of a role that issues: waits, whatever the abort word says, for the last round of
+// `bars` (full: the producer's copies have landed; empty: the MMAs have read their
+// stages).  Stages that were never used count as complete.
+__device__ __forceinline__ void ring_drain(const Ring& r, uint64_t* bars) {
+  Ring d = r;
+  for (int s = 0; s < r.stages; ++s, d.advance()) mbar_wait(&bars[d.stage], d.phase ^ 1);
+  __syncwarp();
 }
 
 // ---------------------------------------------------------------------------

@@ -16,7 +16,8 @@
 //               rotate over the groups, tile t in accumulator t % EG for all its
 //               K chunks, so a long epilogue of one tile runs while the other
 //               groups drain and process the next tiles
-// All waits are bounded; on timeout the CTA records an error and runs to its end.
+// All waits are bounded; on timeout the CTA records an error, stops issuing, waits for what is
+// in flight and returns.
 #pragma once
 
 #include "common.cuh"
@@ -258,44 +259,34 @@ __device__ __forceinline__ void umma_body(const Src& src) {
 
   // The producer and MMA warps run their loops whole, one elected lane issues:
   // see mbar_wait_or_abort.
+  Ring ring{full, empty, ST};
   if (warp == 0) {
-    int stage = 0;
-    uint32_t phase = 0;
     for (int it_ = blockIdx.x; it_ < tiles; it_ += gridDim.x) {
       int local;
       const UmmaParams<Epi>& P = src.entry(it_, local);
       const UmmaShape& S = P.s;
       const TileAt t = locate(S, local);
       const int arow = t.mti * S.a_step, abat = S.a_batched ? t.b : 0, brow = t.nti * S.b_step;
-      for (int kb = 0; kb < t.KB; ++kb) {
-        mbar_wait_or_abort(&empty[stage], phase ^ 1, abort_s, S.err);
-        if (elect_one()) {
-          mbar_arrive_expect_tx(&full[stage], stage_bytes);
-          uint8_t* sa = smem + stage * stage_bytes;
-          uint8_t* sb = sa + npa * a_bytes;
-          const int k = t.k0 + kb * kUBK;
-          for (int i = 0; i < npa; ++i)
-            tma_load_3d(sa + i * a_bytes, &P.ta[i], &full[stage], k, arow, abat);
-          for (int j = 0; j < npb; ++j)
-            tma_load_3d(sb + j * b_bytes, &P.tb[j], &full[stage], k, brow, t.b);
-        }
-        __syncwarp();
-        if (++stage == ST) { stage = 0; phase ^= 1; }
-      }
+      const bool ok = ring_fill(ring, t.KB, abort_s, S.err, [&](int stage, int kb) {
+        mbar_arrive_expect_tx(&full[stage], stage_bytes);
+        uint8_t* sa = smem + stage * stage_bytes;
+        uint8_t* sb = sa + npa * a_bytes;
+        const int k = t.k0 + kb * kUBK;
+        for (int i = 0; i < npa; ++i)
+          tma_load_3d(sa + i * a_bytes, &P.ta[i], &full[stage], k, arow, abat);
+        for (int j = 0; j < npb; ++j)
+          tma_load_3d(sb + j * b_bytes, &P.tb[j], &full[stage], k, brow, t.b);
+      });
+      if (!ok) break;
     }
-    // drain: wait (bounded) until the MMA side released every stage we filled
-    for (int s = 0; s < ST; ++s) {
-      mbar_wait_or_abort(&empty[stage], phase ^ 1, abort_s, P0.s.err);
-      if (++stage == ST) { stage = 0; phase ^= 1; }
-    }
+    ring_drain(ring, full);
   } else if (warp == 1) {
     constexpr uint32_t idesc = instr_desc(kUBM, BN, 1);
     const uint32_t smem_base = su32(smem);
-    int stage = 0;
-    uint32_t phase = 0;
     int it = 0, t = 0;
     uint32_t uses[NBUF] = {};  // EG > 1: chunks accumulated so far in each buffer
-    for (int it_ = blockIdx.x; it_ < tiles; it_ += gridDim.x, ++t) {
+    bool ok = true;
+    for (int it_ = blockIdx.x; ok && it_ < tiles; it_ += gridDim.x, ++t) {
       int local;
       const UmmaParams<Epi>& P = src.entry(it_, local);
       const UmmaShape& S = P.s;
@@ -305,17 +296,18 @@ __device__ __forceinline__ void umma_body(const Src& src) {
       const int kc = S.kc > 0 ? S.kc : KB;
       const int klen = min(S.kchunk, S.K - tl.k0);
       const int tail = (klen - (KB - 1) * kUBK + 15) >> 4;  // 16-wide K steps of the last block
-      for (int c0 = 0; c0 < KB; c0 += kc, ++it) {
+      for (int c0 = 0; ok && c0 < KB; c0 += kc, ++it) {
         const int buf = EG > 1 ? (t % EG) : (it & 1);
         const uint32_t use = EG > 1 ? uses[buf]++ : (uint32_t)(it >> 1);
-        mbar_wait_or_abort(&acce[buf], (use & 1) ^ 1, abort_s, S.err);
+        ok = mbar_wait_or_abort(&acce[buf], (use & 1) ^ 1, abort_s, S.err);
         tc_fence_after();
         const uint32_t dt = tbase + buf * acc_stride;
         const int c1 = min(KB, c0 + kc);
+        if (!ok) break;
         for (int kb = c0; kb < c1; ++kb) {
-          mbar_wait_or_abort(&full[stage], phase, abort_s, S.err);
+          mbar_wait_run_on(&full[ring.stage], ring.phase, abort_s, S.err);
           tc_fence_after();
-          const uint32_t sa = smem_base + stage * stage_bytes;
+          const uint32_t sa = smem_base + ring.stage * stage_bytes;
           const uint32_t sb = sa + npa * a_bytes;
           const int nks = kb + 1 < KB ? 4 : tail;
           if (elect_one()) {
@@ -335,15 +327,16 @@ __device__ __forceinline__ void umma_body(const Src& src) {
                                kb != c0 || ks != 0 || !first);
               }
             }
-            umma_commit(&empty[stage]);
+            umma_commit(&empty[ring.stage]);
           }
           __syncwarp();
-          if (++stage == ST) { stage = 0; phase ^= 1; }
+          ring.advance();
         }
         if (elect_one()) umma_commit(&accf[buf]);
         __syncwarp();
       }
     }
+    ring_drain(ring, empty);
   } else {
     const int sub = warp & 3;
     const int eg = (warp - 2) >> 2;  // epilogue warpgroup
@@ -365,7 +358,7 @@ __device__ __forceinline__ void umma_body(const Src& src) {
       for (int ch = 0; ch < nch; ++ch, ++it) {
         const int buf = EG > 1 ? eg : (it & 1);
         const uint32_t use = EG > 1 ? uses++ : (uint32_t)(it >> 1);
-        mbar_wait_or_abort(&accf[buf], use & 1, abort_s, S.err);
+        mbar_wait_run_on(&accf[buf], use & 1, abort_s, S.err);
         tc_fence_after();
         const uint32_t taddr = tbase + ((uint32_t)(sub * 32) << 16) + buf * acc_stride;
         if (nch == 1) {
