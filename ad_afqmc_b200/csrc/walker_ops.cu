@@ -186,6 +186,151 @@ __device__ void qr_inplace(double2* A, int lda, int N, int no, double2* tau, dou
   __syncthreads();
 }
 
+// ---- the same factorisation with each warp's column rows in registers ----
+// Lane l holds rows r0 + l + 32 t (t < RPL) of the column it works on, where
+// r0 is the reflector's first row; N <= 32 RPL.  All RPL loads of a column are
+// in flight together and the product and update run on registers, so a
+// column step costs one round of loads, the shuffles and one round of stores.
+template <int RPL>
+__device__ __forceinline__ void rcol_load(const double2* A, int lda, int N, int r0, int j,
+                                          double2 (&a)[RPL]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int t = 0; t < RPL; ++t) {
+    const int p = r0 + lane + 32 * t;
+    a[t] = p < N ? A[p * lda + j] : make_double2(0.0, 0.0);
+  }
+}
+
+template <int RPL>
+__device__ __forceinline__ void rcol_store(double2* A, int lda, int N, int r0, int j,
+                                           const double2 (&a)[RPL]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int t = 0; t < RPL; ++t) {
+    const int p = r0 + lane + 32 * t;
+    if (p < N) A[p * lda + j] = a[t];
+  }
+}
+
+// a -= c v (v^H a); rows beyond N hold zeros in both
+template <int RPL>
+__device__ __forceinline__ void rcol_reflect(double2 (&a)[RPL], const double2 (&v)[RPL], double2 c) {
+  double2 w0 = make_double2(0.0, 0.0), w1 = make_double2(0.0, 0.0);
+#pragma unroll
+  for (int t = 0; t < RPL; ++t) {
+    if (t & 1)
+      w1 = cadd(w1, cmul(cconj(v[t]), a[t]));
+    else
+      w0 = cadd(w0, cmul(cconj(v[t]), a[t]));
+  }
+  const double2 cw = cmul(c, warp_sum2(cadd(w0, w1)));
+#pragma unroll
+  for (int t = 0; t < RPL; ++t) a[t] = csub(a[t], cmul(v[t], cw));
+}
+
+// reflector k (zlarfg) of a column held from row k - d: pivot in lane d, t = 0
+template <int RPL>
+__device__ __forceinline__ void rcol_reflector(double2 (&a)[RPL], int d, int k, double2* tau,
+                                               double* beta) {
+  const int lane = threadIdx.x & 31;
+  double s = 0.0;
+#pragma unroll
+  for (int t = 0; t < RPL; ++t)
+    if (t > 0 || lane > d) s += a[t].x * a[t].x + a[t].y * a[t].y;
+  s = warp_sum(s);
+  const double2 al = make_double2(__shfl_sync(0xffffffffu, a[0].x, d), __shfl_sync(0xffffffffu, a[0].y, d));
+  double2 tk, sc;
+  double b;
+  if (s == 0.0 && al.y == 0.0) {
+    tk = make_double2(0.0, 0.0);
+    b = al.x;
+    sc = make_double2(1.0, 0.0);
+  } else {
+    b = -copysign(sqrt(al.x * al.x + al.y * al.y + s), al.x);
+    tk = make_double2((b - al.x) / b, -al.y / b);
+    sc = cdiv(make_double2(1.0, 0.0), make_double2(al.x - b, al.y));
+  }
+#pragma unroll
+  for (int t = 0; t < RPL; ++t)
+    if (t > 0 || lane > d) a[t] = cmul(a[t], sc);
+  if (lane == d) a[0] = make_double2(b, 0.0);
+  if (lane == 0) {
+    tau[k] = tk;
+    beta[k] = b;
+  }
+}
+
+// the reflector's rows r0 + l + 32 t (v_r0 = 1) into registers
+template <int RPL>
+__device__ __forceinline__ void rcol_vector(const double2* A, int lda, int N, int r0,
+                                            double2 (&v)[RPL]) {
+  rcol_load<RPL>(A, lda, N, r0, r0, v);
+  if ((threadIdx.x & 31) == 0) v[0] = make_double2(1.0, 0.0);
+}
+
+template <int RPL>
+__device__ void qr_inplace_reg(double2* A, int lda, int N, int no, double2* tau, double* beta) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  double2 v[RPL], a[RPL];
+  // ---- geqr2 ----------------------------------------------------------------
+  if (warp == 0) {
+    rcol_load<RPL>(A, lda, N, 0, 0, a);
+    rcol_reflector<RPL>(a, 0, 0, tau, beta);
+    rcol_store<RPL>(A, lda, N, 0, 0, a);
+  }
+  __syncthreads();
+  for (int k = 0; k + 1 < no; ++k) {
+    const double2 ct = cconj(tau[k]);
+    const bool active = ct.x != 0.0 || ct.y != 0.0;
+    const int j0 = qr_first_col(k, warp, nw);
+    if (j0 < no) {
+      rcol_vector<RPL>(A, lda, N, k, v);
+      for (int j = j0; j < no; j += nw) {
+        rcol_load<RPL>(A, lda, N, k, j, a);
+        if (active) rcol_reflect<RPL>(a, v, ct);
+        if (j == k + 1) rcol_reflector<RPL>(a, 1, k + 1, tau, beta);
+        rcol_store<RPL>(A, lda, N, k, j, a);
+      }
+    }
+    __syncthreads();
+  }
+  // ---- zung2r ---------------------------------------------------------------
+  for (int i = no - 2; i >= 0; --i) {
+    const double2 ti = tau[i];
+    const bool active = ti.x != 0.0 || ti.y != 0.0;
+    const int j0 = qr_first_col(i, warp, nw);
+    if (j0 < no) {
+      rcol_vector<RPL>(A, lda, N, i, v);
+      for (int j = j0; j < no; j += nw) {
+        rcol_load<RPL>(A, lda, N, i, j, a);
+        if (j == i + 1) {  // column j of Q from reflector j: window starts one row above it
+          const double2 tj = tau[j];
+#pragma unroll
+          for (int t = 0; t < RPL; ++t) {
+            if (t == 0 && lane == 0) a[t] = make_double2(0.0, 0.0);
+            else if (t == 0 && lane == 1) a[t] = make_double2(1.0 - tj.x, -tj.y);
+            else a[t] = cmul(make_double2(-tj.x, -tj.y), a[t]);
+          }
+          for (int p = lane; p < i; p += 32) A[p * lda + j] = make_double2(0.0, 0.0);
+        }
+        if (active) rcol_reflect<RPL>(a, v, ti);
+        rcol_store<RPL>(A, lda, N, i, j, a);
+      }
+    }
+    __syncthreads();
+  }
+  if (warp == 0) {  // column 0 of Q
+    rcol_load<RPL>(A, lda, N, 0, 0, a);
+    const double2 t0 = tau[0];
+#pragma unroll
+    for (int t = 0; t < RPL; ++t)
+      a[t] = (t == 0 && lane == 0) ? make_double2(1.0 - t0.x, -t0.y) : cmul(make_double2(-t0.x, -t0.y), a[t]);
+    rcol_store<RPL>(A, lda, N, 0, 0, a);
+  }
+  __syncthreads();
+}
+
 // ---- panels of four reflectors, columns in registers -----------------------
 // Lane l holds rows k0 + l + 32 t (t < RPL) of the column it works on, where k0
 // is the panel's first row; N <= 32 RPL.  A panel's reflectors v_m (unit entry
@@ -194,10 +339,8 @@ __device__ void qr_inplace(double2* A, int lda, int N, int no, double2* tau, dou
 //   w_m = v_m^H a (four products reduced together),
 //   c_m = conj(tau_m) (w_m - sum_{l<m} G_ml c_l),   a -= sum_m v_m c_m
 // which is the four reflectors one after the other (the same for Q, last to
-// first, with tau_m and conj(G_lm)).  Warp 0 forms a panel on its own.  One
-// reflector at a time, a block barrier, a shuffle reduction and a pass over the
-// columns for each, took 17.4 ms at N = 300 (60 + 58 columns, 1024 walkers, rows from
-// L2) and 0.76 ms at N = 157 (39 columns, 231 walkers); this takes 8.3 and 0.45 ms.
+// first, with tau_m and conj(G_lm)).  Warp 0 forms a panel on its own.  Where it is
+// the faster form, and by how much: see launch_qr.
 constexpr int kQrPanel = 4;
 
 template <int RPL>
@@ -395,11 +538,14 @@ __device__ void qr_inplace_panel(double2* A, int lda, int N, int no, double2* ta
   }
 }
 
-// grid (W, ns).  use_smem: walker copied to shared memory with row stride no+1.
-// RPL > 0: panels, register-resident columns (N <= 32 RPL, 512 threads; four
-// reflectors of 32 RPL rows behind the walker in shared memory); 0: the loop form for
-// any N (1024 threads).
-template <int RPL>
+// grid (W, ns).  use_smem: walker copied to shared memory, row stride no | 1: with 16-byte
+// entries an odd stride spreads a column over all banks (at no + 1, No = 39 put eight
+// lanes on one: N = 157, 231 walkers 781 us, 313 at no | 1).
+enum { QR_LOOP = 0, QR_REFLECTORS = 1, QR_PANELS = 2 };
+
+// RPL > 0: register-resident columns (N <= 32 RPL, 512 threads; QR_PANELS: four
+// reflectors of 32 RPL rows behind the walker in shared memory); QR_LOOP: any N (1024 threads).
+template <int METHOD, int RPL>
 __device__ __forceinline__ void qr_walker(int N, int no0, int no1, double* w0, double* w1,
                                           int sign_fix, int use_smem, double* sector_norm) {
   extern __shared__ double2 qsm[];
@@ -412,7 +558,7 @@ __device__ __forceinline__ void qr_walker(int N, int no0, int no1, double* w0, d
   double2* A = G;
   int lda = no;
   if (use_smem) {
-    lda = no + 1;
+    lda = no | 1;
     A = qsm;
     for (int e = threadIdx.x; e < N * no; e += blockDim.x) {
       const int p = e / no, j = e - (e / no) * no;
@@ -420,8 +566,10 @@ __device__ __forceinline__ void qr_walker(int N, int no0, int no1, double* w0, d
     }
     __syncthreads();
   }
-  if (RPL > 0)
-    qr_inplace_panel<(RPL > 0 ? RPL : 1)>(A, lda, N, no, tau, beta, qsm + (use_smem ? N * lda : 0), G_);
+  if (METHOD == QR_PANELS)
+    qr_inplace_panel<RPL>(A, lda, N, no, tau, beta, qsm + (use_smem ? N * lda : 0), G_);
+  else if (METHOD == QR_REFLECTORS)
+    qr_inplace_reg<RPL>(A, lda, N, no, tau, beta);
   else
     qr_inplace(A, lda, N, no, tau, beta);
   // prod diag R (real) and optional sign fix of column 0
@@ -451,14 +599,14 @@ constexpr int kQrRegThreads = 512;
 __global__ void __launch_bounds__(kQrThreads, 1)
     qr_kernel(int N, int no0, int no1, double* w0, double* w1, int sign_fix, int use_smem,
               double* sector_norm /* (ns, W) */) {
-  qr_walker<0>(N, no0, no1, w0, w1, sign_fix, use_smem, sector_norm);
+  qr_walker<QR_LOOP, 1>(N, no0, no1, w0, w1, sign_fix, use_smem, sector_norm);
 }
 
-template <int RPL>
+template <int METHOD, int RPL>
 __global__ void __launch_bounds__(kQrRegThreads, 1)
     qr_reg_kernel(int N, int no0, int no1, double* w0, double* w1, int sign_fix, int use_smem,
                   double* sector_norm /* (ns, W) */) {
-  qr_walker<RPL>(N, no0, no1, w0, w1, sign_fix, use_smem, sector_norm);
+  qr_walker<METHOD, RPL>(N, no0, no1, w0, w1, sign_fix, use_smem, sector_norm);
 }
 
 __global__ void qr_norm_kernel(int W, int ns, int restricted, const double* sector_norm,
@@ -663,28 +811,42 @@ static cudaError_t launch_qr_kernel(K kernel, int threads, dim3 grid, size_t dyn
   return cudaGetLastError();
 }
 
+// Panels of four reflectors or one reflector at a time?  Panels save passes over the columns, but
+// their products are three loads where the other form's operands are in registers: they pay
+// where the rows come from L2 (N = 300, No = 60, 1000 walkers 9.5 -> 4.3 ms) and, with ten rows
+// a lane, from about 13 columns on (N = 300, No = 40: 1.87 -> 1.69 ms; No = 10: 0.27 -> 0.29).
+// From shared memory with up to seven rows a lane they cost 9 to 40 % (N = 200, No = 40: 1.20 -> 1.34).
+template <int RPL>
+static cudaError_t launch_qr_rows(bool panels, size_t dyn, dim3 grid, cudaStream_t st, const Layout& L,
+                                  double* const walkers[2], int use_smem, double* secn) {
+  if (panels)
+    return launch_qr_kernel(qr_reg_kernel<QR_PANELS, RPL>, kQrRegThreads, grid,
+                            dyn + size_t(kQrPanel) * 32 * RPL * sizeof(double2), st, L, walkers, use_smem, secn);
+  return launch_qr_kernel(qr_reg_kernel<QR_REFLECTORS, RPL>, kQrRegThreads, grid, dyn, st, L, walkers, use_smem, secn);
+}
+
 cudaError_t launch_qr(const Layout& L, double* const walkers[2], double* norms, double* work,
                       cudaStream_t st) {
-  const size_t smem = size_t(L.N) * (L.nomax + 1) * sizeof(double2);
+  const size_t smem = size_t(L.N) * (L.nomax | 1) * sizeof(double2);
   const int use_smem = smem <= 200 * 1024 && L.tune.qr_mode != 2;
   const size_t dyn = use_smem ? smem : 0;
-  auto panel = [](int rpl) { return size_t(kQrPanel) * 32 * rpl * sizeof(double2); };
   double* secn = work;  // (ns, W) doubles of scratch at the start of the workspace
   dim3 grid(L.W, L.ns);
   cudaError_t e;
   {
     ProfScope ps(K_QR, st);
-    const int N = L.N, T = kQrRegThreads;
+    const int N = L.N;
+    const bool panels = L.nomax > 12 && (!use_smem || N > 224);
     if (N <= 32)
-      e = launch_qr_kernel(qr_reg_kernel<1>, T, grid, dyn + panel(1), st, L, walkers, use_smem, secn);
+      e = launch_qr_rows<1>(panels, dyn, grid, st, L, walkers, use_smem, secn);
     else if (N <= 64)
-      e = launch_qr_kernel(qr_reg_kernel<2>, T, grid, dyn + panel(2), st, L, walkers, use_smem, secn);
+      e = launch_qr_rows<2>(panels, dyn, grid, st, L, walkers, use_smem, secn);
     else if (N <= 128)
-      e = launch_qr_kernel(qr_reg_kernel<4>, T, grid, dyn + panel(4), st, L, walkers, use_smem, secn);
+      e = launch_qr_rows<4>(panels, dyn, grid, st, L, walkers, use_smem, secn);
     else if (N <= 224)
-      e = launch_qr_kernel(qr_reg_kernel<7>, T, grid, dyn + panel(7), st, L, walkers, use_smem, secn);
+      e = launch_qr_rows<7>(panels, dyn, grid, st, L, walkers, use_smem, secn);
     else if (N <= 320)
-      e = launch_qr_kernel(qr_reg_kernel<10>, T, grid, dyn + panel(10), st, L, walkers, use_smem, secn);
+      e = launch_qr_rows<10>(panels, dyn, grid, st, L, walkers, use_smem, secn);
     else
       e = launch_qr_kernel(qr_kernel, kQrThreads, grid, dyn, st, L, walkers, use_smem, secn);
   }
