@@ -15,8 +15,7 @@ Knobs (0 = the built-in rule):
   vhs_bn, fb_bn     tensor-core column tile of the VHS / force-bias GEMMs
   fb_splitk         split-K of the force-bias GEMM
   exch_bn           tensor-core exchange column tile (walkers per tile)
-  f64_exch_bn       row blocks of the FP64 exchange (FP64 path, or spins whose
-                    tensor-core tile does not fit shared memory)
+  f64_exch_bn       accepted in records (80, 120 or 160) and without effect
   max_stages        cap on the tcgen05 pipeline depth
   prop_order        tile order of the tensor-core propagator launches: 0
                     alternates the direction over the walkers from one launch
@@ -57,7 +56,7 @@ import torch
 from . import _lib
 from .walkers import UHFWalkers
 
-_KNOB_ORDER = ("vhs_bn", "fb_bn", "fb_splitk", "exch_bn", "f64_exch_bn", "max_stages", "prop_order")
+_KNOB_ORDER = ("vhs_bn", "fb_bn", "fb_splitk", "exch_bn", "max_stages", "prop_order")
 
 
 def shape_key(d: _lib.afq_dims) -> str:
@@ -67,7 +66,7 @@ def shape_key(d: _lib.afq_dims) -> str:
 
 def candidates(d: _lib.afq_dims) -> Dict[str, List[int]]:
     mixed = d.precision != 0
-    out: Dict[str, List[int]] = {"fb_splitk": [1, 2, 4, 8], "f64_exch_bn": [80, 120, 160]}
+    out: Dict[str, List[int]] = {"fb_splitk": [1, 2, 4, 8]}
     if mixed:
         out.update({"vhs_bn": [64, 128], "fb_bn": [64, 128], "exch_bn": [32, 64, 80, 96, 128],
                     "max_stages": [2, 3, 4], "prop_order": [1]})

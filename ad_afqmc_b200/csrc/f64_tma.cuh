@@ -16,7 +16,11 @@
 //    second, so a lane ends up with four consecutive columns, and an interleaved
 //    complex column gives re and im of the same number: the product with i z is
 //    the same registers exchanged, one negated.
-//  * B (k contiguous) is laid out like A.
+//  * B (k contiguous) is laid out like A; lane (g, t) reads rows 4 (g / 2) + g % 2 and the
+//    row two further on for the group's two MMA tiles, so that a lane ends up with four
+//    consecutive columns here too.  Its rows may be fewer than the tile's columns (F64Tile's
+//    LIVE): MMA tiles of eight columns beyond them are left out, and a group of which eight
+//    are in use takes them in order.
 // Registers-only DMMA runs at 36.5 TF/s on this chip; a cp.async main loop with
 // address arithmetic in every warp and a block barrier per stage reached 22.4.
 // Measured, N = 200, No = 40, G = 1000, 512 walkers, per step: VHS 3.65 -> 2.70 ms
@@ -25,21 +29,22 @@
 // propagator 5.20 -> 1.0 ms.
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "umma.cuh"
 
 namespace afq {
 
 enum { F64_REAL = 0, F64_COMPLEX = 1 };
-enum { F64_B_N = 0, F64_B_K = 1 };  // B contiguous along n (boxes of walkers' or plain columns), or along k
+enum { F64_B_N = 0, F64_B_K = 1 };  // B contiguous along n, or along k
 
 struct F64Shape {
   int K;               // summed length
   int mt, nt, nz;      // tiles along rows and columns, batches (or K splits)
   int arow_step;       // rows of A per tile
   int a_batched;       // A's third coordinate follows the batch
-  int gpw;             // column groups of 16 per walker (B_N with z = walker); 1 << 30: plain columns
-  int wpt;             // walkers per column tile (z advances by it), 0: z = batch
+  int brow_step;       // B_K: rows of B (columns of D) per tile, also the height of its box
   int ksplit;          // nz splits K into chunks of this length (0: no split)
   int stages;
   int epi_bytes;       // shared memory of the epilogue
@@ -53,9 +58,11 @@ struct F64Params {
   Epi epi;
 };
 
-template <int FM_, int WN_, int NG_, int KIND_, int BMODE_>
+// LIVE: brow_step may be less than BN
+template <int FM_, int WN_, int NG_, int KIND_, int BMODE_, bool LIVE_ = false>
 struct F64Tile {
   static constexpr int FM = FM_, WN = WN_, NG = NG_, KIND = KIND_, BMODE = BMODE_;
+  static constexpr bool LIVE = LIVE_;
   static constexpr int BM = 32 * FM, GROUPS = WN * NG, BN = 16 * GROUPS;
   static constexpr int CW = 4 * WN;                     // consumer warps
   static constexpr int NT = 32 * (CW + 1);
@@ -90,6 +97,7 @@ __global__ void __launch_bounds__(T::NT, 1) f64_gemm_kernel(const __grid_constan
   }
   __syncthreads();
   const int tiles = P.s.mt * P.s.nt * P.s.nz;
+  const uint32_t tx = T::LIVE ? T::STAGE - T::B_BYTES + P.s.brow_step * 128 : T::STAGE;  // bytes per stage
   auto locate = [&](int t) {
     F64At a;
     a.nti = t % P.s.nt;
@@ -111,11 +119,10 @@ __global__ void __launch_bounds__(T::NT, 1) f64_gemm_kernel(const __grid_constan
       int k0, kt;
       krange(a, k0, kt);
       const int arow = a.mti * P.s.arow_step;
-      const int zb = P.s.wpt ? a.nti * P.s.wpt : (P.s.ksplit ? 0 : a.z);
+      const int zb = P.s.ksplit ? 0 : a.z;
       const int az = P.s.a_batched ? a.z : 0;
-      const int cg0 = P.s.wpt ? 0 : a.nti * T::GROUPS;
       const bool ok = ring_fill(ring, kt, abort_s, P.s.err, [&](int stage, int kb) {
-        mbar_arrive_expect_tx(&full[stage], T::STAGE);
+        mbar_arrive_expect_tx(&full[stage], tx);
         uint8_t* sa = smem + stage * T::STAGE;
         const int k = k0 + kb * 16;
 #pragma unroll
@@ -128,14 +135,10 @@ __global__ void __launch_bounds__(T::NT, 1) f64_gemm_kernel(const __grid_constan
         if (T::BMODE == F64_B_K) {
 #pragma unroll
           for (int h = 0; h < 2; ++h)
-            tma_load_3d(sb + h * (T::B_BYTES / 2), &P.tb, &full[stage], k + 8 * h, a.nti * T::BN, 0);
+            tma_load_3d(sb + h * (T::B_BYTES / 2), &P.tb, &full[stage], k + 8 * h, a.nti * P.s.brow_step, 0);
         } else {
-          int w = 0, c = cg0;
-          for (int q = 0; q < T::GROUPS; ++q) {
-            if (c == P.s.gpw) { c = 0; ++w; }
-            tma_load_3d(sb + q * 2048, &P.tb, &full[stage], c * 16, k, zb + w);
-            ++c;
-          }
+          for (int q = 0; q < T::GROUPS; ++q)
+            tma_load_3d(sb + q * 2048, &P.tb, &full[stage], (a.nti * T::GROUPS + q) * 16, k, zb);
         }
       });
       if (!ok) break;
@@ -146,7 +149,7 @@ __global__ void __launch_bounds__(T::NT, 1) f64_gemm_kernel(const __grid_constan
     const int g = lane >> 2, t4 = lane & 3;
     // byte offsets of this lane's fragments inside a stage
     const uint32_t a_off = (wm * T::FM * 8 + g) * 64 + t4 * 16;
-    const uint32_t b_off0 = T::BMODE == F64_B_N ? (2 * t4) * 128 + ((g ^ (2 * t4)) << 4) : g * 64 + t4 * 16;
+    const uint32_t b_off0 = T::BMODE == F64_B_N ? (2 * t4) * 128 + ((g ^ (2 * t4)) << 4) : (4 * (g >> 1) + (g & 1)) * 64 + t4 * 16;
     const uint32_t b_off1 = (2 * t4 + 1) * 128 + ((g ^ (2 * t4 + 1)) << 4);
     Ring ring{full, empty, ST};
     for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
@@ -159,79 +162,103 @@ __global__ void __launch_bounds__(T::NT, 1) f64_gemm_kernel(const __grid_constan
 #pragma unroll
         for (int n = 0; n < T::NG; ++n)
           acc[i][n][0][0] = acc[i][n][0][1] = acc[i][n][1][0] = acc[i][n][1][1] = 0.0;
+      // the K loop with the first LV of this warp's MMA tiles (eight columns each)
+      auto kloop = [&](auto lv) {
+        constexpr int LV = decltype(lv)::value;
 #pragma unroll 1
-      for (int kb = 0; kb < kt; ++kb) {
-        mbar_wait_run_on(&full[ring.stage], ring.phase, abort_s, P.s.err);
-        const uint8_t* sa = smem + ring.stage * T::STAGE;
-        const uint8_t* sb = sa + T::STAGE - T::B_BYTES;
+        for (int kb = 0; kb < kt; ++kb) {
+          mbar_wait_run_on(&full[ring.stage], ring.phase, abort_s, P.s.err);
+          const uint8_t* sa = smem + ring.stage * T::STAGE;
+          const uint8_t* sb = sa + T::STAGE - T::B_BYTES;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          // b[n][ks][j]: MMA tile j of group n, k step ks
-          double b[T::NG][2][2];
-#pragma unroll
-          for (int n = 0; n < T::NG; ++n) {
-            const int q = wn * T::NG + n;
-            if (T::BMODE == F64_B_N) {
-              const double2 u = *reinterpret_cast<const double2*>(sb + q * 2048 + h * 1024 + b_off0);
-              const double2 v = *reinterpret_cast<const double2*>(sb + q * 2048 + h * 1024 + b_off1);
-              b[n][0][0] = u.x; b[n][0][1] = u.y;
-              b[n][1][0] = v.x; b[n][1][1] = v.y;
-            } else {
-              const uint8_t* p = sb + h * (T::B_BYTES / 2) + q * 1024 + b_off0;
-              const double2 u = *reinterpret_cast<const double2*>(p);
-              const double2 v = *reinterpret_cast<const double2*>(p + 512);
-              b[n][0][0] = u.x; b[n][1][0] = u.y;
-              b[n][0][1] = v.x; b[n][1][1] = v.y;
-            }
-          }
-#pragma unroll
-          for (int i = 0; i < T::FM; ++i) {
-            const double2 a = *reinterpret_cast<const double2*>(sa + h * (T::A_BYTES / 2) + a_off + i * 512);
+          for (int h = 0; h < 2; ++h) {
+            // b[n][ks][j]: MMA tile j of group n, k step ks
+            double b[T::NG][2][2];
 #pragma unroll
             for (int n = 0; n < T::NG; ++n) {
-              dmma_8x8x4(acc[i][n][0][0], acc[i][n][0][1], a.x, b[n][0][0]);
-              dmma_8x8x4(acc[i][n][1][0], acc[i][n][1][1], a.x, b[n][0][1]);
+              if (2 * n >= LV) continue;
+              const int q = wn * T::NG + n;
+              if (T::BMODE == F64_B_N) {
+                const double2 u = *reinterpret_cast<const double2*>(sb + q * 2048 + h * 1024 + b_off0);
+                const double2 v = *reinterpret_cast<const double2*>(sb + q * 2048 + h * 1024 + b_off1);
+                b[n][0][0] = u.x; b[n][0][1] = u.y;
+                b[n][1][0] = v.x; b[n][1][1] = v.y;
+              } else {
+                const bool half = 2 * n + 1 >= LV;
+                const uint8_t* p = sb + h * (T::B_BYTES / 2) + q * 1024 + (half ? g * 64 + t4 * 16 : b_off0);
+                const double2 u = *reinterpret_cast<const double2*>(p);
+                b[n][0][0] = u.x; b[n][1][0] = u.y;
+                if (!half) {
+                  const double2 v = *reinterpret_cast<const double2*>(p + 128);
+                  b[n][0][1] = v.x; b[n][1][1] = v.y;
+                }
+              }
             }
-#pragma unroll
-            for (int n = 0; n < T::NG; ++n) {
-              dmma_8x8x4(acc[i][n][0][0], acc[i][n][0][1], a.y, b[n][1][0]);
-              dmma_8x8x4(acc[i][n][1][0], acc[i][n][1][1], a.y, b[n][1][1]);
-            }
-          }
-          if (T::KIND == F64_COMPLEX) {
 #pragma unroll
             for (int i = 0; i < T::FM; ++i) {
-              const double2 a = *reinterpret_cast<const double2*>(sa + T::A_BYTES + h * (T::A_BYTES / 2) +
-                                                                  a_off + i * 512);
+              if (LV == 0) continue;
+              const double2 a = *reinterpret_cast<const double2*>(sa + h * (T::A_BYTES / 2) + a_off + i * 512);
 #pragma unroll
               for (int n = 0; n < T::NG; ++n) {
-                dmma_8x8x4(acc[i][n][0][0], acc[i][n][0][1], -a.x, b[n][0][1]);
-                dmma_8x8x4(acc[i][n][1][0], acc[i][n][1][1], a.x, b[n][0][0]);
+                if (2 * n < LV) dmma_8x8x4(acc[i][n][0][0], acc[i][n][0][1], a.x, b[n][0][0]);
+                if (2 * n + 1 < LV) dmma_8x8x4(acc[i][n][1][0], acc[i][n][1][1], a.x, b[n][0][1]);
               }
 #pragma unroll
               for (int n = 0; n < T::NG; ++n) {
-                dmma_8x8x4(acc[i][n][0][0], acc[i][n][0][1], -a.y, b[n][1][1]);
-                dmma_8x8x4(acc[i][n][1][0], acc[i][n][1][1], a.y, b[n][1][0]);
+                if (2 * n < LV) dmma_8x8x4(acc[i][n][0][0], acc[i][n][0][1], a.y, b[n][1][0]);
+                if (2 * n + 1 < LV) dmma_8x8x4(acc[i][n][1][0], acc[i][n][1][1], a.y, b[n][1][1]);
+              }
+            }
+            if (T::KIND == F64_COMPLEX) {
+#pragma unroll
+              for (int i = 0; i < T::FM; ++i) {
+                const double2 a = *reinterpret_cast<const double2*>(sa + T::A_BYTES + h * (T::A_BYTES / 2) +
+                                                                    a_off + i * 512);
+#pragma unroll
+                for (int n = 0; n < T::NG; ++n) {
+                  dmma_8x8x4(acc[i][n][0][0], acc[i][n][0][1], -a.x, b[n][0][1]);
+                  dmma_8x8x4(acc[i][n][1][0], acc[i][n][1][1], a.x, b[n][0][0]);
+                }
+#pragma unroll
+                for (int n = 0; n < T::NG; ++n) {
+                  dmma_8x8x4(acc[i][n][0][0], acc[i][n][0][1], -a.y, b[n][1][1]);
+                  dmma_8x8x4(acc[i][n][1][0], acc[i][n][1][1], a.y, b[n][1][0]);
+                }
               }
             }
           }
+          // every lane's reads of the stage complete before the TMA that refills it
+          // (generic reads, async-proxy writes: without the fence short stages were
+          // overwritten under a warp's last loads)
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&empty[ring.stage]);
+          ring.advance();
         }
-        // every lane's reads of the stage complete before the TMA that refills it
-        // (generic reads, async-proxy writes: without the fence short stages were
-        // overwritten under a warp's last loads)
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&empty[ring.stage]);
-        ring.advance();
+      };
+      if (!T::LIVE) {
+        kloop(std::integral_constant<int, 2 * T::NG>{});
+      } else {  // warp-uniform
+        const int live = (P.s.brow_step + 7) / 8 - wn * 2 * T::NG;
+        if (live >= 2 * T::NG)
+          kloop(std::integral_constant<int, 2 * T::NG>{});
+        else if (T::NG > 1 && live == 3)
+          kloop(std::integral_constant<int, (T::NG > 1 ? 3 : 0)>{});
+        else if (T::NG > 1 && live == 2)
+          kloop(std::integral_constant<int, (T::NG > 1 ? 2 : 0)>{});
+        else if (live == 1)
+          kloop(std::integral_constant<int, 1>{});
+        else
+          kloop(std::integral_constant<int, 0>{});
       }
       P.epi.template tile<T>(at, acc, wm, wn, g, t4, epi_smem);
     }
   }
 }
 
-// Calls f(row, col, v) for the lane's accumulators of one tile: v holds the
-// four consecutive columns col .. col + 3 (B_N: two complex numbers), row and col relative
-// to the tile.  B_K: columns col, col + 1 and col + 8, col + 9.
+// Calls f(row, col, v) for the lane's accumulators of one tile: v holds the four
+// consecutive columns col .. col + 3 (interleaved: two complex numbers), row and col relative
+// to the tile.  (LIVE: see exch_stage.)
 template <class T, class F>
 __device__ __forceinline__ void f64_each(double (&acc)[T::FM][T::NG][2][2], int wm, int wn, int g, int t4,
                                          F&& f) {
@@ -239,11 +266,11 @@ __device__ __forceinline__ void f64_each(double (&acc)[T::FM][T::NG][2][2], int 
   for (int i = 0; i < T::FM; ++i)
 #pragma unroll
     for (int n = 0; n < T::NG; ++n) {
-      const int row = (wm * T::FM + i) * 8 + g, c = (wn * T::NG + n) * 16;
+      const int row = (wm * T::FM + i) * 8 + g, c = (wn * T::NG + n) * 16 + 4 * t4;
       if (T::BMODE == F64_B_N)
-        f(row, c + 4 * t4, acc[i][n][0][0], acc[i][n][1][0], acc[i][n][0][1], acc[i][n][1][1]);
+        f(row, c, acc[i][n][0][0], acc[i][n][1][0], acc[i][n][0][1], acc[i][n][1][1]);
       else
-        f(row, c + 2 * t4, acc[i][n][0][0], acc[i][n][0][1], acc[i][n][1][0], acc[i][n][1][1]);
+        f(row, c, acc[i][n][0][0], acc[i][n][0][1], acc[i][n][1][0], acc[i][n][1][1]);
     }
 }
 

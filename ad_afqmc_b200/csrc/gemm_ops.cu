@@ -21,8 +21,6 @@ int sm_count();
 
 namespace {
 
-constexpr int kPlain = 1 << 30;  // column groups of a plain (not per-walker) operand: more than any has (N^2 < 2^31)
-
 // ---------------------------------------------------------------------------
 // force bias: C[z] (2W x G) = Gpl (2W x Kfb) * RCcat^T, K split over z
 // ---------------------------------------------------------------------------
@@ -39,7 +37,7 @@ struct FbEpi {
       if (m >= M) return;
       double* p = Cz + m * ldc + n;  // ldc even, n even: pairs are aligned, the pad column is never read
       if (n < N) *reinterpret_cast<double2*>(p) = make_double2(v0, v1);
-      if (n + 8 < N) *reinterpret_cast<double2*>(p + 8) = make_double2(v2, v3);
+      if (n + 2 < N) *reinterpret_cast<double2*>(p + 2) = make_double2(v2, v3);
     });
   }
 };
@@ -203,19 +201,26 @@ __device__ __forceinline__ void f64_consumer_sync() {
   asm volatile("bar.sync 1, %0;" ::"n"(32 * T::CW) : "memory");
 }
 
-// The tile of f in shared memory: rows (Cholesky vector, i), a walker's columns
-// at a stride of 16 gpw doubles; row stride BN + 2 doubles, so that 16-byte loads
+// The tile of f in shared memory: rows (Cholesky vector, i), a walker's 2 No columns
+// one after the other; row stride BN + 2 doubles, so that 16-byte loads
 // down a column (4 banks apart) and along a row are conflict-free.
 template <class T>
-__device__ __forceinline__ double* exch_stage(double (&acc)[T::FM][T::NG][2][2], int wm, int wn, int g, int t4,
-                                              uint8_t* smem) {
+__device__ __forceinline__ double* exch_stage(double (&acc)[T::FM][T::NG][2][2], int cols, int wm, int wn, int g,
+                                              int t4, uint8_t* smem) {
   constexpr int CS = T::BN + 2;
   double* Ct = reinterpret_cast<double*>(smem);
-  f64_each<T>(acc, wm, wn, g, t4, [&](int row, int c, double v0, double v1, double v2, double v3) {
-    double2* p = reinterpret_cast<double2*>(Ct + row * CS + c);
-    p[0] = make_double2(v0, v1);
-    p[1] = make_double2(v2, v3);
-  });
+#pragma unroll
+  for (int n = 0; n < T::NG; ++n) {
+    const int c0 = (wn * T::NG + n) * 16;
+    if (c0 >= cols) continue;  // warp-uniform
+    const bool half = cols - c0 <= 8;  // only the first MMA tile, its columns in order
+    double* p = Ct + (wm * T::FM * 8 + g) * CS + c0 + (half ? 2 : 4) * t4;
+#pragma unroll
+    for (int i = 0; i < T::FM; ++i) {
+      *reinterpret_cast<double2*>(p + i * 8 * CS) = make_double2(acc[i][n][0][0], acc[i][n][0][1]);
+      if (!half) *reinterpret_cast<double2*>(p + i * 8 * CS + 2) = make_double2(acc[i][n][1][0], acc[i][n][1][1]);
+    }
+  }
   f64_consumer_sync<T>();
   return Ct;
 }
@@ -226,67 +231,54 @@ inline size_t exch_stage_bytes(int extra) {
 
 // ---------------------------------------------------------------------------
 // fused exchange: tile = gpt Cholesky vectors x wpt walkers.  Per block (g, w):
-// tr f and sum_ij f_ij f_ji = sum_i f_ii^2 + 2 sum_{i<j} f_ij f_ji, rows dealt to
-// the warps of the block.
+// tr f and sum_ij f_ij f_ji = sum_i f_ii^2 + 2 sum_{i<j} f_ij f_ji.
 // ---------------------------------------------------------------------------
 struct ExchEpi {
-  int G, no, W, gpt, wpt, gpw;
+  int G, no, W, gpt, wpt;
   double* cout;
   double* excout;
   template <class T>
   __device__ void tile(const F64At& at, double (&acc)[T::FM][T::NG][2][2], int wm, int wn, int g, int t4,
                        uint8_t* smem) const {
     constexpr int CS = T::BN + 2, CW = T::CW;
-    const double* Ct = exch_stage<T>(acc, wm, wn, g, t4, smem);
+    const double* Ct = exch_stage<T>(acc, 2 * no * wpt, wm, wn, g, t4, smem);
     double4* blk = reinterpret_cast<double4*>(smem + size_t(T::BM) * CS * 8);  // [CW or more][block]
     const int g0 = at.mti * gpt, w0 = at.nti * wpt;
     const int gcount = min(gpt, G - g0), wcount = min(wpt, W - w0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nblk = gcount * wcount, parts = max(1, CW / nblk);
-    // No < 32: the lanes walk the whole square i, j (No^2 / 32 passes); from 32 on rows
-    // of the triangle (fewer passes there).  With rows, No = 10 left 22 lanes of 32 idle:
-    // No = 10 + 9, 238 walkers 363 -> 265 us, No = 17, 60 walkers 199 -> 154 us.
-    const int di = 32 * parts / no, dj = 32 * parts - di * no;
+    // The lanes walk the triangle i <= j folded to a rectangle: row r holds the No - r
+    // entries of row r and the r + 1 of row No - 1 - r (odd No: the middle row alone).
+    const int len = no + 1, di = 32 * parts / len, dj = 32 * parts - di * len;
     for (int e = warp; e < nblk * parts; e += CW) {
       const int b = e / parts, part = e - b * parts;
       const int gl = b % gcount, wl = b / gcount;
-      const double* F = Ct + gl * no * CS + wl * 16 * gpw;
+      const double* F = Ct + (gl * CS + 2 * wl) * no;
       double er = 0, ei = 0, dr = 0, dgi = 0, cr = 0, ci = 0;
-      if (no < 32) {
-        int i = (part * 32 + lane) / no, j = part * 32 + lane - i * no;
-        while (i < no) {
+      int r = (part * 32 + lane) / len, q = part * 32 + lane - r * len;
+      while (2 * r < no) {
+        const bool second = q >= no - r;
+        const int i = second ? no - 1 - r : r, j = second ? i + q - (no - r) : r + q;
+        if (!second || 2 * r + 1 < no) {
           const double2 fij = *reinterpret_cast<const double2*>(F + i * CS + 2 * j);
           const double2 fji = *reinterpret_cast<const double2*>(F + j * CS + 2 * i);
-          er += fij.x * fji.x - fij.y * fji.y;
-          ei += fij.x * fji.y + fij.y * fji.x;
+          const double pr = fij.x * fji.x - fij.y * fji.y, pi = fij.x * fji.y + fij.y * fji.x;
           if (i == j) {
+            dr += pr;
+            dgi += pi;
             cr += fij.x;
             ci += fij.y;
-          }
-          i += di;
-          j += dj;
-          if (j >= no) {
-            j -= no;
-            ++i;
+          } else {
+            er += pr;
+            ei += pi;
           }
         }
-        er *= 0.5;  // doubled again below (exact)
-        ei *= 0.5;
-      } else {
-        for (int i = part; i < no; i += parts)
-          for (int j = i + lane; j < no; j += 32) {
-            const double2 fij = *reinterpret_cast<const double2*>(F + i * CS + 2 * j);
-            const double2 fji = *reinterpret_cast<const double2*>(F + j * CS + 2 * i);
-            if (j == i) {
-              dr += fij.x * fij.x - fij.y * fij.y;
-              dgi += 2.0 * fij.x * fij.y;
-              cr += fij.x;
-              ci += fij.y;
-            } else {
-              er += fij.x * fji.x - fij.y * fji.y;
-              ei += fij.x * fji.y + fij.y * fji.x;
-            }
-          }
+        r += di;
+        q += dj;
+        if (q >= len) {
+          q -= len;
+          ++r;
+        }
       }
       er = dr + 2.0 * er;
       ei = dgi + 2.0 * ei;
@@ -312,14 +304,19 @@ struct ExchEpi {
       cout[co] = s.z;
       cout[co + 1] = s.w;
     }
-    for (int wl = threadIdx.x; wl < wcount; wl += 32 * CW) {
+    for (int wl = CW - 1 - warp; wl < wcount; wl += CW) {  // a warp per walker
+      const double4* u = blk + wl * gcount * parts;
       double sx = 0, sy = 0;
-      for (int e = wl * gcount * parts; e < (wl + 1) * gcount * parts; ++e) {
-        sx += blk[e].x;
-        sy += blk[e].y;
+      for (int e = lane; e < gcount * parts; e += 32) {
+        sx += u[e].x;
+        sy += u[e].y;
       }
-      excout[2 * ((long long)at.mti * W + w0 + wl)] = sx;
-      excout[2 * ((long long)at.mti * W + w0 + wl) + 1] = sy;
+      sx = warp_sum(sx);
+      sy = warp_sum(sy);
+      if (lane == 0) {
+        excout[2 * ((long long)at.mti * W + w0 + wl)] = sx;
+        excout[2 * ((long long)at.mti * W + w0 + wl) + 1] = sy;
+      }
     }
     f64_consumer_sync<T>();
   }
@@ -336,7 +333,7 @@ struct ExchEpi {
 constexpr int kMaxLo = 8;
 
 struct OrbEpi {
-  int G, no, W, gpt, wpt, gpw, nlo;
+  int G, no, W, gpt, wpt, nlo;
   const double* prj;
   double* orbout;
   template <class T>
@@ -346,14 +343,14 @@ struct OrbEpi {
     double* P = reinterpret_cast<double*>(smem) + T::BM * CS;  // nlo x no projector rows
     double2* blk = reinterpret_cast<double2*>(P + kMaxLo * 64);
     for (int e = threadIdx.x; e < nlo * no; e += 32 * CW) P[e] = prj[e];
-    const double* Ct = exch_stage<T>(acc, wm, wn, g, t4, smem);
+    const double* Ct = exch_stage<T>(acc, 2 * no * wpt, wm, wn, g, t4, smem);
     const int g0 = at.mti * gpt, w0 = at.nti * wpt;
     const int gcount = min(gpt, G - g0), wcount = min(wpt, W - w0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nblk = gcount * wcount;
     for (int bi = warp; bi < nblk; bi += CW) {
       const int gl = bi % gcount, wl = bi / gcount;
-      const double* F = Ct + gl * no * CS + wl * 16 * gpw;
+      const double* F = Ct + (gl * CS + 2 * wl) * no;
       double cr = 0, ci = 0, ar = 0, ai = 0, br = 0, bi_ = 0;
       for (int k = lane; k < no; k += 32) {
         cr += F[k * CS + 2 * k];
@@ -401,14 +398,12 @@ struct OrbEpi {
   }
 };
 
-// Theta (W, N, No) complex: rows p < No set to zero (the occupied block)
-__global__ void theta_zero_occ_kernel(double2* theta, int W, int N, int no) {
-  const long long n = (long long)W * no * no;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
-       e += (long long)gridDim.x * blockDim.x) {
-    const long long w = e / ((long long)no * no), r = e - w * no * no;
-    theta[w * N * no + r] = make_double2(0.0, 0.0);
-  }
+// Theta (rows (walker, i, re/im) of N doubles at stride ld): columns p < No set to
+// zero (the occupied block)
+__global__ void theta_zero_occ_kernel(double* theta, long long rows, long long ld, int no) {
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < rows * no;
+       e += (long long)gridDim.x * blockDim.x)
+    theta[e / no * ld + e % no] = 0.0;
 }
 
 // orbital energy per walker: sum of the row-tile partials (one warp per walker)
@@ -539,7 +534,6 @@ cudaError_t prop_run(const Layout& L, double* work, int nc, const PropCall& c, c
   P.s.nz = W;
   P.s.arow_step = T::BM;
   P.s.a_batched = c.abs != 0;
-  P.s.gpw = kPlain;
   P.s.err = f64_err(L, work);
   P.epi = PropEpi{c.out, c.yin, c.scale, N, nc};
   const size_t smem = 1024 + f64_stages<T>(0) * size_t(T::STAGE) + 256;
@@ -582,39 +576,58 @@ cudaError_t prop_gemm(const Layout& L, double* work, int nc, const PropCall& c, 
 #undef AFQ_PROP_WN
 }
 
-// Exchange and orbital-energy tiles: 128 rows (the layout's gpt Cholesky vectors), wpt
-// walkers of gpw column groups; calls f with the tile type.
+// Exchange and orbital-energy tiles: 128 rows (gpt Cholesky vectors) and the 2 No columns
+// of wpt walkers, which lie one after the other in Theta's rows; calls f with the tile type.
+// The choice with the smallest ceil(tiles / SMs) times the tile's MMA tiles of eight columns
+// (plus 2.2 for its share of A, its loads and barriers: the fit to No = 9 with 1 to 4 walkers);
+// at most 512 (Cholesky vector, walker) blocks, whose sums sit in shared memory.
+// 80 columns leave room for four operand stages; 96, with three, pay where they hold more
+// of the walkers (No = 15, 16, 21 to 24); 112, in 28 warps, two walkers of No = 25 to 28 (N = 60,
+// No = 26, 1024 walkers 2.87 -> 2.38 ms); 128, with two stages, only hold what needs them.
+// With every walker padded to groups of 16 columns, at most four to a tile, No = 2, 4, 9, 10, 26
+// took longer than the kernel before, whose tiles held whole walkers without
+// padding (energies at N = 300, 1024 walkers, ms, that one, padded, now: No = 2 0.90, 1.24, 0.66;
+// No = 9 5.95, 7.25, 4.32; No = 10 7.02, 8.42, 5.38; No = 20 25.6, 23.7, 20.3).
 template <class F>
-cudaError_t with_exch_tile(int no, int& wpt, int& gpw, F&& f) {
-  gpw = (2 * no + 15) / 16;
-  wpt = gpw == 1 ? 4 : (gpw <= 3 ? 2 : 1);
-  switch (gpw) {
-    case 1:
-    case 2:
-    case 4: return f(F64Tile<4, 4, 1, F64_REAL, F64_B_N>());
-    case 3:
-    case 6: return f(F64Tile<4, 3, 2, F64_REAL, F64_B_N>());
-    case 5: return f(F64Tile<4, 5, 1, F64_REAL, F64_B_N>());
-    default: return f(F64Tile<4, 4, 2, F64_REAL, F64_B_N>());  // 7, 8
+cudaError_t with_exch_tile(int no, int G, int W, int& wpt, F&& f) {
+  const int gpt = 128 / no, most = 512 / gpt, sms = sm_count();
+  const long long mt = (G + gpt - 1) / gpt;
+  double best = 1e300;
+  int bn = 128;
+  wpt = 1;
+  for (int b : {80, 96, 112})
+    for (int n = 1; n <= most && 2 * no * n <= b && (b < 112 || (no >= 25 && no <= 28)); ++n) {
+      const long long waves = (mt * ((W + n - 1) / n) + sms - 1) / sms;
+      const double cost = double(waves) * ((2 * no * n + 7) / 8 + 2.2) * (b > 80 ? 1.05 : 1.0);
+      if (cost < best - 1e-9) {
+        best = cost;
+        bn = b;
+        wpt = n;
+      }
+    }
+  switch (bn) {
+    case 80: return f(F64Tile<4, 5, 1, F64_REAL, F64_B_K, true>());
+    case 96: return f(F64Tile<4, 3, 2, F64_REAL, F64_B_K, true>());
+    case 112: return f(F64Tile<4, 7, 1, F64_REAL, F64_B_K, true>());
+    default: return f(F64Tile<4, 4, 2, F64_REAL, F64_B_K, true>());
   }
 }
 
 template <class T, class Epi>
 cudaError_t exch_run(const Layout& L, const double* prep, double* work, int s, F64Params<Epi>& P, int wpt,
-                     int gpw, int extra, cudaStream_t st) {
-  const int no = L.no[s], gpt = L.ex[s].bm / no;
+                     int extra, cudaStream_t st) {
+  const int no = L.no[s], gpt = L.ex[s].gpt;
+  const long long rows = (long long)L.W * 2 * no;
   if (make_tmap_f64(&P.ta, prep + L.p_rc[s], L.N, (long long)L.G * no, 1, L.Npad, L.Npad * L.G * no, 8, T::BM) !=
           AFQ_OK ||
-      make_tmap_f64(&P.tb, work + L.w_theta[s], 2 * no, L.N, L.W, 2 * no, (long long)L.N * 2 * no, 16, 16) !=
-          AFQ_OK)
+      make_tmap_f64(&P.tb, work + L.w_theta[s], L.N, rows, 1, L.Npad, L.Npad * rows, 8, wpt * 2 * no) != AFQ_OK)
     return cudaErrorInvalidValue;
   P.s.K = L.N;
   P.s.mt = (L.G + gpt - 1) / gpt;
   P.s.nt = (L.W + wpt - 1) / wpt;
   P.s.nz = 1;
   P.s.arow_step = gpt * no;
-  P.s.gpw = gpw;
-  P.s.wpt = wpt;
+  P.s.brow_step = wpt * 2 * no;
   P.s.err = f64_err(L, work);
   P.s.epi_bytes = (int)exch_stage_bytes<T>(extra);
   ProfScope ps(K_EXCH, st);
@@ -646,6 +659,7 @@ cudaError_t launch_fb_gemm(const Layout& L, const double* prep, double* work, cu
     P.s.nt = (N + T::BN - 1) / T::BN;
     P.s.nz = ks;
     P.s.arow_step = T::BM;
+    P.s.brow_step = T::BN;
     P.s.ksplit = kchunk;
     P.s.err = f64_err(L, work);
     P.epi = FbEpi{part, L.Gpad, zs, M, N};
@@ -714,7 +728,6 @@ cudaError_t launch_vhs_gemm(const Layout& L, const double* prep, double* work, c
     P.s.nt = (NN + T::BN - 1) / T::BN;
     P.s.nz = 1;
     P.s.arow_step = T::BM;
-    P.s.gpw = kPlain;
     P.s.err = f64_err(L, work);
     P.epi = VhsEpi{work + L.w_vhs, M, NN, L.N, L.Npad};
     ProfScope ps(K_VHS, st);
@@ -755,13 +768,13 @@ cudaError_t launch_propagate_walkers(const Layout& L, const double* prep, double
 
 cudaError_t launch_exchange(const Layout& L, const double* prep, double* work, int s,
                             cudaStream_t st) {
-  const int no = L.no[s], gpt = L.ex[s].bm / no;
-  int wpt, gpw;
-  return with_exch_tile(no, wpt, gpw, [&](auto tile) {
+  const int no = L.no[s], gpt = L.ex[s].gpt;
+  int wpt;
+  return with_exch_tile(no, L.G, L.W, wpt, [&](auto tile) {
     using T = decltype(tile);
     F64Params<ExchEpi> P{};
-    P.epi = ExchEpi{L.G, no, L.W, gpt, wpt, gpw, work + L.w_c[s], work + L.w_exc[s]};
-    return exch_run<T>(L, prep, work, s, P, wpt, gpw, 4 * (gpt * wpt + T::CW), st);
+    P.epi = ExchEpi{L.G, no, L.W, gpt, wpt, work + L.w_c[s], work + L.w_exc[s]};
+    return exch_run<T>(L, prep, work, s, P, wpt, 4 * (gpt * wpt + T::CW), st);
   });
 }
 
@@ -770,18 +783,17 @@ cudaError_t launch_orbenergy(const Layout& L, const double* prep, double* work, 
   if (nlo < 1 || nlo > kMaxLo || L.no[0] > 64) return cudaErrorInvalidValue;
   {
     ProfScope ps(K_MISC, st);
-    theta_zero_occ_kernel<<<256, 256, 0, st>>>(reinterpret_cast<double2*>(work + L.w_theta[0]), L.W,
-                                               L.N, L.no[0]);
+    theta_zero_occ_kernel<<<256, 256, 0, st>>>(work + L.w_theta[0], (long long)L.W * 2 * L.no[0], L.Npad, L.no[0]);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  const int no = L.no[0], gpt = L.ex[0].bm / no;
-  int wpt, gpw;
-  e = with_exch_tile(no, wpt, gpw, [&](auto tile) {
+  const int no = L.no[0], gpt = L.ex[0].gpt;
+  int wpt;
+  e = with_exch_tile(no, L.G, L.W, wpt, [&](auto tile) {
     using T = decltype(tile);
     F64Params<OrbEpi> P{};
-    P.epi = OrbEpi{L.G, no, L.W, gpt, wpt, gpw, nlo, prj, work + L.w_orb};
-    return exch_run<T>(L, prep, work, 0, P, wpt, gpw, kMaxLo * 64 + 2 * gpt * wpt, st);
+    P.epi = OrbEpi{L.G, no, L.W, gpt, wpt, nlo, prj, work + L.w_orb};
+    return exch_run<T>(L, prep, work, 0, P, wpt, kMaxLo * 64 + 2 * gpt * wpt, st);
   });
   if (e != cudaSuccess) return e;
   const int wpb = 8;

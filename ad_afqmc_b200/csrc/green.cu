@@ -186,7 +186,7 @@ __device__ __forceinline__ void green_body(const GreenArgs& a, int mode, int w, 
 
   // ---- Theta = W S^-1, transposed copies, E1 --------------------------------
   double2 e1 = make_double2(0.0, 0.0);
-  double2* th = S_.theta ? reinterpret_cast<double2*>(S_.theta) + (long long)w * N * no : nullptr;
+  double* th = S_.theta ? S_.theta + (long long)w * 2 * no * S_.ldth : nullptr;
   double2* go = S_.gout ? reinterpret_cast<double2*>(S_.gout) + (long long)w * no * N : nullptr;
   double* gre = a.gpl ? a.gpl + (2LL * w) * a.ldg + S_.koff : nullptr;
   double* gim = a.gpl ? a.gpl + (2LL * w + 1) * a.ldg + S_.koff : nullptr;
@@ -253,7 +253,6 @@ __device__ __forceinline__ void green_body(const GreenArgs& a, int mode, int w, 
         if (r < rows && j < no) {
           const double2 sv = make_double2(tacc[ri][0], tacc[ri][1]);
           tstage[r * ts + j] = sv;
-          if (th) th[(long long)(p0 + r) * no + j] = sv;
           if (S_.rh1) {
             const double h = S_.rh1[(long long)j * N + p0 + r];
             e1.x = fma(sv.x, h, e1.x);
@@ -263,10 +262,14 @@ __device__ __forceinline__ void green_body(const GreenArgs& a, int mode, int w, 
       }
     }
     __syncthreads();
-    if (go || gre || gb || tb) {
+    if (th || go || gre || gb || tb) {
       for (int e = tid; e < rows * no; e += T) {
         const int j = rows == kRowChunk ? e / kRowChunk : e / rows, r = e - j * rows;
         const double2 v = tstage[r * ts + j];
+        if (th) {
+          th[2 * j * S_.ldth + p0 + r] = v.x;
+          th[(2 * j + 1) * S_.ldth + p0 + r] = v.y;
+        }
         if (go) go[(long long)j * N + p0 + r] = v;
         if (gre) {
           gre[(long long)j * N + p0 + r] = v.x;

@@ -19,14 +19,11 @@ void tuning_store(const afq_dims& d, const afq_tuning* t);
 inline long long round_even(long long x) { return (x + 1) & ~1LL; }
 inline long long align_up(long long x, long long a) { return (x + a - 1) / a * a; }
 
-// Exchange-energy tile choice (see exchange kernel): gpt Cholesky vectors
-// per BM-row tile and wpt walkers per BN-column tile.
+// Rows of the FP64 exchange's blocks: gpt Cholesky vectors, 128 rows at most.
 struct ExchTile {
-  int bm;   // 120 or 128
-  int bn;   // 80, 120 or 160
-  int gpt;  // Cholesky vectors per tile
-  int wpt;  // walkers per tile
-  int mt;   // number of row tiles = ceil(G / gpt)
+  int bn;   // f64_exch_bn as reported
+  int gpt;  // Cholesky vectors per block
+  int mt;   // number of blocks = ceil(G / gpt)
 };
 
 // Shared memory of the tensor-core exchange epilogue: the f block as
@@ -115,30 +112,13 @@ struct Layout {
   long long w_c[2], w_exc[2], w_orb, w_s, w_cum, w_idx, w_misc, work;
 };
 
-inline ExchTile choose_exch_tile(int no, int G, int W) {
-  // (BM, BN) of the FP64 exchange kernels: 120 x 80, 120 x 120, 128 x 160
-  const int bms[3] = {120, 120, 128}, bns[3] = {80, 120, 160};
-  ExchTile best{0, 0, 0, 0, 0};
-  double best_eff = -1.0;
-  for (int i = 0; i < 3; ++i) {
-    const int bm = bms[i], bn = bns[i];
-    if (2 * no > bn || no > bm) continue;
-    const int gpt = bm / no, wpt = bn / (2 * no);
-    const double eff = double(gpt * no) / bm * double(wpt * 2 * no) / double(bn);
-    if (eff > best_eff + 1e-9) {
-      best_eff = eff;
-      best = ExchTile{bm, bn, gpt, wpt, (G + gpt - 1) / gpt};
-    }
-  }
-  (void)W;
-  return best;
-}
-
+// f64_exch_bn once chose among three column tiles; records that name one are taken as before (a
+// value that cannot hold a walker is refused) and change nothing.
 inline ExchTile exch_tile_for(int no, int G, int bn) {
-  const int bm = bn == 160 ? 128 : 120;
-  if ((bn != 80 && bn != 120 && bn != 160) || 2 * no > bn || no > bm) return ExchTile{0, 0, 0, 0, 0};
-  const int gpt = bm / no;
-  return ExchTile{bm, bn, gpt, bn / (2 * no), (G + gpt - 1) / gpt};
+  const int gpt = 128 / no, mt = (G + gpt - 1) / gpt;
+  if (bn == 0) bn = no <= 40 ? 80 : (no <= 60 ? 120 : 160);
+  if ((bn != 80 && bn != 120 && bn != 160) || 2 * no > bn) return ExchTile{0, gpt, mt};
+  return ExchTile{bn, gpt, mt};
 }
 
 // Returns AFQ_OK and fills L, or a shape error.
@@ -204,9 +184,8 @@ inline int make_layout(const afq_dims* d, Layout& L, const afq_tuning* record = 
   if (T.vhs_bn != 0 && T.vhs_bn != 64 && T.vhs_bn != 128) return AFQ_ERR_ARG;
   if (T.fb_splitk > 0) L.splitk = T.fb_splitk;
   for (int s = 0; s < 2; ++s) {
-    L.ex[s] = T.f64_exch_bn ? exch_tile_for(L.no[s], L.G, T.f64_exch_bn)
-                            : choose_exch_tile(L.no[s], L.G, L.W);
-    if (T.f64_exch_bn && L.ex[s].bn == 0 && s < L.ns) return AFQ_ERR_ARG;
+    L.ex[s] = exch_tile_for(L.no[s], L.G, T.f64_exch_bn);
+    if (L.ex[s].bn == 0 && s < L.ns) return AFQ_ERR_ARG;
   }
   L.mixed = d->precision != AFQ_FP64;
   L.npc = d->precision == AFQ_MIXED_HI ? 3 : 2;
@@ -224,7 +203,6 @@ inline int make_layout(const afq_dims* d, Layout& L, const afq_tuning* record = 
     }
   }
   for (int s = 0; s < 2; ++s) {
-    if (L.ex[s].bn == 0 && s < L.ns) return AFQ_ERR_SHAPE;
     // three-piece operands of a large occupied block leave no room for two
     // pipeline stages of the tensor-core exchange: that spin's exchange runs
     // on the FP64 kernel (exact) instead
@@ -282,7 +260,7 @@ inline int make_layout(const afq_dims* d, Layout& L, const afq_tuning* record = 
   const long long W = L.W, N = L.N;
   L.w_gpl = take(W * 2 * L.Kfb);
   for (int s = 0; s < 2; ++s) L.w_theta[s] = -1;
-  for (int s = 0; s < L.ns; ++s) L.w_theta[s] = take(W * N * 2 * L.no[s]);
+  for (int s = 0; s < L.ns; ++s) L.w_theta[s] = take(W * 2 * L.no[s] * L.Npad);
   L.w_xt = take(2 * W * L.Gpad);
   L.w_wscal = take(W * 16);
   L.w_vhs = take(W * N * 2 * L.Npad);

@@ -15,7 +15,8 @@ struct GreenSector {
   const double* rh1;    // (no, N) or nullptr
   int no;
   long long koff;       // offset of this sector inside a G-planar row
-  double* theta;        // (W, N, no) complex or nullptr
+  double* theta;        // rows (w, j, re/im) of N doubles, row stride ldth, or nullptr
+  long long ldth;
   double* gout;         // (W, no, N) complex or nullptr
   bf16* gtb[3];         // exchange operand pieces: rows (w, j, re/im), row stride ldtb, or nullptr
   long long ldtb;
@@ -120,6 +121,7 @@ inline GreenArgs green_args_mo(const Layout& L, const double* const mo[2], doubl
     a.sec[s].no = L.no[s];
     a.sec[s].koff = L.koff[s];
     a.sec[s].theta = nullptr;
+    a.sec[s].ldth = L.Npad;
     a.sec[s].gout = nullptr;
     for (int i = 0; i < 3; ++i) a.sec[s].gtb[i] = nullptr;
     a.sec[s].ldtb = L.Nb;

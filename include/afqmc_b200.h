@@ -288,7 +288,7 @@ typedef struct afq_tuning {
   int32_t fb_bn;       /* tensor-core force-bias column tile: 64 or 128                  */
   int32_t vhs_bn;      /* tensor-core VHS column tile: 64 or 128                          */
   int32_t exch_bn;     /* tensor-core exchange column tile: 32, 64, 80, 96 or 128         */
-  int32_t f64_exch_bn; /* rows of the FP64 exchange's blocks: 80, 120 or 160 (120, 120, 128) */
+  int32_t f64_exch_bn; /* 80, 120 or 160, at least 2 No: accepted, without effect         */
   int32_t max_stages;  /* cap on tcgen05 pipeline stages: 2..8                             */
   int32_t grid_cap;    /* CTAs of the persistent tensor-core kernels: 1..number of SMs     */
   int32_t prop_epi_groups; /* epilogue warpgroups of the tensor-core propagator: 1 to 3    */
