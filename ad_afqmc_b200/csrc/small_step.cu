@@ -16,6 +16,8 @@
 
 namespace afq {
 
+int sm_count();
+
 namespace {
 
 constexpr int kSmallThreads = 256;
@@ -304,14 +306,28 @@ __global__ void __launch_bounds__(kSmallThreads) small_step_kernel(const SmallAr
 
 }  // namespace
 
-// Where this kernel is the faster one.  Recorded blocks of 10 steps, us, this
-// kernel against the tensor-core launches: N = 6 UHF, 50 walkers 336 / 697; N = 10,
-// 100 walkers 324 / 574; N = 16, 400 walkers 787 / 827; N = 20 UHF, 100 walkers
-// 704 / 900, 384 walkers 1503 / 1496; N = 24, 64 walkers 563 / 619, 300 walkers
-// 1123 / 902; N = 32, 100 walkers 720 / 683.  So up to 20 orbitals, and to 24
-// while the walkers are one wave.
+// Where this kernel is the faster one.  Per walker it takes
+//   5.1e-4 G N (N + 1.7 No) + No (4e-3 N No + 2) - 19 ns  (No: a sum over spins; 19 per spin)
+// more than the tensor-core launches, a fit to both at N = 4 to 24, No = 1 to N, G = 2 N to 16 N and
+// 20 to 10000 walkers (recorded steps); the launches cost some 18 us more whatever the
+// walkers, and below one walker per SM a walker's own time counts.  With this rule no size of
+// that range is slower than the launches it replaced, and the sizes together are within
+// 0.5 % of always taking the faster one.  Recorded steps, us, this kernel / the launches: N = 6, No = 1,
+// G = 12, 296 walkers 19 / 52, 10000 345 / 620; N = 20, No = 10, G = 160, 296 walkers 55 / 71, 10000
+// 1.47 times the launches; N = 16, No = 16, G = 256, 4000 walkers 945 / 449; N = 24, No = 24,
+// G = 384, 20 walkers 153 / 76.  (All of N <= 20 took this kernel before: N = 16, No = 16, G = 256,
+// 4000 walkers 945 us, 513 before it existed.)
 bool small_step_fits(const Layout& L) {
-  if (L.mixed || L.N > 24 || (L.N > 20 && L.W > 148)) return false;
+  if (L.mixed || L.N > 24) return false;
+  double ns = 0.0;
+  int no = 0;
+  for (int s = 0; s < L.ns; ++s) {
+    no += L.no[s];
+    ns += L.no[s] * (4e-3 * L.N * L.no[s] + 2.0) - 19.0;
+  }
+  ns += 5.1e-4 * L.G * L.N * (L.N + 1.7 * no);
+  const int w = L.W > sm_count() ? L.W : sm_count();
+  if (ns * w >= 18000.0) return false;
   return small_smem(L.N, L.G, L.no[0], L.no[1], L.ns).total * sizeof(double) <= 200 * 1024;
 }
 
