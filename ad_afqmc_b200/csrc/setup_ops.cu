@@ -837,7 +837,7 @@ int afq_natural_orbitals(int32_t n, int32_t k, const double* rdm, double* orbs, 
   int rc = afq_natural_orbitals_workspace_size(n, k, &need);
   if (rc != AFQ_OK) return rc;
   if (work_bytes < need) return AFQ_ERR_WORKSPACE;
-  if (!al16(work) || !al16(rdm)) return AFQ_ERR_ALIGN;
+  if (!al16(work) || (!(n & 1) && !al16(rdm))) return AFQ_ERR_ALIGN;  // odd n: read as a padded copy
   cudaStream_t st = as_stream(stream);
   const long long ld = even(n);
   const int p = std::min(n, k + 8);

@@ -401,7 +401,8 @@ int afq_eigh_desc(int32_t n, const double* A, double* evals, double* evecs, void
  * on the projected matrix) until every Ritz residual is below 1e-13 of the
  * spectral radius (one iteration for a projector density); when that does not
  * happen within 40 iterations (occupations too close at the cut) the full
- * afq_eigh_desc.  Synchronizes `stream` once per iteration.  k <= 64.
+ * afq_eigh_desc.  Synchronizes `stream` once per iteration.  k <= 64.  rdm is
+ * 16-byte aligned for even n (a spin's slice of an odd (2, n, n) tensor is not).
  * work: afq_natural_orbitals_workspace_size() bytes. */
 int afq_natural_orbitals_workspace_size(int32_t n, int32_t k, size_t* bytes);
 int afq_natural_orbitals(int32_t n, int32_t k, const double* rdm, double* orbs, double* occ, void* work,
