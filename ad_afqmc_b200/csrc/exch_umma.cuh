@@ -569,6 +569,14 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint4& a, const u
                : "memory");
 }
 
+// the first n of eight bf16 values, zeros in place of the others
+__device__ __forceinline__ uint4 bf16_first(uint4 v, int n) {
+  auto word = [n](uint32_t u, int i) {  // values 2 i (low half) and 2 i + 1
+    return n >= 2 * i + 2 ? u : (n == 2 * i + 1 ? u & 0xffffu : 0u);
+  };
+  return make_uint4(word(v.x, 0), word(v.y, 1), word(v.z, 2), word(v.w, 3));
+}
+
 // Row operand in TMEM, two-piece operands.  The CTA walks a contiguous range of
 // tiles, so its rot_chol rows change a few times in all; four epilogue warps
 // write new ones to TMEM when they meet the first tile that needs them.  MMA
@@ -728,7 +736,11 @@ __global__ void __launch_bounds__(kExchThreads, 1)
             const int steps = pc == 0 ? KS : min(KS, lot * 4);
             const uint32_t col = lane_t + kACol + (pc ? 8 * KS : 0);
             for (int k = 0; k < steps; ++k) {
-              const uint4 x = in ? src[2 * k] : zero, y = in ? src[2 * k + 1] : zero;
+              uint4 x = in ? src[2 * k] : zero, y = in ? src[2 * k + 1] : zero;
+              if (16 * (k + 1) > P.K) {  // beyond K: whatever the rows' padding holds
+                x = bf16_first(x, P.K - 16 * k);
+                y = bf16_first(y, P.K - 16 * k - 8);
+              }
               __syncwarp();
               tmem_st8(col + 8 * k, x, y);
             }
