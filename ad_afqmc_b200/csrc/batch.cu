@@ -147,7 +147,7 @@ int afq_batch_create(int32_t n, const afq_dims* dims, const void* const* prepare
     p.sdt = sqrt(dims[f].dt);
     p.fields = fields[f];
     p.mf = P[f] + l.p_mf;
-    p.xt = Wk[f] + l.w_xt;
+    p.xt = nullptr;  // mixed: the bf16 pieces
     p.wscal = Wk[f] + l.w_wscal;
     piece_ptrs(Wk[f], l.v_xt, l.v_xt_ps, l.npc, p.xb);
     prep[f] = p;

@@ -681,7 +681,7 @@ cudaError_t launch_prep(const Layout& L, const double* prep, double* work, const
   if (L.mixed) piece_ptrs(work, L.v_xt, L.v_xt_ps, L.npc, xb);
   prep_kernel<<<L.W, 256, 0, st>>>(L.W, L.G, L.Gpad, L.splitk, work + L.w_fbpart, L.mixed ? 1 : 0,
                                    (double)L.mult, fields, prep + L.p_mf, sqrt(dt),
-                                   work + L.w_xt, work + L.w_wscal, fb_out, L.npc, xb[0], xb[1],
+                                   L.mixed ? nullptr : work + L.w_xt, work + L.w_wscal, fb_out, L.npc, xb[0], xb[1],
                                    xb[2], L.Gb);
   return cudaGetLastError();
 }
@@ -710,7 +710,7 @@ cudaError_t launch_free_fields(const Layout& L, double* work, const double* fiel
   ProfScope ps(K_PREP, st);
   bf16* xb[3] = {nullptr, nullptr, nullptr};
   if (L.mixed) piece_ptrs(work, L.v_xt, L.v_xt_ps, L.npc, xb);
-  free_fields_kernel<<<L.W, 256, 0, st>>>(L.G, L.Gpad, fields, sqrt(dt), work + L.w_xt, L.npc, xb[0],
+  free_fields_kernel<<<L.W, 256, 0, st>>>(L.G, L.Gpad, fields, sqrt(dt), L.mixed ? nullptr : work + L.w_xt, L.npc, xb[0],
                                           xb[1], xb[2], L.Gb);
   return cudaGetLastError();
 }

@@ -108,8 +108,8 @@ struct Layout {
   // prepared buffer offsets (doubles)
   long long p_mo[2], p_rh1[2], p_rc[2], p_rccat, p_chol, p_exph1[2], p_mf, p_scal, prepared;
   // workspace offsets (doubles)
-  long long w_gpl, w_theta[2], w_fbpart, w_xt, w_wscal, w_vhs, w_y, w_acc, w_ta, w_tb;
-  long long w_c[2], w_exc[2], w_orb, w_s, w_cum, w_idx, w_misc, work;
+  long long w_gpl, w_theta[2], w_fbpart, w_xt, w_wscal, w_vhs, w_y, w_ta, w_tb;  // FP64 path only: all but w_theta, w_fbpart, w_wscal
+  long long w_c[2], w_exc[2], w_orb, w_s, w_misc, work;
 };
 
 // f64_exch_bn once chose among three column tiles; records that name one are taken as before (a
@@ -258,21 +258,24 @@ inline int make_layout(const afq_dims* d, Layout& L, const afq_tuning* record = 
   // ---- workspace
   o = 0;
   const long long W = L.W, N = L.N;
-  L.w_gpl = take(W * 2 * L.Kfb);
+  take(2 * W);  // launch_qr's norms, at the start of whatever scratch it is given
+  L.w_gpl = L.w_xt = L.w_vhs = L.w_y = L.w_ta = L.w_tb = -1;
   for (int s = 0; s < 2; ++s) L.w_theta[s] = -1;
-  for (int s = 0; s < L.ns; ++s) L.w_theta[s] = take(W * 2 * L.no[s] * L.Npad);
-  L.w_xt = take(2 * W * L.Gpad);
+  // Theta of the FP64 exchange and of the orbital energy (restricted walkers)
+  for (int s = 0; s < L.ns; ++s)
+    if (L.exch_f64[s] || L.restricted) L.w_theta[s] = take(W * 2 * L.no[s] * L.Npad);
   L.w_wscal = take(W * 16);
-  L.w_vhs = take(W * N * 2 * L.Npad);
-  const long long pb = W * N * 2 * L.nomax;  // (fp64 path) y / acc / t buffers
-  L.w_y = take(pb);
-  L.w_acc = take(pb);
-  L.w_ta = take(pb);
-  L.w_tb = take(pb);
+  if (!L.mixed) {
+    L.w_gpl = take(W * 2 * L.Kfb);
+    L.w_xt = take(2 * W * L.Gpad);
+    L.w_vhs = take(W * N * 2 * L.Npad);
+    const long long pb = W * N * 2 * L.nomax;
+    L.w_y = take(pb);
+    L.w_ta = take(pb);
+    L.w_tb = take(pb);
+  }
   for (int s = 0; s < 2; ++s) L.w_c[s] = L.w_exc[s] = -1;
   for (int s = 0; s < L.ns; ++s) L.w_c[s] = take(W * L.G * 2);
-  L.w_cum = take(W);
-  L.w_idx = take(W);  // int32 indices stored in double slots
   L.w_misc = take(64);
   for (int s = 0; s < 2; ++s) L.v_gt[s] = -1;
   if (L.mixed) {
