@@ -4,7 +4,7 @@
 //
 // The tile is 128 rows (gpt Cholesky vectors of No rows) by BN columns (wpt
 // walkers of 2 No columns).  Roles as in umma_gemm.cuh: a TMA producer warp, an
-// MMA warp, one epilogue warpgroup behind two TMEM buffers.  What sets it
+// MMA warp, eight epilogue warps behind one or two TMEM buffers and four reducing warps.  What sets it
 // apart from the general GEMM:
 //  * The shared-memory port (128 bytes per cycle) is what bounds it: an MMA of
 //    128 x N x 16 reads 4096 + 32 N bytes of it, TMA writes the operands through it
@@ -19,7 +19,7 @@
 //  * Boxes hold the rows in use (gpt No, wpt 2 No), not the MMA's 128 x BN:
 //    the MMA reads on into whatever follows, and those rows and columns of the
 //    accumulator are never looked at.
-//  * Eight epilogue warps share a tile (see exch_tile).
+//  * Eight epilogue warps share a tile (see exch_tile); its sums end in FP64 (exch_finish).
 // Measured on a B200, two pieces, per launch: N = 200, No = 40, G = 1000, W = 512
 // 4.74 -> 2.43 ms; N = 300, No = 60, G = 1500, W = 1024 29.7 -> 22.8 ms; N = 250,
 // No = 62, G = 1250, W = 256 4.98 -> 3.47 ms.
@@ -537,7 +537,7 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t dtmem, uint32_t atmem, uin
       "{\n .reg .pred p;\n .reg .b64 db;\n setp.ne.b32 p, %4, 0;\n"
       " mov.b64 db, {%2, %5};\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n}" ::"r"(dtmem),
-      "r"(atmem), "r"(blo), "r"(idesc), "r"(accumulate), "r"(0x40004040u)
+      "r"(atmem), "r"(blo), "r"(idesc), "r"(accumulate), "r"(kDescHi)
       : "memory");
 }
 

@@ -1,20 +1,15 @@
-// FP64 tensor-core (DMMA m8n8k4) tile GEMM core for the walker path.
+// FP64 tensor-core (DMMA m8n8k4) tile GEMM core of the set-up.
 //
-// Every FP64 contraction of the step (force bias, VHS build, one-body
-// half-steps, Taylor chain, exchange energy) is one instantiation of this
-// CTA-level main loop with its own epilogue.  Operands stream through a
-// multistage cp.async pipeline into padded shared-memory tiles whose row
-// strides (== 4 mod 16 doubles) make every fragment read conflict-free.
+// The set-up's contractions (rot_h1, rot_chol, v0, the matrix exponential, the natural
+// orbitals) are instantiations of this CTA-level main loop; the walker path's FP64
+// contractions run in f64_tma.cuh.  Operands stream through a multistage cp.async
+// pipeline into padded shared-memory tiles whose row strides (== 4 mod 16 doubles) make
+// every fragment read conflict-free.
 //
 // Operand addressing (element (k, n) of B, (m, k) of A):
-//   A          : ptr + b*bstride + m*ld + k                  (k contiguous)
-//   B, KMAJOR  : ptr + b*bstride + k*ld + col(n)             (n contiguous)
-//   B, NMAJOR  : ptr + b*bstride + col(n)*ld + k             (k contiguous)
-//   col(n)     = (n / seg) * segstride + n % seg             (walker batches
-//                laid side by side along n; seg = 1<<30 means plain)
-// `rot` applies x -> i*x to interleaved complex columns of B on the fly:
-//   B'[k][2j] = -B[k][2j+1], B'[k][2j+1] = B[k][2j]
-// which turns a complex x complex product into one real GEMM with K doubled.
+//   A          : ptr + b*bstride + m*ld + k          (k contiguous)
+//   B, KMAJOR  : ptr + b*bstride + k*ld + n          (n contiguous)
+//   B, NMAJOR  : ptr + b*bstride + n*ld + k          (k contiguous)
 #pragma once
 
 #include "common.cuh"
@@ -42,8 +37,6 @@ struct F64Operand {
   const double* ptr;
   long long ld;
   long long bstride;
-  long long segstride;  // only B: stride between column segments
-  int seg;              // only B: columns per segment (1<<30 = unsegmented)
 };
 
 enum { B_KMAJOR = 0, B_NMAJOR = 1 };
@@ -54,8 +47,7 @@ template <class Cfg, int BMODE>
 __device__ __forceinline__ void f64_mainloop(double (&acc)[Cfg::FM][Cfg::FN][2],
                                              const F64Operand& A, const F64Operand& B,
                                              int M_lim, int N_lim, int k_begin, int k_end,
-                                             int m0, int n0, int batch, bool rot,
-                                             double* smem) {
+                                             int m0, int n0, int batch, double* smem) {
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, NT = Cfg::NT, ST = Cfg::STAGES;
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
@@ -93,8 +85,7 @@ __device__ __forceinline__ void f64_mainloop(double (&acc)[Cfg::FM][Cfg::FN][2],
         const double* src = Bb;
         if (gk < k_end && gn < N_lim) {
           bytes = (gn + 1 < N_lim) ? 16 : 8;
-          const long long col = (long long)(gn / B.seg) * B.segstride + (gn % B.seg);
-          src = Bb + (long long)gk * B.ld + col;
+          src = Bb + (long long)gk * B.ld + gn;
         }
         cp_async16(Bs + r * Cfg::BSN + nc, src, bytes);
       }
@@ -113,9 +104,6 @@ __device__ __forceinline__ void f64_mainloop(double (&acc)[Cfg::FM][Cfg::FN][2],
       }
     }
   };
-
-  const double sgn = rot ? ((g & 1) ? 1.0 : -1.0) : 1.0;
-  const int cx = rot ? 1 : 0;
 
 #pragma unroll 1
   for (int s = 0; s < ST - 1; ++s) {
@@ -142,7 +130,7 @@ __device__ __forceinline__ void f64_mainloop(double (&acc)[Cfg::FM][Cfg::FN][2],
       for (int j = 0; j < Cfg::FN; ++j) {
         const int col = wn * Cfg::TN + j * 8 + g;
         if (BMODE == B_KMAJOR)
-          b[j] = sgn * Bs[(kk * 4 + t) * Cfg::BSN + (col ^ cx)];
+          b[j] = Bs[(kk * 4 + t) * Cfg::BSN + col];
         else
           b[j] = Bs[col * Cfg::BSK + kk * 4 + t];
       }

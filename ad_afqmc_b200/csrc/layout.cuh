@@ -6,6 +6,8 @@
 
 #include <stddef.h>
 
+#include <initializer_list>
+
 #include "afqmc_b200.h"
 
 namespace afq {
@@ -26,61 +28,41 @@ struct ExchTile {
   int mt;   // number of blocks = ceil(G / gpt)
 };
 
-// Shared memory of the tensor-core exchange epilogue: the f block as
-// (re, im) float pairs with an odd row stride in pairs, per-row partials
-// (double4) and per-Cholesky-vector sums (double2) for 128 rows.
-__host__ __device__ inline int exch_fs2(int no) { return (no + 1) | 1; }
-__host__ __device__ inline long long exch_fs_bytes(int no) {
-  return (128LL * exch_fs2(no) * 8 + 31) & ~31LL;
-}
-__host__ __device__ inline long long exch_epi_extra(int no) {
-  return exch_fs_bytes(no) + 128 * 32 + 128 * 16;
-}
-
 // Exchange tile of the tensor-core path: 128 rows hold gpt Cholesky
 // vectors, BN columns hold wpt walkers.
 struct UExchTile {
   int bn, gpt, wpt, mt;
 };
 
-// Column tile of the exchange (two accumulator groups, double buffered:
-// BN <= 128) holding whole walkers with the least padding, with room for two
-// pipeline stages plus the epilogue's staging of one walker's f block.
-inline UExchTile choose_uexch_tile(int no, int G, int npc) {
-  UExchTile t;
-  const int bns[5] = {128, 96, 80, 64, 32};
-  const long long budget = 227 * 1024 - 1024 - 256;
-  const long long extra = exch_epi_extra(no);
-  t.bn = 0;
-  double best = -1.0;
-  for (int i = 0; i < 5; ++i) {
-    const int bn = bns[i];
-    if (((2 * no + 15) & ~15) > bn) continue;
-    const long long stage = (long long)npc * (128 * 128 + bn * 128);
-    if (2 * stage + extra > budget) continue;
-    const int wpt = bn / (2 * no);
-    const double eff = double(wpt * 2 * no) / bn;
-    if (eff > best + 1e-9) { best = eff; t.bn = bn; }
-  }
-  t.gpt = 128 / no;
-  t.wpt = t.bn ? t.bn / (2 * no) : 0;
-  t.mt = (G + t.gpt - 1) / t.gpt;
-  return t;
-}
-
-// The exchange tile of one column width, or bn = 0 when it cannot hold a
-// walker or does not fit shared memory (same rules as choose_uexch_tile).
+// The exchange tile of one column width, or bn = 0 when it is not used.  It holds a walker
+// padded to 16 columns; three-piece operands take 128 columns up to No = 26 only, so
+// that from No = 49 on such a spin's exchange runs on the FP64 kernel: the line was drawn
+// by shared memory once (the plan of exch_umma.cuh would admit a few more) and is kept,
+// since FP64 is the more precise.
 inline UExchTile uexch_tile_for(int no, int G, int npc, int bn) {
   UExchTile t{0, 128 / no, 0, 0};
-  const long long budget = 227 * 1024 - 1024 - 256;
-  const long long extra = exch_epi_extra(no);
-  const long long stage = (long long)npc * (128 * 128 + bn * 128);
-  if (((2 * no + 15) & ~15) <= bn && 2 * stage + extra <= budget) {
+  if (((2 * no + 15) & ~15) <= bn && !(npc == 3 && bn == 128 && no > 26)) {
     t.bn = bn;
     t.wpt = bn / (2 * no);
   }
   t.mt = (G + t.gpt - 1) / t.gpt;
   return t;
+}
+
+// The width that holds whole walkers with the least padding (two accumulator groups, double
+// buffered: BN <= 128).
+inline UExchTile choose_uexch_tile(int no, int G, int npc) {
+  UExchTile best = uexch_tile_for(no, G, npc, 0);
+  double eff = -1.0;
+  for (int bn : {128, 96, 80, 64, 32}) {
+    const UExchTile t = uexch_tile_for(no, G, npc, bn);
+    const double e = double(t.wpt * 2 * no) / bn;
+    if (t.bn && e > eff + 1e-9) {
+      eff = e;
+      best = t;
+    }
+  }
+  return best;
 }
 
 // Row strides of the bf16 operands: whole 128-byte lines (64 elements).  A TMA

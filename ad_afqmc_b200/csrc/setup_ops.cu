@@ -10,7 +10,7 @@
 //                (wave_function.get_init_walkers, wavefunctions.py:427-466)
 //
 // The contractions run on the FP64 tensor cores through the same DMMA main
-// loop as the walker kernels (gemm_f64.cuh), which copies 16-byte pieces:
+// loop (gemm_f64.cuh), which copies 16-byte pieces:
 // every operand it reads has an even leading dimension (odd N: the Cholesky
 // vectors and square matrices are first copied to padded rows).  v0 is a split-K GEMM over the
 // Cholesky index with partial sums added in a fixed order, so results do not
@@ -38,7 +38,6 @@
 namespace afq {
 namespace {
 
-constexpr int kUnsegS = 1 << 30;
 using CfgS = F64Cfg<2, 4, 4, 2>;    // 64 x 64, 8 warps: rot_chol, rot_h1, expm
 using CfgV0 = F64Cfg<4, 8, 4, 2>;   // 128 x 128, 8 warps: v0
 
@@ -71,7 +70,7 @@ __global__ void __launch_bounds__(Cfg::NT) dgemm_kernel(DgemmArgs a) {
     b1 = min(a.nbatch, b0 + a.bsum);
   }
   for (int b = b0; b < b1; ++b)
-    f64_mainloop<Cfg, BMODE>(acc, a.A, a.B, a.M, a.N, 0, a.K, m0, n0, b, false, smem);
+    f64_mainloop<Cfg, BMODE>(acc, a.A, a.B, a.M, a.N, 0, a.K, m0, n0, b, smem);
   double* Cz = a.C + (long long)z * a.c_bs;
   const double* Iz = a.cin ? a.cin + (long long)z * a.cin_bs : nullptr;
   f64_foreach<Cfg>(acc, m0, n0, [&](int m, int n, double v0, double v1) {
@@ -106,8 +105,8 @@ template <int BMODE>
 cudaError_t gemm2(int M, int N, int K, const double* A, long long lda, const double* B, long long ldb,
                   double alpha, double* C, long long ldc, cudaStream_t st) {
   DgemmArgs a{};
-  a.A = F64Operand{A, lda, 0, 0, kUnsegS};
-  a.B = F64Operand{B, ldb, 0, 0, kUnsegS};
+  a.A = F64Operand{A, lda, 0};
+  a.B = F64Operand{B, ldb, 0};
   a.M = M;
   a.N = N;
   a.K = K;
@@ -123,8 +122,8 @@ cudaError_t gemm2(int M, int N, int K, const double* A, long long lda, const dou
 cudaError_t square_gemm(int n, long long ld, const double* A, const double* B, double alpha,
                         double diag, double* C, cudaStream_t st) {
   DgemmArgs a{};
-  a.A = F64Operand{A, ld, 0, 0, kUnsegS};
-  a.B = F64Operand{B, ld, 0, 0, kUnsegS};
+  a.A = F64Operand{A, ld, 0};
+  a.B = F64Operand{B, ld, 0};
   a.M = a.N = a.K = n;
   a.nbatch = 1;
   a.alpha = alpha;
@@ -657,8 +656,8 @@ int afq_measurement_intermediates(int32_t norb, const int32_t nocc[2], int32_t n
     }
     // rot_h1[s] = mo^T h (no x n)
     DgemmArgs a{};
-    a.A = F64Operand{mt, ld, 0, 0, kUnsegS};
-    a.B = F64Operand{hrot + s * hs, ld, 0, 0, kUnsegS};
+    a.A = F64Operand{mt, ld, 0};
+    a.B = F64Operand{hrot + s * hs, ld, 0};
     a.M = no;
     a.N = n;
     a.K = n;
@@ -669,8 +668,8 @@ int afq_measurement_intermediates(int32_t norb, const int32_t nocc[2], int32_t n
     if (dgemm<CfgS>(a, 1, st) != cudaSuccess) return AFQ_ERR_CUDA;
     // rot_chol[s][g] = mo^T L_g (no x n), batched over g
     DgemmArgs b{};
-    b.A = F64Operand{mt, ld, 0, 0, kUnsegS};
-    b.B = F64Operand{B, ld, (long long)n * ld, 0, kUnsegS};
+    b.A = F64Operand{mt, ld, 0};
+    b.B = F64Operand{B, ld, (long long)n * ld};
     b.M = no;
     b.N = n;
     b.K = n;
@@ -790,8 +789,8 @@ int afq_propagation_intermediates(int32_t norb, int32_t nchol, int32_t walker_ty
   // v0 partials: part[z] = sum_{g in z} L_g L_g
   {
     DgemmArgs a{};
-    a.A = F64Operand{Bc, ld, (long long)n * ld, 0, kUnsegS};
-    a.B = F64Operand{Bc, ld, (long long)n * ld, 0, kUnsegS};
+    a.A = F64Operand{Bc, ld, (long long)n * ld};
+    a.B = F64Operand{Bc, ld, (long long)n * ld};
     a.M = a.N = a.K = n;
     a.nbatch = G;
     a.bsum = bsum;

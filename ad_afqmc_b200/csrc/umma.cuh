@@ -272,19 +272,6 @@ __device__ __forceinline__ void acc_ld16(uint32_t taddr, int ngroups, int bn, fl
 // ---------------------------------------------------------------------------
 // tcgen05.mma (single CTA, A and B from shared memory)
 // ---------------------------------------------------------------------------
-// Shared-memory matrix descriptor, K-major operand in the 128-byte swizzle
-// layout written by TMA (rows of 128 bytes, 8-row atoms of 1024 bytes).
-__device__ __forceinline__ uint64_t smem_desc_sw128(const void* base) {
-  const uint64_t addr = su32(base);
-  uint64_t d = 0;
-  d |= (addr >> 4) & 0x3FFFull;            // start address
-  d |= (uint64_t)(16 >> 4) << 16;          // leading byte offset (unused for SW128 K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;        // stride byte offset: 8 rows x 128 B
-  d |= (uint64_t)1 << 46;                  // descriptor version (sm100)
-  d |= (uint64_t)2 << 61;                  // layout: SWIZZLE_128B
-  return d;
-}
-
 // Instruction descriptor: dense, FP32 accumulate, A/B K-major.
 // fmt: 1 = BF16 (kind::f16), 2 = TF32 (kind::tf32)
 __host__ __device__ constexpr uint32_t instr_desc(int M, int N, int fmt) {
@@ -295,19 +282,13 @@ __host__ __device__ constexpr uint32_t instr_desc(int M, int N, int fmt) {
          | ((uint32_t)(M >> 4) << 24);  // M
 }
 
-__device__ __forceinline__ void umma_bf16(uint32_t dtmem, uint64_t adesc, uint64_t bdesc,
-                                          uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(dtmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// The low words of two such descriptors (the high word is the same for every
-// K-major SW128 operand): 32-bit address arithmetic per MMA, which issues one
-// MMA every ~50 cycles where 64-bit descriptors built from operand pointers
-// took 66-80.
+// Shared-memory matrix descriptor, K-major operand in the 128-byte swizzle layout written
+// by TMA (rows of 128 bytes, 8-row atoms of 1024 bytes): low word the start address and the
+// leading byte offset (unused, 1), both in 16 bytes; high word, the same for every operand,
+// the stride byte offset 1024 / 16, the version (bit 14) and SWIZZLE_128B (2 << 29).
+// 32-bit address arithmetic per MMA, which issues one MMA every ~50 cycles where
+// 64-bit descriptors built from operand pointers took 66-80.
+constexpr uint32_t kDescHi = (1024 >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t smem_desc_lo(uint32_t saddr) { return (saddr >> 4) | (1u << 16); }
 __device__ __forceinline__ void umma_bf16_lo(uint32_t dtmem, uint32_t alo, uint32_t blo,
                                              uint32_t idesc, uint32_t accumulate) {
@@ -315,7 +296,7 @@ __device__ __forceinline__ void umma_bf16_lo(uint32_t dtmem, uint32_t alo, uint3
       "{\n .reg .pred p;\n .reg .b64 da, db;\n setp.ne.b32 p, %4, 0;\n"
       " mov.b64 da, {%1, %5};\n mov.b64 db, {%2, %5};\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n}" ::"r"(dtmem),
-      "r"(alo), "r"(blo), "r"(idesc), "r"(accumulate), "r"(0x40004040u)
+      "r"(alo), "r"(blo), "r"(idesc), "r"(accumulate), "r"(kDescHi)
       : "memory");
 }
 
