@@ -6,8 +6,6 @@
 
 #include <stddef.h>
 
-#include <initializer_list>
-
 #include "afqmc_b200.h"
 
 namespace afq {
@@ -34,6 +32,9 @@ struct UExchTile {
   int bn, gpt, wpt, mt;
 };
 
+// Column widths the tensor-core exchange is compiled for.
+constexpr int kUExchWidths[5] = {128, 96, 80, 64, 32};
+
 // The exchange tile of one column width, or bn = 0 when it is not used.  It holds a walker
 // padded to 16 columns; three-piece operands take 128 columns up to No = 26 only, so
 // that from No = 49 on such a spin's exchange runs on the FP64 kernel: the line was drawn
@@ -41,11 +42,12 @@ struct UExchTile {
 // since FP64 is the more precise.
 inline UExchTile uexch_tile_for(int no, int G, int npc, int bn) {
   UExchTile t{0, 128 / no, 0, 0};
-  if (((2 * no + 15) & ~15) <= bn && !(npc == 3 && bn == 128 && no > 26)) {
-    t.bn = bn;
-    t.wpt = bn / (2 * no);
-  }
   t.mt = (G + t.gpt - 1) / t.gpt;
+  for (int w : kUExchWidths)
+    if (bn == w && ((2 * no + 15) & ~15) <= bn && !(npc == 3 && bn == 128 && no > 26)) {
+      t.bn = bn;
+      t.wpt = bn / (2 * no);
+    }
   return t;
 }
 
@@ -54,7 +56,7 @@ inline UExchTile uexch_tile_for(int no, int G, int npc, int bn) {
 inline UExchTile choose_uexch_tile(int no, int G, int npc) {
   UExchTile best = uexch_tile_for(no, G, npc, 0);
   double eff = -1.0;
-  for (int bn : {128, 96, 80, 64, 32}) {
+  for (int bn : kUExchWidths) {
     const UExchTile t = uexch_tile_for(no, G, npc, bn);
     const double e = double(t.wpt * 2 * no) / bn;
     if (t.bn && e > eff + 1e-9) {
