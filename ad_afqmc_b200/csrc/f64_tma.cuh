@@ -282,16 +282,17 @@ int make_tmap_f64(CUtensorMap* map, const void* base, long long x, long long y, 
 
 constexpr size_t kF64SmemBudget = 227 * 1024;
 
+// stages of a launch of `per` CTAs an SM
 template <class T>
-inline int f64_stages(size_t epi_bytes) {
+inline int f64_stages(size_t epi_bytes, int per = 1) {
   for (int st = 6; st >= 2; --st)
-    if (1024 + st * size_t(T::STAGE) + 256 + epi_bytes <= kF64SmemBudget) return st;
+    if (1024 + st * size_t(T::STAGE) + 256 + epi_bytes <= kF64SmemBudget / per) return st;
   return 0;
 }
 
 template <class T, class Epi>
 cudaError_t f64_launch(F64Params<Epi>& P, int ctas, cudaStream_t st) {
-  P.s.stages = f64_stages<T>(P.s.epi_bytes);
+  if (P.s.stages == 0) P.s.stages = f64_stages<T>(P.s.epi_bytes);
   if (P.s.stages < 2) return cudaErrorInvalidValue;
   const size_t smem = 1024 + P.s.stages * size_t(T::STAGE) + 256 + P.s.epi_bytes;
   cudaError_t e = cudaFuncSetAttribute(f64_gemm_kernel<T, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize,

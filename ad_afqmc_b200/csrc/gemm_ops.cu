@@ -536,7 +536,13 @@ cudaError_t prop_run(const Layout& L, double* work, int nc, const PropCall& c, c
   P.s.a_batched = c.abs != 0;
   P.s.err = f64_err(L, work);
   P.epi = PropEpi{c.out, c.yin, c.scale, N, nc};
-  const size_t smem = 1024 + f64_stages<T>(0) * size_t(T::STAGE) + 256;
+  // few warps: two or three CTAs an SM if each keeps three stages, so that one's
+  // loads and stores run under another's MMAs (N = 34, No = 12, 10000 walkers, seven launches:
+  // 1.56 ms with six stages and one CTA, 1.24 so; 1.26 with the cp.async kernel before)
+  int per = T::CW <= 4 ? 3 : (T::CW <= 8 ? 2 : 1);
+  while (per > 1 && f64_stages<T>(0, per) < 3) --per;
+  P.s.stages = f64_stages<T>(0, per);
+  const size_t smem = 1024 + P.s.stages * size_t(T::STAGE) + 256;
   ProfScope ps(K_PROP, st);
   return f64_launch<T>(P, f64_ctas(T::NT, smem), st);
 }
