@@ -12,6 +12,13 @@ namespace afq {
 constexpr int kMaxNocc = 64;     // largest occupied block a walker kernel accepts
 constexpr int kMaxWalkers = 1 << 16;
 
+// raises the dynamic shared memory `kernel` may be launched with to `bytes` (smem.cu)
+cudaError_t allow_smem(const void* kernel, size_t bytes);
+template <class K>
+inline cudaError_t allow_smem(K* kernel, size_t bytes) {
+  return allow_smem(reinterpret_cast<const void*>(kernel), bytes);
+}
+
 // ---------------------------------------------------------------------------
 // small complex helpers (interleaved re, im as double2)
 // ---------------------------------------------------------------------------

@@ -295,8 +295,7 @@ cudaError_t f64_launch(F64Params<Epi>& P, int ctas, cudaStream_t st) {
   if (P.s.stages == 0) P.s.stages = f64_stages<T>(P.s.epi_bytes);
   if (P.s.stages < 2) return cudaErrorInvalidValue;
   const size_t smem = 1024 + P.s.stages * size_t(T::STAGE) + 256 + P.s.epi_bytes;
-  cudaError_t e = cudaFuncSetAttribute(f64_gemm_kernel<T, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
+  cudaError_t e = allow_smem(f64_gemm_kernel<T, Epi>, smem);
   if (e != cudaSuccess) return e;
   const long long tiles = (long long)P.s.mt * P.s.nt * P.s.nz;
   if (tiles >= (1LL << 31)) return cudaErrorInvalidValue;

@@ -579,7 +579,7 @@ cudaError_t launch_green_grouped(const GreenArgs* args, const BlockMap& m, int m
   const int threads = green_threads(nomax);
   const size_t smem = green_smem_bytes(nomax);
   return with_green_kernel(threads, [&](auto, auto kernel) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kernel, smem);
     if (e != cudaSuccess) return e;
     kernel<<<m.start[m.n], threads, smem, st>>>(args, m, mode);
     return cudaGetLastError();
@@ -587,8 +587,7 @@ cudaError_t launch_green_grouped(const GreenArgs* args, const BlockMap& m, int m
 }
 
 cudaError_t launch_gj_grouped(const GjArgs* args, const BlockMap& m, size_t smem, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(gj_kernel_grouped, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
+  cudaError_t e = allow_smem(gj_kernel_grouped, smem);
   if (e != cudaSuccess) return e;
   ProfScope ps(K_GREEN, st);
   gj_kernel_grouped<<<m.start[m.n], kGjThreads, smem, st>>>(args, m);
@@ -612,7 +611,7 @@ cudaError_t launch_green(const GreenArgs& a, cudaStream_t st) {
   for (int s = 0; s < a.ns; ++s)
     need_theta = need_theta || a.sec[s].theta || a.sec[s].gout || a.sec[s].rh1 || a.sec[s].gtb[0];
   return with_green_kernel(threads, [&](auto kernel, auto) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kernel, smem);
     if (e != cudaSuccess) return e;
     if (!a.sbuf || !need_theta) {  // one kernel: S, its inverse and det, Theta and outputs
       kernel<<<grid, threads, smem, st>>>(a, 0);
@@ -623,9 +622,7 @@ cudaError_t launch_green(const GreenArgs& a, cudaStream_t st) {
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     const int bstride = nomax * (nomax | 1);
     const size_t gsmem = gj_smem_bytes(nomax);
-    if ((e = cudaFuncSetAttribute(gj_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsmem)) !=
-        cudaSuccess)
-      return e;
+    if ((e = allow_smem(gj_kernel, gsmem)) != cudaSuccess) return e;
     gj_kernel<<<grid, kGjThreads, gsmem, st>>>(a.W, a.sec[0].no, a.ns > 1 ? a.sec[1].no : 0, a.sbuf,
                                                a.sstride, bstride, a.wscal);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;

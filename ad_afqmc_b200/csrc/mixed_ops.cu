@@ -423,8 +423,7 @@ int prop_launch(const Layout& L, const double* prep, double* work, int s, int nc
 
 template <class Kernel>
 int exch_run(Kernel kernel, int threads, const ExchParams& P, size_t smem, int ctas, cudaStream_t st) {
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return AFQ_ERR_CUDA;
+  if (allow_smem(kernel, smem) != cudaSuccess) return AFQ_ERR_CUDA;
   const long long tiles = (long long)P.mt * P.nt;
   ProfScope ps(K_EXCH, st);
   kernel<<<(int)(tiles < ctas ? tiles : ctas), threads, smem, st>>>(P);

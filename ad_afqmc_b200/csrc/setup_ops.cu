@@ -91,8 +91,7 @@ __global__ void __launch_bounds__(Cfg::NT) dgemm_kernel(DgemmArgs a) {
 // B_KMAJOR: B element (k, n) at ptr + k ld + n;  B_NMAJOR: at ptr + n ld + k
 template <class Cfg, int BMODE = B_KMAJOR>
 cudaError_t dgemm(const DgemmArgs& a, int zdim, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(dgemm_kernel<Cfg, BMODE>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM);
+  cudaError_t e = allow_smem(dgemm_kernel<Cfg, BMODE>, Cfg::SMEM);
   if (e != cudaSuccess) return e;
   dim3 grid((a.M + Cfg::BM - 1) / Cfg::BM, (a.N + Cfg::BN - 1) / Cfg::BN, zdim);
   ProfScope ps(K_MISC, st);
@@ -885,9 +884,7 @@ int afq_natural_orbitals(int32_t n, int32_t k, const double* rdm, double* orbs, 
     bool packed = false;
     const size_t smem = jacobi_smem(p, &packed);
     if (!packed) return AFQ_ERR_SHAPE;
-    if (cudaFuncSetAttribute(jacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-      return AFQ_ERR_CUDA;
+    if (allow_smem(jacobi_kernel, smem) != cudaSuccess) return AFQ_ERR_CUDA;
     {
       ProfScope ps(K_MISC, st);
       // eigenvalues (descending) into theta, eigenvectors as columns of U (p x p, dense)
@@ -958,9 +955,7 @@ int afq_eigh_desc(int32_t n, const double* A, double* evals, double* evecs, void
   int* sweeps = reinterpret_cast<int*>(V + even(nn));
   bool packed = false;
   const size_t smem = jacobi_smem(n, &packed);
-  if (cudaFuncSetAttribute(jacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
-    return AFQ_ERR_CUDA;
+  if (allow_smem(jacobi_kernel, smem) != cudaSuccess) return AFQ_ERR_CUDA;
   ProfScope ps(K_MISC, st);
   jacobi_kernel<<<1, kJacobiThreads, smem, st>>>(n, packed ? 1 : 0, A, Ag, V, evals, evecs, sweeps);
   return cudaGetLastError() == cudaSuccess ? AFQ_OK : AFQ_ERR_CUDA;

@@ -361,7 +361,7 @@ cudaError_t launch_small_step(const Layout& L, const double* prep, double* work,
   a.kused = (int)L.Kfb_used;
   a.sdt = sqrt(dt);
   const size_t smem = small_smem(L.N, L.G, L.no[0], L.no[1], L.ns).total * sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(small_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(small_step_kernel, smem);
   if (e != cudaSuccess) return e;
   ProfScope ps(K_PROP, st);
   small_step_kernel<<<L.W, kSmallThreads, smem, st>>>(a);

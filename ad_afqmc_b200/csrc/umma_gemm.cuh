@@ -421,8 +421,7 @@ cudaError_t launch_umma(const UmmaParams<Epi>& P, int num_sms, cudaStream_t st) 
   if (P.s.stages < 2 || smem > kUmmaSmemBudget || (P.s.epi_bytes & 255) ||
       (EG > 2 ? EG : 2) * P.s.ngroups * BN > 512)
     return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(umma_gemm_kernel<BN, Epi, EG>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(umma_gemm_kernel<BN, Epi, EG>, smem);
   if (e != cudaSuccess) return e;
   const int tiles = P.s.batch * P.s.ksplit * P.s.mt * P.s.nt;
   const int grid = tiles < num_sms ? tiles : num_sms;
@@ -439,8 +438,7 @@ cudaError_t launch_umma_group(const UmmaGroup<Epi>& G, const UmmaShape& shape0, 
   if (G.n < 1 || G.n > kUmmaMaxGroup || G.stages < 2 || smem > kUmmaSmemBudget ||
       (shape0.epi_bytes & 255) || (EG > 2 ? EG : 2) * shape0.ngroups * BN > 512)
     return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(umma_group_kernel<BN, Epi, EG>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(umma_group_kernel<BN, Epi, EG>, smem);
   if (e != cudaSuccess) return e;
   const int tiles = G.start[G.n];
   const int grid = tiles < num_sms ? tiles : num_sms;

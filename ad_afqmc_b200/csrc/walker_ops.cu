@@ -804,7 +804,7 @@ template <class K>
 static cudaError_t launch_qr_kernel(K kernel, int threads, dim3 grid, size_t dyn, cudaStream_t st,
                                    const Layout& L, double* const walkers[2], int use_smem,
                                    double* secn) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+  cudaError_t e = allow_smem(kernel, dyn);
   if (e != cudaSuccess) return e;
   kernel<<<grid, threads, dyn, st>>>(L.N, L.no[0], L.no[1], walkers[0], L.ns == 2 ? walkers[1] : nullptr,
                                      L.restricted ? 0 : 1, use_smem, secn);
@@ -860,8 +860,7 @@ cudaError_t launch_sr(int W, int ranks, const double* weights_in, double zeta,
                       const double* zeta_dev, int mode, double* weights_out, int* indices,
                       cudaStream_t st) {
   const size_t smem = size_t(W) * sizeof(double);
-  cudaError_t e =
-      cudaFuncSetAttribute(sr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_smem(sr_kernel, smem);
   if (e != cudaSuccess) return e;
   ProfScope ps(K_SR, st);
   sr_kernel<<<1, 1024, smem, st>>>(W, ranks, weights_in, zeta, zeta_dev, mode, weights_out,
