@@ -52,12 +52,13 @@ def to_dev(x, dtype=torch.float64) -> torch.Tensor:
 
 
 def small_work(W: int) -> torch.Tensor:
+    """Scratch of the calls that need no engine (overlaps, Green's functions, QR): one
+    per number of walkers and stream, since calls on different streams may overlap."""
     dev = device()
-    key = (dev.index, W)
+    key = (dev.index, W, _lib.stream_handle())
     t = _small_work.get(key)
     if t is None:
-        t = torch.empty(W * 16, dtype=torch.float64, device=dev)
-        _small_work[key] = t
+        t = _small_work.setdefault(key, torch.empty(W * 16, dtype=torch.float64, device=dev))
     return t
 
 

@@ -65,3 +65,16 @@ def test_threads(precision):
     for t in threads:
         t.join()
     assert not failed, failed
+
+
+def test_scratch_per_stream():
+    """Overlaps, Green's functions and QR on two streams do not share scratch."""
+    from ad_afqmc_b200._engine import small_work
+
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(a):
+        x = small_work(6)
+        again = small_work(6)
+    with torch.cuda.stream(b):
+        y = small_work(6)
+    assert x.data_ptr() == again.data_ptr() != y.data_ptr()
