@@ -20,9 +20,9 @@
 //    the MMA reads on into whatever follows, and those rows and columns of the
 //    accumulator are never looked at.
 //  * Eight epilogue warps share a tile (see exch_tile); its sums end in FP64 (exch_finish).
-// Measured on a B200, two pieces, per launch: N = 200, No = 40, G = 1000, W = 512
-// 4.74 -> 2.43 ms; N = 300, No = 60, G = 1500, W = 1024 29.7 -> 22.8 ms; N = 250,
-// No = 62, G = 1250, W = 256 4.98 -> 3.47 ms.
+// Measured on a B200, two pieces, per launch, the general GEMM before -> this: N = 200,
+// No = 40, G = 1000, W = 512 4.74 -> 2.45 ms; N = 300, No = 60, G = 1500, W = 1024 29.7 ->
+// 23.8 ms; N = 250, No = 62, G = 1250, W = 256 4.98 -> 3.53 ms.
 #pragma once
 
 #include "layout.cuh"

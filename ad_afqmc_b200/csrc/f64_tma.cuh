@@ -23,10 +23,10 @@
 //    are in use takes them in order.
 // Registers-only DMMA runs at 36.5 TF/s on this chip; a cp.async main loop with
 // address arithmetic in every warp and a block barrier per stage reached 22.4.
-// Measured, N = 200, No = 40, G = 1000, 512 walkers, per step: VHS 3.65 -> 2.70 ms
-// (30.4 TF/s), propagator 3.50 -> 1.75 ms, force bias 0.77 -> 0.52 ms; exchange 30.1 ->
-// 25.0 ms.  N = 95, G = 471, 161 walkers, per block: VHS 2.15 -> 1.17 ms,
-// propagator 5.20 -> 1.0 ms.
+// Measured, that loop -> this, N = 200, No = 40, G = 1000, 512 walkers, per step: VHS 3.65 ->
+// 2.65 ms (31 TF/s), propagator 3.50 -> 1.79 ms, force bias 0.77 -> 0.52 ms; exchange 30.1 ->
+// 24.0 ms.  N = 95, G = 471, 161 walkers, per block of ten steps: VHS 2.15 -> 1.23 ms,
+// propagator 5.20 -> 1.25 ms.
 #pragma once
 
 #include <type_traits>

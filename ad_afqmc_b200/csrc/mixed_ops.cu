@@ -570,7 +570,7 @@ int vhs_launch(const Layout& L, const double* prep, double* work, cudaStream_t s
   P.epi.ld = L.Kv;
   P.epi.wstride = (long long)L.N * L.Kv;
   // K = G in one TMEM chain per accumulator group (the hi x hi product apart),
-  // which leaves the shared memory to four operand stages (191 us per
+  // which leaves the shared memory to four operand stages (203 us per
   // launch at N = 200, G = 1000, W = 512; block energies 7.8e-6 Ha from FP64),
   // or (vhs_chunk = 2) in chunks of four 64-wide K blocks summed in FP32
   // round-to-nearest through a shared-memory row per TMEM lane (5.0e-6 Ha)

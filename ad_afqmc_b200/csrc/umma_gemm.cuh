@@ -8,7 +8,7 @@
 //
 // Roles (64 + 128*EG threads, one CTA per SM, persistent over tiles):
 //   warp 0      TMA producer: 128-byte-swizzled K-major tiles into a STAGES ring
-//   warp 1      TMEM allocator; lane 0 issues tcgen05.mma into one of two
+//   warp 1      TMEM allocator; an elected lane issues tcgen05.mma into one of two
 //               accumulators and commits stage/accumulator barriers
 //   warps 2..5  epilogue: tcgen05.ld rows of the finished accumulator (one TMEM
 //               lane per thread) and hand 32 columns at a time to the functor

@@ -322,7 +322,7 @@ def measure_config(name, precision, steps, warmup, nb_acc):
 # of one step, from ncu (dram__bytes_read.sum + dram__bytes_write.sum, caches
 # flushed before each launch) on the bench workload (N=200, No=40, G=1000,
 # 512 walkers, mixed, Taylor terms in Horner form).
-PROP_DRAM_BYTES_PER_LAUNCH = 243791506
+PROP_DRAM_BYTES_PER_LAUNCH = 263800000
 
 
 def main():
