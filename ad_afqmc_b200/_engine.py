@@ -52,13 +52,15 @@ def to_dev(x, dtype=torch.float64) -> torch.Tensor:
 
 
 def small_work(W: int) -> torch.Tensor:
-    """Scratch of the calls that need no engine (overlaps, Green's functions, QR): one
-    per number of walkers and stream, since calls on different streams may overlap."""
+    """Scratch of the calls that need no engine (overlaps, Green's functions, QR) for at
+    least W walkers: one per stream, since calls on different streams may overlap, and
+    power of two, so that a stream keeps no more than twice the largest."""
     dev = device()
-    key = (dev.index, W, _lib.stream_handle())
+    walkers = 1 << max(6, (W - 1).bit_length())
+    key = (dev.index, walkers, _lib.stream_handle())
     t = _small_work.get(key)
     if t is None:
-        t = _small_work.setdefault(key, torch.empty(W * 16, dtype=torch.float64, device=dev))
+        t = _small_work.setdefault(key, torch.empty(walkers * 16, dtype=torch.float64, device=dev))
     return t
 
 

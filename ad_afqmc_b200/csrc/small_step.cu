@@ -8,7 +8,7 @@
 // launch.  Every operand a walker needs (chol, rot_chol) is read from L2 once per
 // walker, so the rule below bounds that: beyond it the tensor-core launches, which
 // share the reads among walkers, are faster.
-// Measured (B200, recorded block of 10 steps): see small_step_fits.
+// Measured (B200, recorded steps): see small_step_fits.
 #include "common.cuh"
 #include "gauss_jordan.cuh"
 #include "ops.h"
@@ -363,7 +363,7 @@ cudaError_t launch_small_step(const Layout& L, const double* prep, double* work,
   const size_t smem = small_smem(L.N, L.G, L.no[0], L.no[1], L.ns).total * sizeof(double);
   cudaError_t e = allow_smem(small_step_kernel, smem);
   if (e != cudaSuccess) return e;
-  ProfScope ps(K_PROP, st);
+  ProfScope ps(K_PROP, st);  // the whole step is counted as the propagator
   small_step_kernel<<<L.W, kSmallThreads, smem, st>>>(a);
   return cudaGetLastError();
 }
